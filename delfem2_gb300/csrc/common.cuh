@@ -341,22 +341,25 @@ struct ChainSched {
   dfm2g::DevBuf<unsigned> ctr;      // chain counter and done-ticket of the launch
 };
 
-// Tiles of one sweep direction and value type (tiles.cu; FP32 and FP64 tiles
-// differ in size): tile and step descriptors, the record of each row, group
-// headers and codes, per-step halo lists, and the records (rewritten after
-// each decomposition).
+// Tiles of one sweep direction and value type (tiles.cu): tile and step
+// descriptors, the groups' header words and slot sources, and the records
+// (rewritten after each decomposition).
 struct TileSched {
-  bool built = false, ok = false;
-  unsigned ntiles = 0, nsteps = 0, M = 0, max_groups = 0, max_halo = 0;  // M: dependency slots per row
+  bool built = false, ok = false, thin = false;  // thin: too few rows per tile, not swept unless asked for
+  unsigned ntiles = 0, nsteps = 0, ms = 0, max_groups = 0, max_tile = 0;  // ms: slots per lane
+  unsigned max_list = 0, max_record = 0;  // longest row list, longest record / 16
+  size_t stream16 = 0;                // bytes of the records / 16
   double rows_per_step = 0;           // rows / steps: how full the tiles' steps are
   size_t ngroups = 0;
   unsigned ver = ~0u;                 // factor_version the records were written from
   int coop = 0;                       // resident CTAs of the sweep kernel
-  dfm2g::DevBuf<uint4> tiles;         // 2 per tile: {first step, steps, first group, groups}, {halo words}
-  dfm2g::DevBuf<uint4> steps;         // 2 per step: {first group, rows, local base, groups}, {halo list}
-  dfm2g::DevBuf<unsigned> halo;       // per step: the rows of other tiles it reads
-  dfm2g::DevBuf<unsigned> rec_of;     // 10 * group + position of each row
-  dfm2g::DevBuf<unsigned> gmeta;      // per group: 10 row ids, then codes [10][Mc]
+  dfm2g::DevBuf<uint4> tiles;         // {first step, steps, offset and length of its records / 16}
+  dfm2g::DevBuf<uint4> steps;         // {offset and length of its record / 16, groups and rows, local base}
+  dfm2g::DevBuf<unsigned> codes;      // per group: operand offsets (the record's first bytes)
+  dfm2g::DevBuf<unsigned> src;        // per slot: its factor block
+  dfm2g::DevBuf<unsigned> grow, goff; // rows and record offset / 16 of each group
+  dfm2g::DevBuf<unsigned> lists;      // per step: its own rows, then the rows of other tiles it reads
+  dfm2g::DevBuf<unsigned> loff;       // per four list words: their offset / 16
   dfm2g::DevBuf<unsigned char> bytes; // the records
   dfm2g::DevBuf<unsigned> ctr;        // tile counter and done-ticket of the launch
 };
@@ -430,15 +433,16 @@ int chain_sweep(dfm2g_ilu_s *p, bool forward, const T *in, T *out, const T *vcrs
                 unsigned long long timeout, bool may_alloc, bool *usable);
 void chain_schedules_reset(dfm2g_ilu_s *p);
 template <typename T>
-int tile_sweep(dfm2g_ilu_s *p, bool forward, const T *in, T *out, const T *vcrs, const T *vdia, const int *skip,
-               unsigned long long timeout, bool may_alloc, bool pick, bool *usable);
+int tile_sweep(dfm2g_ilu_s *p, bool forward, const T *in, T *out, const int *skip, unsigned long long timeout,
+               bool may_alloc, bool force, bool *usable, bool *full);
 void tile_schedules_reset(dfm2g_ilu_s *p);
 template <typename T>
 int cluster_sweep(dfm2g_ilu_s *p, bool forward, const T *in, T *out, const T *vcrs, const T *vdia, const int *skip,
                   bool *usable);
 void tile_partition(unsigned n, const unsigned *rs, const unsigned *dia, const unsigned *col, const unsigned *order,
-                    bool fwd, unsigned max_rows, unsigned max_width, std::vector<unsigned> &tile_of,
-                    std::vector<unsigned> &lev, unsigned &ntiles, unsigned &m);
+                    bool fwd, unsigned max_rows, unsigned max_segs, unsigned max_width,
+                    std::vector<unsigned> &tile_of, std::vector<unsigned> &lev, unsigned &ntiles, unsigned &m,
+                    unsigned give_up);
 template <typename T>
 int part_sweep(dfm2g_ilu_s *p, bool forward, const T *in, T *out, const T *vcrs, const T *vdia, const int *skip,
                unsigned long long timeout);

@@ -803,10 +803,10 @@ static int nd_sweep_impl(dfm2g_ilu_s *p, bool forward, const T *in, T *out, cons
   if ((const void *)in == (const void *)out) return fail(DFM2G_ERR_ARG, "sync-free sweep needs in != out");
   if (!prefilled) DFM2G_CUDA(cudaMemsetAsync(out, 0xFF, sizeof(T) * n * B, stream()));
   if (p->sweep_mode == DFM2G_SWEEP_CHAINS || p->sweep_mode == DFM2G_SWEEP_AUTO) {
-    const unsigned nlev_c = forward ? p->nlev_f : p->nlev_b;
-    bool usable = false;
-    DFM2G_TRY(chain_sweep<T>(p, forward, in, out, vcrs, vdia, skip, kWaitTimeoutNs + 20000ull * nlev_c, may_alloc,
-                             &usable));
+    const unsigned long long timeout = kWaitTimeoutNs + 20000ull * (forward ? p->nlev_f : p->nlev_b);
+    bool usable = false, full = false;
+    DFM2G_TRY(tile_sweep<T>(p, forward, in, out, skip, timeout, may_alloc, false, &usable, &full));
+    if (!usable) DFM2G_TRY(chain_sweep<T>(p, forward, in, out, vcrs, vdia, skip, timeout, may_alloc, &usable));
     if (usable) {
       ran = DFM2G_SWEEP_CHAINS;
       return DFM2G_OK;
@@ -887,21 +887,17 @@ static int sweep_impl(dfm2g_ilu_s *p, bool forward, const T *in, T *out, const T
   // sync-free, tile, chain and blob schedules: `out` is filled with the pending marker
   if (!prefilled) DFM2G_CUDA(cudaMemsetAsync(out, 0xFF, sizeof(T) * n * 3, stream()));
   const bool auto_pick = p->sweep_mode == DFM2G_SWEEP_AUTO || p->sweep_mode == DFM2G_SWEEP_CLUSTER;
-  if (p->sweep_mode == DFM2G_SWEEP_TILES || auto_pick) {
-    const unsigned nlev = forward ? p->nlev_f : p->nlev_b;
-    bool usable = false;
-    DFM2G_TRY(tile_sweep<T>(p, forward, in, out, vcrs, vdia, skip, kWaitTimeoutNs + 20000ull * nlev, may_alloc,
-                            auto_pick, &usable));
-    if (usable) {
-      ran = DFM2G_SWEEP_TILES;
-      return DFM2G_OK;
-    }  // else (rows too long for the tiles, not built, or not picked): the chains below
-  }
   if (p->sweep_mode == DFM2G_SWEEP_CHAINS || p->sweep_mode == DFM2G_SWEEP_TILES || auto_pick) {
     const unsigned nlev = forward ? p->nlev_f : p->nlev_b;
-    bool usable = false;
-    DFM2G_TRY(chain_sweep<T>(p, forward, in, out, vcrs, vdia, skip, kWaitTimeoutNs + 20000ull * nlev, may_alloc,
-                             &usable));
+    const unsigned long long timeout = kWaitTimeoutNs + 20000ull * nlev;
+    bool usable = false, full = false;
+    DFM2G_TRY(tile_sweep<T>(p, forward, in, out, skip, timeout, may_alloc, p->sweep_mode == DFM2G_SWEEP_TILES,
+                            &usable, &full));
+    if (usable) {
+      ran = !auto_pick ? p->sweep_mode : full ? DFM2G_SWEEP_TILES : DFM2G_SWEEP_CHAINS;
+      return DFM2G_OK;
+    }  // else (rows too long for the tiles' records, or not built): one warp per chain
+    DFM2G_TRY(chain_sweep<T>(p, forward, in, out, vcrs, vdia, skip, timeout, may_alloc, &usable));
     if (usable) {
       ran = DFM2G_SWEEP_CHAINS;
       return DFM2G_OK;

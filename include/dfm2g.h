@@ -76,21 +76,20 @@ enum dfm2g_sweep {
                                polled in shared memory, only cross-range ones
                                in global memory (when a range's results fit
                                in shared memory)                            */
-  DFM2G_SWEEP_CHAINS = 5,   /* sync-free over chains of consecutive rows in
-                               which each row depends on the one before: one
-                               warp per chain hands that dependency over in
-                               registers and polls only the others; the
-                               chain's factor blocks are TMA-streamed into
-                               shared memory ahead of the warp               */
-  DFM2G_SWEEP_TILES = 6,    /* 3x3: rows in tiles of up to 49
-                               segments of dependency chains (7 x 7 columns
+  DFM2G_SWEEP_CHAINS = 5,   /* chains of consecutive rows in which each row
+                               depends on the one before, bundled into tiles
+                               as below; one warp per chain (that dependency
+                               in registers, the others polled) where rows
+                               have more than 15 blocks in a triangle or
+                               tiles would hold fewer than 16 rows           */
+  DFM2G_SWEEP_TILES = 6,    /* 3x3: rows in tiles of up to 36 (FP32) or 16
+                               (FP64) segments of dependency chains (squares
                                of grid lines on voxel meshes), one CTA per
                                tile walking the tile's local levels with
                                shared-memory hand-offs inside the tile and
-                               copies or polls only across tiles; records
-                               TMA-streamed per level. Patterns whose rows
-                               have more than 16 blocks in a triangle use
-                               the chain schedule                           */
+                               polls only across tiles; records TMA-streamed
+                               per level. Patterns whose rows have more than
+                               15 blocks in a triangle use a warp per chain  */
   DFM2G_SWEEP_CLUSTER = 8,  /* 3x3 systems whose solution vector fits in
                                shared memory (9,400 block rows FP64, 18,900
                                FP32): one thread-block cluster of 8 CTAs
@@ -102,11 +101,9 @@ enum dfm2g_sweep {
                                smallest (a cluster barrier and broadcast cost
                                about 1.3 us per level in FP32, 2.9 in FP64)  */
   DFM2G_SWEEP_AUTO = 7      /* the default: DFM2G_SWEEP_TILES where the tiles'
-                               steps hold 20 rows or more on average, rows
-                               have at most 8 dependency blocks per
-                               triangle and, for FP64, there are at least
-                               half as many tiles as SMs (the FP64 steps are
-                               bound by the SM's FP64 rate);
+                               steps are at least half full, rows have at
+                               most 8 dependency blocks per triangle and, for
+                               FP64, the pattern has at least 77,824 rows;
                                DFM2G_SWEEP_CHAINS otherwise (2-D meshes,
                                fill-in patterns, small grids)                */
 };
@@ -272,7 +269,7 @@ DFM2G_API int dfm2g_chain_partition(unsigned n, const unsigned *row_start, const
  * row i's tile (numbered in dependency order), level[i] its local level inside
  * the tile; tiles hold at most max_width strand segments of at most
  * max_rows / max_width rows each (so at most max_width rows per local level);
- * the sweep uses max_rows 3185 (FP32) or 1617 (FP64), max_width 49.
+ * 3x3 sweeps use 36 segments of 65 rows (FP32) or 16 (FP64).
  * *max_deps the most blocks of a
  * row's triangle (forward: strictly lower, backward: strictly upper). */
 DFM2G_API int dfm2g_tile_partition(unsigned n, const unsigned *row_start, const unsigned *col,
