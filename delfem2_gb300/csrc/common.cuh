@@ -158,6 +158,14 @@ __device__ __forceinline__ void st_relaxed(float *p, float v) {
 __device__ __forceinline__ void st_relaxed(double *p, double v) {
   asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
 }
+__device__ __forceinline__ unsigned ld_acquire(const unsigned *p) {
+  unsigned v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_release(unsigned *p, unsigned v) {
+  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
 __device__ __forceinline__ unsigned long long globaltimer_ns() {
   unsigned long long t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -397,6 +405,10 @@ struct dfm2g_ilu_s {
   dfm2g::DevBuf<int> nsing;
   int coop_cache[2][2][2] = {};         // resident blocks of the sync-free kernel [f64][fwd][wide]
   unsigned max_lower = 0, max_upper = 0; // longest triangle rows (blocks)
+  unsigned max_row = 0;                  // longest row
+  dfm2g::DevBuf<unsigned short> flow_tab;  // one-launch factorisation: update targets,
+  dfm2g::DevBuf<unsigned> flow_flags;      // and the decomposition each row was last finished in
+  unsigned flow_epoch = 0;
   int last_sched[2][2] = {{-1, -1}, {-1, -1}};  // schedule of the last sweep [f64][backward]
 };
 

@@ -483,6 +483,253 @@ __global__ void __launch_bounds__(256) k_ilu_factor_level_nd(const unsigned *__r
 }
 
 // ---------------------------------------------------------------------------
+// Decompose in one launch: a co-resident grid, warp w taking positions w,
+// w + W, ... of the (level, row) order. A row is loaded into shared memory,
+// waits (bounded) until the rows of its lower triangle carry this
+// decomposition's flag, takes their updates in ascending order, as the level
+// kernels above do, and is written and flagged. Every dependency lies earlier
+// in the order and each warp walks its positions in order, so the earliest
+// unfinished row can always proceed.
+//
+// The updates' targets are looked up once per pattern: tab[s maxu + t] is the
+// row-local block that A_ik U_kj updates, (i, k) the block in slot s, U_kj
+// the t-th block of row k's upper triangle (kTabDia: D_i, kTabNone: outside
+// the pattern). R > 0: rounds of 32 entries that cover maxu blocks; the
+// next k's U blocks are loaded while this k's products run.
+//
+// What bounds it: FP64 issue (64 cycles per warp instruction and SM quarter)
+// where levels are wide, the row's chain of products where they are narrow; so
+// a 3x3 pivot's inverse is split over nine lanes (18 FP64 instructions instead
+// of 55). Decompose, one launch per level -> one launch: 65^3 3x3 rows (193
+// levels) 5.29 -> 1.87 ms, 17^3 rows 0.99 -> 0.31, ILU(1) of 26 x 28 x 24 rows
+// 8.76 -> 1.24, a 45 x 45 cloth sheet (177 levels) 3.22 -> 0.73, 65^3 scalar
+// rows 2.35 -> 1.00.
+constexpr unsigned kTabDia = 0xFFFEu, kTabNone = 0xFFFFu;
+constexpr unsigned kFlowWarps = 4;
+
+__global__ void k_ilu_targets(unsigned nblk, const unsigned *__restrict__ row_start, const unsigned *__restrict__ col,
+                              const unsigned *__restrict__ dia_ind, unsigned maxu, unsigned short *__restrict__ tab) {
+  const unsigned lane = threadIdx.x & 31, nwarp = (gridDim.x * blockDim.x) >> 5;
+  for (unsigned i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < nblk; i += nwarp) {
+    const unsigned s0 = row_start[i], s1 = row_start[i + 1], nk = dia_ind[i] - s0;
+    for (unsigned e = lane; e < nk * maxu; e += 32) {
+      const unsigned s = s0 + e / maxu, t = e % maxu, k = col[s];
+      const unsigned u = dia_ind[k] + t;
+      unsigned dst = kTabNone;
+      if (u < row_start[k + 1]) {
+        const unsigned j = col[u];
+        if (j == i) {
+          dst = kTabDia;
+        } else {
+          unsigned lo = s0, hi = s1;
+          while (lo < hi) {
+            const unsigned mid = (lo + hi) >> 1;
+            if (col[mid] < j) lo = mid + 1; else hi = mid;
+          }
+          if (lo < s1 && col[lo] == j) dst = lo - s0;
+        }
+      }
+      tab[(size_t)s0 * maxu + e] = (unsigned short)dst;
+    }
+  }
+}
+
+// A_ij[e] -= row r of A_ik times column c of U_kj: fused for 3x3 blocks, each
+// operation rounded on its own for 1x1 and 2x2 (the reference's arithmetic).
+template <int B>
+__device__ __forceinline__ double ilu_update(double dst, const double *aik, const double u[B]) {
+  if constexpr (B == 3) {
+    return dst - (aik[0] * u[0] + aik[1] * u[1] + aik[2] * u[2]);
+  } else {
+    double sum = __dmul_rn(aik[0], u[0]);
+#pragma unroll
+    for (int q = 1; q < B; ++q) sum = __dadd_rn(sum, __dmul_rn(aik[q], u[q]));
+    return __dsub_rn(dst, sum);
+  }
+}
+
+template <int B, int R>
+__global__ void __launch_bounds__(32 * kFlowWarps) k_ilu_factor_flow(
+    unsigned n, const unsigned *__restrict__ order, const unsigned *__restrict__ row_start,
+    const unsigned *__restrict__ col, const unsigned *__restrict__ dia_ind,
+    const unsigned short *__restrict__ tab, unsigned maxu, unsigned maxnb, unsigned warp_bytes, double *vcrs,
+    double *vdia, unsigned *flags, unsigned epoch, int *nsing, int *err, unsigned long long timeout_ns) {
+  constexpr unsigned BB = B * B;
+  extern __shared__ __align__(16) unsigned char flow_smem[];
+  const unsigned lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
+  const unsigned nwarp = gridDim.x * kFlowWarps;
+  double *row = reinterpret_cast<double *>(flow_smem + (size_t)wib * warp_bytes);  // maxnb blocks, then D_i
+  unsigned short *tb = reinterpret_cast<unsigned short *>(row + (size_t)(maxnb + 1) * BB);
+  double *dia = row + (size_t)maxnb * BB;
+  for (unsigned q = blockIdx.x * kFlowWarps + wib; q < n; q += nwarp) {
+    const unsigned i = order[q];
+    const unsigned s0 = row_start[i], s1 = row_start[i + 1], sd = dia_ind[i];
+    const unsigned nb = s1 - s0, nk = sd - s0;
+    for (unsigned e = lane; e < nb * BB; e += 32) row[e] = vcrs[(size_t)s0 * BB + e];
+    if (lane < BB) dia[lane] = vdia[(size_t)i * BB + lane];
+    for (unsigned e = lane; e < nk * maxu; e += 32) tb[e] = tab[(size_t)s0 * maxu + e];
+    __syncwarp();
+    // readiness of the lower triangle's rows, 32 at a time: bit l of `ready`
+    // once row col[s0 + r0 + l] carries this decomposition's flag. need(l)
+    // waits (bounded) for it, so that the updates from rows of earlier levels
+    // are done while the level just before is still at work.
+    unsigned ready = 0, r0 = ~0u;
+    const unsigned *flag = nullptr;
+    auto need = [&](unsigned l) -> bool {
+      if ((l & ~31u) != r0) {
+        r0 = l & ~31u;
+        ready = 0;
+        if (r0 + lane < nk) flag = flags + col[s0 + r0 + lane];
+      }
+      unsigned long long t0 = 0;
+      unsigned spins = 0;
+      while (!((ready >> (l & 31u)) & 1u)) {
+        bool ok = r0 + lane < nk && ((ready >> lane) & 1u || ld_acquire(flag) == epoch);
+        ready = __ballot_sync(0xffffffffu, ok);
+        if ((++spins & 63u) == 0) {
+          const unsigned long long now = globaltimer_ns();
+          if (t0 == 0) t0 = now;
+          const bool stop = ld_relaxed(err) != 0 || now - t0 > timeout_ns;
+          if (__any_sync(0xffffffffu, stop)) {
+            atomicCAS(err, 0, DFM2G_ERR_WAIT_TIMEOUT);
+            return false;
+          }
+        }
+      }
+      return true;
+    };
+    auto known = [&](unsigned l) { return (l & ~31u) == r0 && ((ready >> (l & 31u)) & 1u); };
+    // entry x of row k's update: block t = x / BB of U_k, component x % BB
+    auto u_base = [&](unsigned l, unsigned &nu) {
+      const unsigned k = col[s0 + l], u0 = dia_ind[k];
+      nu = row_start[k + 1] - u0;
+      return u0;
+    };
+    if constexpr (R > 0) {
+      double un[R][B];
+      unsigned nun = 0;
+      auto fetch = [&](unsigned l) {
+        const unsigned u0 = u_base(l, nun);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const unsigned x = lane + 32u * r, t = x / BB, c = x % BB % B;
+          if (t < nun) {
+#pragma unroll
+            for (int p = 0; p < B; ++p) un[r][p] = __ldcg(vcrs + (size_t)(u0 + t) * BB + p * B + c);
+          }
+        }
+      };
+      unsigned fetched = 0;  // rows whose U blocks are loaded
+      for (unsigned l = 0; l < nk; ++l) {
+        if (!need(l)) return;
+        if (fetched == l) {
+          fetch(l);
+          ++fetched;
+        }
+        double uc[R][B];
+        const unsigned nu = nun;
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+#pragma unroll
+          for (int p = 0; p < B; ++p) uc[r][p] = un[r][p];
+        if (l + 1 < nk && known(l + 1)) {
+          fetch(l + 1);
+          ++fetched;
+        }
+        const double *aik = row + (size_t)l * BB;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const unsigned x = lane + 32u * r, t = x / BB, e = x % BB;
+          if (t < nu) {
+            const unsigned dst = tb[l * maxu + t];
+            if (dst != kTabNone) {
+              double *d = (dst == kTabDia ? dia : row + (size_t)dst * BB) + e;
+              *d = ilu_update<B>(*d, aik + e / B * B, uc[r]);
+            }
+          }
+        }
+        __syncwarp();
+      }
+    } else {
+      for (unsigned l = 0; l < nk; ++l) {
+        if (!need(l)) return;
+        unsigned nu;
+        const unsigned u0 = u_base(l, nu);
+        const double *aik = row + (size_t)l * BB;
+        for (unsigned x = lane; x < nu * BB; x += 32) {
+          const unsigned t = x / BB, e = x % BB;
+          const unsigned dst = tb[l * maxu + t];
+          if (dst == kTabNone) continue;
+          double u[B];
+#pragma unroll
+          for (int p = 0; p < B; ++p) u[p] = __ldcg(vcrs + (size_t)(u0 + t) * BB + p * B + e % B);
+          double *d = (dst == kTabDia ? dia : row + (size_t)dst * BB) + e;
+          *d = ilu_update<B>(*d, aik + e / B * B, u);
+        }
+        __syncwarp();
+      }
+    }
+    // the pivot: inverted when |det| > 1e-30, else counted and left as it is
+    if constexpr (B == 3) {
+      // lane e < 9: entry e of the adjugate, p q - r s; det from its first column
+      const unsigned e = lane < 9 ? lane : 0u;
+      const unsigned er = e / 3u, ec = e - er * 3u;
+      const unsigned r1 = ec == 2u ? 0u : ec + 1u, r2 = ec == 0u ? 2u : ec - 1u;  // the other two rows, cyclic
+      const unsigned c1 = er == 2u ? 0u : er + 1u, c2 = er == 0u ? 2u : er - 1u;  // the other two columns, cyclic
+      const double adj = dia[r1 * 3 + c1] * dia[r2 * 3 + c2] - dia[r1 * 3 + c2] * dia[r2 * 3 + c1];
+      const double a0 = __shfl_sync(0xffffffffu, adj, 0), a1 = __shfl_sync(0xffffffffu, adj, 3),
+                   a2 = __shfl_sync(0xffffffffu, adj, 6);
+      const double det = dia[0] * a0 + dia[1] * a1 + dia[2] * a2;
+      const bool regular = fabs(det) > 1.0e-30;
+      const double v = regular ? (1.0 / det) * adj : dia[e];
+      __syncwarp();
+      if (lane < 9) dia[lane] = v;
+      if (!regular && lane == 0) atomicAdd(nsing, 1);
+    } else {
+      double v = dia[lane < BB ? lane : 0];
+      bool regular;
+      if constexpr (B == 1) {
+        regular = fabs(v) > 1.0e-30;
+        if (regular) v = 1.0 / v;
+      } else {
+        const double det = __dsub_rn(__dmul_rn(dia[0], dia[3]), __dmul_rn(dia[1], dia[2]));
+        regular = fabs(det) > 1.0e-30;
+        if (regular) {
+          const double inv_det = 1.0 / det;
+          const double s = lane == 1 || lane == 2 ? -inv_det : inv_det;
+          v = __dmul_rn(s, lane == 0 ? dia[3] : lane == 3 ? dia[0] : v);
+        }
+      }
+      __syncwarp();
+      if (lane < BB) dia[lane] = v;
+      if (!regular && lane == 0) atomicAdd(nsing, 1);
+    }
+    __syncwarp();
+    // L_ik as updated, U_ij <- D_i^-1 U_ij, D_i^-1
+    for (unsigned x = lane; x < nb * BB; x += 32) {
+      double o;
+      if (x < nk * BB) {
+        o = row[x];
+      } else {
+        const unsigned e = x % BB, r = e / B, c = e % B;
+        const double *t = row + (x - e);
+        if constexpr (B == 3) {
+          o = dia[r * 3 + 0] * t[c] + dia[r * 3 + 1] * t[3 + c] + dia[r * 3 + 2] * t[6 + c];
+        } else if constexpr (B == 2) {
+          o = __dadd_rn(__dmul_rn(dia[r * 2], t[c]), __dmul_rn(dia[r * 2 + 1], t[2 + c]));
+        } else {
+          o = __dmul_rn(t[0], dia[0]);
+        }
+      }
+      vcrs[(size_t)s0 * BB + x] = o;
+    }
+    if (lane < BB) vdia[(size_t)i * BB + lane] = dia[lane];
+    __syncwarp();
+    if (lane == 0) st_release(flags + i, epoch);
+  }
+}
+
+// ---------------------------------------------------------------------------
 // Sweeps. Forward: out_i = D_i^-1 (in_i - sum_{j<i} L_ij out_j). Backward:
 // out_i = in_i - sum_{j>i} U'_ij out_j. One warp per row in the lane layout of
 // rowkern.cuh. Rows are visited in level order through per-position
@@ -1060,8 +1307,9 @@ static int ilu_install_pattern(dfm2g_ilu p, unsigned n, unsigned ndim, size_t nn
       DFM2G_CUDA(cudaMemcpyAsync(hdia.data(), p->dia_ind.p, sizeof(unsigned) * n, cudaMemcpyDeviceToHost, stream()));
       DFM2G_CUDA(cudaStreamSynchronize(stream()));
     }
-    p->max_lower = p->max_upper = 0;
+    p->max_lower = p->max_upper = p->max_row = 0;
     for (unsigned i = 0; i < n; ++i) {
+      p->max_row = std::max(p->max_row, hrs[i + 1] - hrs[i]);
       p->max_lower = std::max(p->max_lower, hdia[i] - hrs[i]);
       p->max_upper = std::max(p->max_upper, hrs[i + 1] - hdia[i]);
     }
@@ -1074,6 +1322,8 @@ static int ilu_install_pattern(dfm2g_ilu p, unsigned n, unsigned ndim, size_t nn
   stream_schedules_reset(p);
   chain_schedules_reset(p);
   tile_schedules_reset(p);
+  p->flow_tab.release();
+  p->flow_flags.release();
   if (ndim == 3) {  // the blob and row-range schedules are written for 3x3 blocks
     DFM2G_TRY(group_schedules_build(p));
     DFM2G_TRY(part_schedules_build(p));
@@ -1094,6 +1344,70 @@ static int ilu_install_pattern(dfm2g_ilu p, unsigned n, unsigned ndim, size_t nn
   DFM2G_CUDA(cudaStreamSynchronize(stream()));
   p->has_pattern = true;
   return DFM2G_OK;
+}
+
+// The factorisation in one launch (k_ilu_factor_flow); *flowed stays false
+// when a row does not fit shared memory or the target table would exceed
+// kFlowTabMax bytes (then one launch per level).
+constexpr size_t kFlowTabMax = size_t(1) << 30;
+
+template <int B, int R>
+static int launch_flow(dfm2g_ilu p, unsigned maxu, unsigned maxnb, unsigned warp_bytes, bool *flowed) {
+  auto kernel = k_ilu_factor_flow<B, R>;
+  const size_t smem = (size_t)kFlowWarps * warp_bytes;
+  static size_t allowed[64] = {};  // per instantiation and device; the attribute only grows
+  const int dev = ctx().device;
+  if (dev < 0 || dev >= 64) return DFM2G_OK;
+  if (smem > allowed[dev]) {
+    DFM2G_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allowed[dev] = smem;
+  }
+  int per_sm = 0;
+  DFM2G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 32 * kFlowWarps, smem));
+  if (per_sm <= 0) return DFM2G_OK;
+  const unsigned blocks =
+      std::min<unsigned>((unsigned)per_sm * (unsigned)ctx().num_sms, (p->nblk + kFlowWarps - 1) / kFlowWarps);
+  unsigned n = p->nblk, epoch = ++p->flow_epoch;
+  const unsigned *order = p->order_f.p, *rs = p->row_start.p, *col = p->col.p, *dia = p->dia_ind.p;
+  const unsigned short *tab = p->flow_tab.p;
+  double *vcrs = p->vcrs.p, *vdia = p->vdia.p;
+  unsigned *flags = p->flow_flags.p;
+  int *nsing = p->nsing.p, *err = p->err.p;
+  unsigned long long timeout = kWaitTimeoutNs + 20000ull * p->nlev_f;
+  void *args[] = {&n, &order, &rs, &col, &dia, &tab, &maxu, &maxnb, &warp_bytes, &vcrs, &vdia, &flags, &epoch,
+                  &nsing, &err, &timeout};
+  DFM2G_CUDA(cudaLaunchCooperativeKernel((void *)kernel, dim3(blocks), dim3(32 * kFlowWarps), args, smem, stream()));
+  note_launches(1);
+  *flowed = true;
+  return DFM2G_OK;
+}
+
+template <int B>
+static int factor_flow(dfm2g_ilu p, bool *flowed) {
+  *flowed = false;
+  const unsigned maxu = std::max(1u, p->max_upper), maxnb = p->max_row;
+  if (p->nblk == 0 || maxnb >= kTabDia) return DFM2G_OK;
+  const size_t warp_bytes = ((size_t)(maxnb + 1) * B * B * 8 + (size_t)p->max_lower * maxu * 2 + 15) / 16 * 16;
+  const size_t tab = p->nnz * maxu;
+  if (warp_bytes * kFlowWarps > 200u * 1024u || tab * 2 > kFlowTabMax) return DFM2G_OK;
+  if (!p->flow_tab.p) {
+    DFM2G_TRY(p->flow_tab.resize(tab + 1));
+    DFM2G_TRY(p->flow_flags.resize(p->nblk));
+    DFM2G_CUDA(cudaMemsetAsync(p->flow_flags.p, 0, sizeof(unsigned) * p->nblk, stream()));
+    p->flow_epoch = 0;
+    k_ilu_targets<<<blocks_for((size_t)p->nblk * 32, 256, ctx().num_sms * 16), 256, 0, stream()>>>(
+        p->nblk, p->row_start.p, p->col.p, p->dia_ind.p, maxu, p->flow_tab.p);
+    note_launches(1);
+    DFM2G_LAUNCH_CHECK();
+  }
+  if (p->flow_epoch == 0xFFFFFFFEu) {  // the flags' epochs are used up: start over
+    DFM2G_CUDA(cudaMemsetAsync(p->flow_flags.p, 0, sizeof(unsigned) * p->nblk, stream()));
+    p->flow_epoch = 0;
+  }
+  const unsigned rounds = (maxu * B * B + 31) / 32;
+  if (rounds <= 2) return launch_flow<B, 2>(p, maxu, maxnb, (unsigned)warp_bytes, flowed);
+  if (rounds <= 4) return launch_flow<B, 4>(p, maxu, maxnb, (unsigned)warp_bytes, flowed);
+  return launch_flow<B, 0>(p, maxu, maxnb, (unsigned)warp_bytes, flowed);
 }
 
 static int check_ilu(dfm2g_ilu p, bool pattern, bool factor) {
@@ -1180,8 +1494,15 @@ int dfm2g_ilu_copy_value(dfm2g_ilu p, dfm2g_bsr m) try {
 int dfm2g_ilu_decompose(dfm2g_ilu p, int *n_singular) try {
   DFM2G_TRY(check_ilu(p, true, false));
   DFM2G_CUDA(cudaMemsetAsync(p->nsing.p, 0, sizeof(int), stream()));
+  bool flowed = false;
+  if (p->ndim == 3)
+    DFM2G_TRY(factor_flow<3>(p, &flowed));
+  else if (p->ndim == 2)
+    DFM2G_TRY(factor_flow<2>(p, &flowed));
+  else
+    DFM2G_TRY(factor_flow<1>(p, &flowed));
   const std::vector<unsigned> &ls = p->h_lstart_f;
-  for (size_t l = 0; l + 1 < ls.size(); ++l) {
+  for (size_t l = 0; !flowed && l + 1 < ls.size(); ++l) {
     const unsigned nrows = ls[l + 1] - ls[l];
     const unsigned blocks = blocks_for((size_t)nrows * 32, 256);
     if (p->ndim == 3)
@@ -1195,9 +1516,15 @@ int dfm2g_ilu_decompose(dfm2g_ilu p, int *n_singular) try {
                                                              p->dia_ind.p, p->vcrs.p, p->vdia.p, p->nsing.p);
   }
   DFM2G_LAUNCH_CHECK();
-  int ns = 0;
+  int ns = 0, e = 0;
   DFM2G_CUDA(cudaMemcpyAsync(&ns, p->nsing.p, sizeof(int), cudaMemcpyDeviceToHost, stream()));
+  if (flowed) DFM2G_CUDA(cudaMemcpyAsync(&e, p->err.p, sizeof(int), cudaMemcpyDeviceToHost, stream()));
   DFM2G_CUDA(cudaStreamSynchronize(stream()));
+  if (e != 0) {
+    DFM2G_CUDA(cudaMemsetAsync(p->err.p, 0, sizeof(int), stream()));
+    p->has_factor = false;
+    return fail(e, "decompose: device-side wait timed out");
+  }
   if (n_singular) *n_singular = ns;
   p->has_factor = true;
   p->f32_valid = false;
