@@ -420,8 +420,12 @@ struct dfm2g_tetmesh_s {
   dfm2g::DevBuf<double> xyz;
   dfm2g::DevBuf<unsigned> tet;        // ntet*4, original order
   dfm2g::DevBuf<unsigned> slot;       // ntet*16 slot ids (diagonal: 0xffffffff)
-  dfm2g::DevBuf<unsigned> by_color;   // tets sorted by colour (stable)
-  std::vector<unsigned> color_start;  // ncolor+1
+  std::vector<unsigned> color_start;  // ncolor+1 (of the node colouring, reported only)
+  dfm2g::DevBuf<double> geo;          // ntet*16: shape-function gradients, volume
+  dfm2g::DevBuf<double> stress;       // ntet*6, grown on demand
+  // gather lists (fem.cu): edges with their tets, nodes with theirs
+  unsigned nedge = 0, nedge_entries = 0, nnode_entries = 0;
+  dfm2g::DevBuf<unsigned> eslot, eoff, elist, noff, nlist;
 };
 
 namespace dfm2g {

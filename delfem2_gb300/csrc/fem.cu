@@ -1,11 +1,26 @@
-// Linear tets on the device: colour-scheduled, atomic-free assembly of the
-// elasticity K and b (3x3 blocks, per-tet Young's modulus), the adjoint element
-// term dL/dE, and the scalar Poisson K and b (1x1 blocks).
+// Linear tets on the device: atomic-free assembly of the elasticity K and b
+// (3x3 blocks, per-tet Young's modulus), of the dynamic forms, of the scalar
+// Poisson K and b (1x1 blocks), and the adjoint element term dL/dE.
 //
-// Layout: tet[4*ntet] node ids, slot[16*ntet] with slot[16e + 4a + b] the
-// val_crs_ slot of block (tet[e][a], tet[e][b]) (0xffffffff on the diagonal),
-// by_color = tets grouped by colour. Within one colour no two tets share a
-// node, so each thread (tet, node a) owns block row a of its tet exclusively.
+// The matrix is gathered, not scattered: a thread owns a pair of blocks (i, j),
+// (j, i) or a node and adds up the tets that touch it, in tet order, so each
+// block is read and written once per assembly and the sums do not depend on
+// the schedule. Lists made once per mesh: `elist` holds, edge by edge (the
+// upper slots, compacted in `eslot`, offsets `eoff`), the codes 16 e + 4 a + b
+// of the tets e with tet[e][a] = i, tet[e][b] = j; `nlist`, node by node
+// (offsets `noff`), the codes with both nodes at i (a = b, and pairs of a tet
+// that names a node twice). The tets' gradients and volume are made with them:
+// geo[16 e + 4 k .. + 3) = dN_k, geo[16 e + 3] = vol.
+//
+// With moduli in a fixed ratio the tets' blocks come from one 3x3 sum,
+// X = sum E vol dN_a dN_b^T: K_ij = lambda1 X + myu1 X^T + myu1 tr(X) I
+// (AddEmat_LinearSolid3, include/delfem2/fem_solidlinear.cpp:55-79), 13 FP64
+// operations per tet and edge where the element matrix takes 31; GB300's FP64
+// pipe bounds the assembly, with the matrix read and written once next to it.
+// 3.5M tets (96 x 95 x 64 voxels), K and b with a displacement: 1.95 ms (edges
+// 0.95, nodes 0.66, stresses 0.34); scattering the element matrices colour by
+// colour, four threads a tet and 33 launches, took 10.1 ms.
+#include <algorithm>
 #include <cstring>
 
 #include "common.cuh"
@@ -36,266 +51,486 @@ __device__ __forceinline__ double tet_geometry(const double P[4][3], double dN[4
   return vol;
 }
 
-// One thread per (tet of this colour, local node a): block row a of K_e,
-// K_e[a][b][r][c] = vol (lambda dN_a[r] dN_b[c] + myu dN_b[r] dN_a[c]
-//                        + myu (dN_a . dN_b) delta_rc)
-// (AddEmat_LinearSolid3, include/delfem2/fem_solidlinear.cpp:55-79), added into
-// the diagonal block or the mapped slot; b_i += rho g vol/4 - sum_b K_ab u_b.
-__global__ void __launch_bounds__(128) k_tet_assemble(unsigned n, const unsigned *__restrict__ list,
-                                                      const unsigned *__restrict__ tet,
-                                                      const unsigned *__restrict__ slot,
-                                                      const double *__restrict__ xyz, const double *__restrict__ young,
-                                                      double nu, double rho, double gx, double gy, double gz,
-                                                      const double *__restrict__ disp, double *vcrs, double *vdia,
-                                                      double *rhs) {
-  const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n * 4u) return;
-  const unsigned e = list[t >> 2], a = t & 3u;
-  unsigned nd[4];
-  double P[4][3];
+// ---- the gather lists ---------------------------------------------------------
+__global__ void k_tet_geo(size_t ntet, const unsigned *__restrict__ tet, const double *__restrict__ xyz,
+                          double *__restrict__ geo) {
+  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < ntet; e += (size_t)gridDim.x * blockDim.x) {
+    double P[4][3], dN[4][3];
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    nd[k] = tet[(size_t)e * 4 + k];
+    for (int k = 0; k < 4; ++k)
 #pragma unroll
-    for (int d = 0; d < 3; ++d) P[k][d] = xyz[(size_t)nd[k] * 3 + d];
-  }
-  double dN[4][3];
-  const double vol = tet_geometry(P, dN);
-  const double E = young[e];
-  const double lam = E * nu / ((1.0 + nu) * (1.0 - 2.0 * nu));
-  const double myu = E / (2.0 * (1.0 + nu));
-  const unsigned i = nd[a];
-  double res[3] = {vol * rho * gx * 0.25, vol * rho * gy * 0.25, vol * rho * gz * 0.25};
-  double da[3];
+      for (int d = 0; d < 3; ++d) P[k][d] = xyz[(size_t)tet[e * 4 + k] * 3 + d];
+    const double vol = tet_geometry(P, dN);
+    double2 *g = reinterpret_cast<double2 *>(geo + e * 16);
 #pragma unroll
-  for (int d = 0; d < 3; ++d) da[d] = (a == 0) ? dN[0][d] : (a == 1) ? dN[1][d] : (a == 2) ? dN[2][d] : dN[3][d];
-#pragma unroll
-  for (int b = 0; b < 4; ++b) {
-    const double dd = da[0] * dN[b][0] + da[1] * dN[b][1] + da[2] * dN[b][2];
-    double k[9];
-#pragma unroll
-    for (int r = 0; r < 3; ++r)
-#pragma unroll
-      for (int c = 0; c < 3; ++c)
-        k[r * 3 + c] = vol * (lam * da[r] * dN[b][c] + myu * dN[b][r] * da[c] + (r == c ? myu * dd : 0.0));
-    if (disp) {
-      const double *u = disp + (size_t)nd[b] * 3;
-#pragma unroll
-      for (int r = 0; r < 3; ++r) res[r] -= k[r * 3 + 0] * u[0] + k[r * 3 + 1] * u[1] + k[r * 3 + 2] * u[2];
+    for (int k = 0; k < 4; ++k) {
+      g[2 * k] = make_double2(dN[k][0], dN[k][1]);
+      g[2 * k + 1] = make_double2(dN[k][2], k == 0 ? vol : 0.0);
     }
-    const unsigned s = slot[(size_t)e * 16 + a * 4 + b];
-    double *dst = (s == kDiagSlot) ? vdia + (size_t)i * 9 : vcrs + (size_t)s * 9;
-#pragma unroll
-    for (int q = 0; q < 9; ++q) dst[q] += k[q];
   }
-#pragma unroll
-  for (int r = 0; r < 3; ++r) rhs[(size_t)i * 3 + r] += res[r];
 }
 
-// One thread per (tet of this colour, local node a): row a of the scalar
-// element matrix of EMat_Poisson_Tet3D (include/delfem2/fem_poisson.cpp:
-// 163-194), K_e[a][b] = alpha vol (dN_a . dN_b), added to the diagonal (the
-// (a, a) entry when both nodes are one block, as the reference's Merge does)
-// or to the mapped slot; b_i += source vol / 4 - sum_b K_ab val_b.
-__global__ void __launch_bounds__(128) k_tet_poisson(unsigned n, const unsigned *__restrict__ list,
-                                                     const unsigned *__restrict__ tet,
-                                                     const unsigned *__restrict__ slot,
-                                                     const double *__restrict__ xyz, double alpha, double source,
-                                                     const double *__restrict__ val, double *vcrs, double *vdia,
-                                                     double *rhs) {
-  const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n * 4u) return;
-  const unsigned e = list[t >> 2], a = t & 3u;
-  unsigned nd[4];
-  double P[4][3];
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    nd[k] = tet[(size_t)e * 4 + k];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) P[k][d] = xyz[(size_t)nd[k] * 3 + d];
+// Counts (fill = 0) or writes (fill = 1) the list entries of every (tet, a, b):
+// edges by their upper slot, node entries by node.
+__global__ void k_tet_lists(size_t ntet, const unsigned *__restrict__ tet, const unsigned *__restrict__ slot, int fill,
+                            unsigned *edge_at, unsigned *node_at, unsigned *__restrict__ elist,
+                            unsigned *__restrict__ nlist) {
+  for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < ntet * 16;
+       k += (size_t)gridDim.x * blockDim.x) {
+    const size_t e = k >> 4;
+    const unsigned i = tet[e * 4 + ((k >> 2) & 3)], j = tet[e * 4 + (k & 3)], s = slot[k];
+    if (s == kDiagSlot) {
+      const unsigned at = atomicAdd(node_at + i, 1u);
+      if (fill) nlist[at] = (unsigned)k;
+    } else if (i < j) {
+      const unsigned at = atomicAdd(edge_at + s, 1u);
+      if (fill) elist[at] = (unsigned)k;
+    }
   }
-  double dN[4][3];
-  const double vol = tet_geometry(P, dN);
-  double da[3];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) da[d] = (a == 0) ? dN[0][d] : (a == 1) ? dN[1][d] : (a == 2) ? dN[2][d] : dN[3][d];
-  const double kaa = alpha * vol * (da[0] * da[0] + da[1] * da[1] + da[2] * da[2]);
-  const unsigned i = nd[a];
-  double res = source * vol * 0.25;
-#pragma unroll
-  for (int b = 0; b < 4; ++b) {
-    const double k = alpha * vol * (da[0] * dN[b][0] + da[1] * dN[b][1] + da[2] * dN[b][2]);
-    if (val) res -= k * val[nd[b]];
-    const unsigned s = slot[(size_t)e * 16 + a * 4 + b];
-    if (s == kDiagSlot)
-      vdia[i] += kaa;
-    else
-      vcrs[s] += k;
-  }
-  rhs[i] += res;
 }
 
-// Row a of the dynamic linear-tet element matrices (3x3 blocks), one thread
-// per (tet of this colour, local node a), K_ab as in k_tet_assemble
-// (SetEmat_LinearSolid3<4>, include/delfem2/fem_solidlinear.h:128-153):
-//  kBEuler: MergeLinSys_SolidLinear_BEuler_MeshTet3D (fem_solidlinear.h:
-//    381-443): r_a = vol rho g/4 - sum_b K_ab (u_b + dt v_b); E_ab = K_ab +
-//    rho vol/(4 dt^2) I [a == b]; b_i += r_a / dt.
-//  kWarp: MergeLinSys_SolidStiffwarp_BEuler_MeshTet3D (445-530): the same
-//    with K_ab <- R_a K_ab R_a^T and u_b + dt v_b <- P_b + u_b + dt v_b -
-//    R_a P_b (R_a = rot of node i, row-major).
-//  kNewmark: MergeLinSys_SolidLinear_NewmarkBeta_MeshTet3D (331-379, with
-//    EMat_SolidLinear_NewmarkBeta_MeshTet3D, fem_solidlinear.cpp:437-488,
-//    first iteration): M_ab = rho vol/20 (1 + [a == b]) I, E_ab = M_ab +
-//    beta dt^2 K_ab, r_a = vol rho g/4 - K u - M acc - dt K v - dt^2/2 K acc
-//    (summed in that order); b_i += r_a.
-// E_ab goes to the diagonal (the (a, a) block when both nodes are one block,
-// as the reference's Merge does) or to the mapped slot.
-enum { kBEuler = 0, kWarp = 1, kNewmark = 2 };
+// Exclusive scan of a[0, n) in tiles of kScanTile: tile sums, their scan by one
+// block, and the tiles' own scans on top. `flag` scans (a[k] > 0) instead.
+constexpr unsigned kScanTile = 2048;
 
+__global__ void __launch_bounds__(256) k_scan_tile(const unsigned *__restrict__ a, unsigned n, int flag,
+                                                   const unsigned *__restrict__ base, unsigned *__restrict__ out,
+                                                   unsigned *__restrict__ sums) {
+  __shared__ unsigned sh[8];
+  const unsigned lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
+  const size_t k0 = (size_t)blockIdx.x * kScanTile + threadIdx.x * 8u;
+  unsigned v[8], t = 0;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const unsigned x = k0 + q < n ? a[k0 + q] : 0u;
+    v[q] = t;
+    t += flag ? (x > 0u) : x;
+  }
+  unsigned x = t;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= (unsigned)o) x += y;
+  }
+  if (lane == 31) sh[w] = x;
+  __syncthreads();
+  unsigned before = 0, all = 0;
+  for (unsigned q = 0; q < 8; ++q) {
+    if (q < w) before += sh[q];
+    all += sh[q];
+  }
+  if (!out) {
+    if (threadIdx.x == 0) sums[blockIdx.x] = all;
+    return;
+  }
+  const unsigned off = base[blockIdx.x] + before + x - t;
+#pragma unroll
+  for (int q = 0; q < 8; ++q)
+    if (k0 + q < n) out[k0 + q] = off + v[q];
+}
+
+__global__ void __launch_bounds__(1024) k_scan_sums(unsigned *sums, unsigned n, unsigned *total) {
+  __shared__ unsigned sh[32];
+  __shared__ unsigned carry;
+  const unsigned lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
+  if (threadIdx.x == 0) carry = 0;
+  __syncthreads();
+  for (unsigned k0 = 0; k0 < n; k0 += 1024) {
+    const unsigned k = k0 + threadIdx.x, v = k < n ? sums[k] : 0u;
+    unsigned x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= (unsigned)o) x += y;
+    }
+    if (lane == 31) sh[w] = x;
+    __syncthreads();
+    unsigned before = carry, all = 0;
+    for (unsigned q = 0; q < 32; ++q) {
+      if (q < w) before += sh[q];
+      all += sh[q];
+    }
+    if (k < n) sums[k] = before + x - v;
+    __syncthreads();
+    if (threadIdx.x == 0) carry += all;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) *total = carry;
+}
+
+// Edges with tets, compacted: eslot (their upper slot) and eoff (their first
+// list entry); at[s]: the slot's first entry, rank[s]: its number among them.
+__global__ void k_tet_edges_compact(unsigned nnz, const unsigned *__restrict__ count, const unsigned *__restrict__ at,
+                                    const unsigned *__restrict__ rank, unsigned *__restrict__ eslot,
+                                    unsigned *__restrict__ eoff) {
+  for (unsigned s = blockIdx.x * blockDim.x + threadIdx.x; s < nnz; s += gridDim.x * blockDim.x) {
+    if (count[s] == 0) continue;
+    eslot[rank[s]] = s;
+    eoff[rank[s]] = at[s];
+  }
+}
+
+// Each list in ascending order (the fill's order is not deterministic).
+__global__ void k_sort_lists(unsigned n, const unsigned *__restrict__ off, unsigned total, unsigned *list) {
+  for (unsigned k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+    const unsigned b = off[k], e = k + 1 < n ? off[k + 1] : total;
+    for (unsigned p = b + 1; p < e; ++p) {
+      const unsigned v = list[p];
+      unsigned q = p;
+      while (q > b && list[q - 1] > v) {
+        list[q] = list[q - 1];
+        --q;
+      }
+      list[q] = v;
+    }
+  }
+}
+
+// ---- assembly -------------------------------------------------------------------
+// Modes: kStatic: moduli E_e (lambda1, myu1), b_i += rho g vol/4 - (K u)_i
+// (fem_solidlinear.h:192-237). kBEuler: MergeLinSys_SolidLinear_BEuler_MeshTet3D
+// (fem_solidlinear.h:381-443): E = K + rho vol/(4 dt^2) I on the diagonal,
+// b += (rho g vol/4 - K (u + dt v)) / dt. kWarp:
+// MergeLinSys_SolidStiffwarp_BEuler_MeshTet3D (445-530): the same with
+// K_ij <- R_i K_ij R_i^T and u_j + dt v_j <- P_j + u_j + dt v_j - R_i P_j (R_i =
+// rot of node i, row-major). kNewmark:
+// MergeLinSys_SolidLinear_NewmarkBeta_MeshTet3D (331-379, with
+// EMat_SolidLinear_NewmarkBeta_MeshTet3D, fem_solidlinear.cpp:437-488, first
+// iteration): M_ij = rho vol/20 (1 + [i == j]) I, E = M + beta dt^2 K,
+// b += rho g vol/4 - K (u + dt v + dt^2/2 acc) - M acc.
+enum { kStatic = 0, kBEuler = 1, kWarp = 2, kNewmark = 3 };
+
+struct TetParam {
+  double lam, myu;            // of unit modulus (kStatic) or the material's
+  double rho, g[3], dt, beta;
+  const double *young;        // kStatic: per tet
+  const double *rot, *acc;    // kWarp, kNewmark
+  const double *disp, *velo;  // dynamic modes; kStatic: disp or null
+};
+
+__device__ __forceinline__ void tet_grad(const double *__restrict__ geo, unsigned e, unsigned a, double d[3],
+                                         double *vol) {
+  const double2 *g = reinterpret_cast<const double2 *>(geo + (size_t)e * 16);
+  const double2 xy = __ldg(g + 2 * a), zv = __ldg(g + 2 * a + 1);
+  d[0] = xy.x;
+  d[1] = xy.y;
+  d[2] = zv.x;
+  *vol = a == 0 ? zv.y : __ldg(geo + (size_t)e * 16 + 3);
+}
+
+// K_ij of the summed X (see above).
+__device__ __forceinline__ void tet_block(const double X[9], double lam, double myu, double k[9]) {
+  const double d = myu * (X[0] + X[4] + X[8]);
+#pragma unroll
+  for (int r = 0; r < 3; ++r)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) k[r * 3 + c] = lam * X[r * 3 + c] + myu * X[c * 3 + r] + (r == c ? d : 0.0);
+}
+
+__device__ __forceinline__ void rotate_block(const double R[9], double k[9]) {  // k <- R k R^T
+  double t[9];
+#pragma unroll
+  for (int r = 0; r < 3; ++r)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) t[r * 3 + c] = k[r * 3] * R[c * 3] + k[r * 3 + 1] * R[c * 3 + 1] + k[r * 3 + 2] * R[c * 3 + 2];
+#pragma unroll
+  for (int r = 0; r < 3; ++r)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) k[r * 3 + c] = R[r * 3] * t[c] + R[r * 3 + 1] * t[3 + c] + R[r * 3 + 2] * t[6 + c];
+}
+
+// One thread per edge: the blocks (i, j) and (j, i).
 template <int MODE>
-__global__ void __launch_bounds__(128) k_tet_dynamic(unsigned n, const unsigned *__restrict__ list,
-                                                     const unsigned *__restrict__ tet,
-                                                     const unsigned *__restrict__ slot,
-                                                     const double *__restrict__ xyz, double myu, double lam,
-                                                     double rho, double gx, double gy, double gz, double dt,
-                                                     double beta, const double *__restrict__ disp,
-                                                     const double *__restrict__ velo,
-                                                     const double *__restrict__ acc_or_rot, double *vcrs,
-                                                     double *vdia, double *rhs) {
-  const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n * 4u) return;
-  const unsigned e = list[t >> 2], a = t & 3u;
-  unsigned nd[4];
-  double P[4][3];
+__global__ void __launch_bounds__(128) k_tet_edges(unsigned nedge, const unsigned *__restrict__ eslot,
+                                                   const unsigned *__restrict__ eoff, unsigned total,
+                                                   const unsigned *__restrict__ elist,
+                                                   const unsigned *__restrict__ slot,
+                                                   const unsigned *__restrict__ tet, const double *__restrict__ geo,
+                                                   const TetParam p, double *vcrs) {
+  const unsigned k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= nedge) return;
+  const unsigned l0 = eoff[k], l1 = k + 1 < nedge ? eoff[k + 1] : total;
+  double X[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, vsum = 0.0;
+  unsigned code = 0;
+  for (unsigned l = l0; l < l1; ++l) {
+    code = elist[l];
+    const unsigned e = code >> 4;
+    double a[3], b[3], vol;
+    tet_grad(geo, e, (code >> 2) & 3u, a, &vol);
+    tet_grad(geo, e, code & 3u, b, &vol);
+    const double w = MODE == kStatic ? p.young[e] * vol : vol;
+    if (MODE == kNewmark) vsum += vol;
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    nd[k] = tet[(size_t)e * 4 + k];
+    for (int r = 0; r < 3; ++r) {
+      const double wa = w * a[r];
 #pragma unroll
-    for (int d = 0; d < 3; ++d) P[k][d] = xyz[(size_t)nd[k] * 3 + d];
+      for (int c = 0; c < 3; ++c) X[r * 3 + c] += wa * b[c];
+    }
   }
-  double dN[4][3];
-  const double vol = tet_geometry(P, dN);
-  double da[3];
+  double kij[9], kji[9];
+  tet_block(X, p.lam, p.myu, kij);
+  if (MODE == kNewmark) {
+    const double s = p.beta * p.dt * p.dt, m = p.rho * vsum * 0.05;
 #pragma unroll
-  for (int d = 0; d < 3; ++d) da[d] = (a == 0) ? dN[0][d] : (a == 1) ? dN[1][d] : (a == 2) ? dN[2][d] : dN[3][d];
-  const unsigned i = nd[a];
-  double R[9];
-  if constexpr (MODE == kWarp) {
-#pragma unroll
-    for (int q = 0; q < 9; ++q) R[q] = acc_or_rot[(size_t)i * 9 + q];
+    for (int q = 0; q < 9; ++q) kij[q] = (q % 4 == 0 ? m : 0.0) + s * kij[q];
   }
-  // K_ab (warped for kWarp)
-  auto kblock = [&](int b, double k[9]) {
-    const double dd = da[0] * dN[b][0] + da[1] * dN[b][1] + da[2] * dN[b][2];
 #pragma unroll
-    for (int r = 0; r < 3; ++r)
+  for (int r = 0; r < 3; ++r)
 #pragma unroll
-      for (int c = 0; c < 3; ++c)
-        k[r * 3 + c] = vol * (lam * da[r] * dN[b][c] + myu * dN[b][r] * da[c] + (r == c ? myu * dd : 0.0));
-    if constexpr (MODE == kWarp) {
-      double tmp[9];
+    for (int c = 0; c < 3; ++c) kji[r * 3 + c] = kij[c * 3 + r];
+  const unsigned e = code >> 4, a = (code >> 2) & 3u, b = code & 3u;
+  if (MODE == kWarp) {
+    double R[9];
+    const double *Ri = p.rot + (size_t)tet[(size_t)e * 4 + a] * 9, *Rj = p.rot + (size_t)tet[(size_t)e * 4 + b] * 9;
 #pragma unroll
-      for (int r = 0; r < 3; ++r)
+    for (int q = 0; q < 9; ++q) R[q] = Ri[q];
+    rotate_block(R, kij);
 #pragma unroll
-        for (int c = 0; c < 3; ++c)
-          tmp[r * 3 + c] = k[r * 3 + 0] * R[c * 3 + 0] + k[r * 3 + 1] * R[c * 3 + 1] + k[r * 3 + 2] * R[c * 3 + 2];
+    for (int q = 0; q < 9; ++q) R[q] = Rj[q];
+    rotate_block(R, kji);
+  }
+  double *up = vcrs + (size_t)eslot[k] * 9, *lo = vcrs + (size_t)slot[(size_t)e * 16 + b * 4 + a] * 9;
 #pragma unroll
-      for (int r = 0; r < 3; ++r)
+  for (int q = 0; q < 9; ++q) up[q] += kij[q];
 #pragma unroll
-        for (int c = 0; c < 3; ++c)
-          k[r * 3 + c] = R[r * 3 + 0] * tmp[0 * 3 + c] + R[r * 3 + 1] * tmp[1 * 3 + c] + R[r * 3 + 2] * tmp[2 * 3 + c];
-    }
-  };
-  // E_ab, the block that is merged
-  const double mass = (MODE == kNewmark) ? rho * vol * 0.05 : rho * vol * 0.25 / (dt * dt);
-  auto eblock = [&](int b, double k[9]) {
-    kblock(b, k);
-    if constexpr (MODE == kNewmark) {
-      const double bdt2 = beta * dt * dt;
-      const double m = (b == (int)a) ? mass + mass : mass;
+  for (int q = 0; q < 9; ++q) lo[q] += kji[q];
+}
+
+// S = vol (lam tr(G) I + myu (G + G^T)), G = sum_b w_b dN_b^T: the nodal forces
+// K_e w are S dN_a. Stored as {xx, yy, zz, xy, yz, zx}.
+__device__ __forceinline__ void tet_stress(const double G[9], double lam, double myu, double S[6]) {
+  const double t = lam * (G[0] + G[4] + G[8]);
+  S[0] = t + 2.0 * myu * G[0];
+  S[1] = t + 2.0 * myu * G[4];
+  S[2] = t + 2.0 * myu * G[8];
+  S[3] = myu * (G[1] + G[3]);
+  S[4] = myu * (G[5] + G[7]);
+  S[5] = myu * (G[6] + G[2]);
+}
+
+// One thread per tet: S of w = u (kStatic), u + dt v (kBEuler), u + dt v + dt^2/2 acc (kNewmark).
+template <int MODE>
+__global__ void __launch_bounds__(128) k_tet_stress(size_t ntet, const unsigned *__restrict__ tet,
+                                                    const double *__restrict__ geo, const TetParam p,
+                                                    double *__restrict__ stress) {
+  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < ntet; e += (size_t)gridDim.x * blockDim.x) {
+    double G[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, vol = 0.0;
 #pragma unroll
-      for (int q = 0; q < 9; ++q) k[q] = ((q % 4 == 0) ? m : 0.0) + bdt2 * k[q];
-    } else {
-      if (b == (int)a) {
-        k[0] += mass;
-        k[4] += mass;
-        k[8] += mass;
-      }
-    }
-  };
-  double res[3] = {vol * rho * gx * 0.25, vol * rho * gy * 0.25, vol * rho * gz * 0.25};
-  if constexpr (MODE == kNewmark) {
-    // (matrix, vector, scale): (K, u, -1), (M, acc, -1), (K, v, -dt), (K, acc, -dt^2/2)
-#pragma unroll
-    for (int pass = 0; pass < 4; ++pass) {
-      const double *vec = pass == 0 ? disp : (pass == 2 ? velo : acc_or_rot);
-      const double sc = pass == 2 ? -dt : (pass == 3 ? -0.5 * dt * dt : -1.0);
-#pragma unroll
-      for (int b = 0; b < 4; ++b) {
-        const double *x = vec + (size_t)nd[b] * 3;
-        if (pass == 1) {
-          const double m = (b == (int)a) ? mass + mass : mass;
-#pragma unroll
-          for (int r = 0; r < 3; ++r) res[r] += sc * (m * x[r]);
-        } else {
-          double k[9];
-          kblock(b, k);
-#pragma unroll
-          for (int r = 0; r < 3; ++r) res[r] += sc * (k[r * 3 + 0] * x[0] + k[r * 3 + 1] * x[1] + k[r * 3 + 2] * x[2]);
-        }
-      }
-    }
-  } else {
-#pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      double k[9], w[3];
-      kblock(b, k);
-      const double *u = disp + (size_t)nd[b] * 3, *v = velo + (size_t)nd[b] * 3;
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        if constexpr (MODE == kWarp)
-          w[d] = P[b][d] + u[d] + dt * v[d] - (R[d * 3 + 0] * P[b][0] + R[d * 3 + 1] * P[b][1] + R[d * 3 + 2] * P[b][2]);
-        else
-          w[d] = u[d] + dt * v[d];
-      }
+    for (unsigned b = 0; b < 4; ++b) {
+      const size_t n = (size_t)tet[e * 4 + b] * 3;
+      double d[3], v;
+      tet_grad(geo, (unsigned)e, b, d, &v);
+      if (b == 0) vol = v;
 #pragma unroll
       for (int r = 0; r < 3; ++r) {
-        res[r] -= k[r * 3 + 0] * w[0];
-        res[r] -= k[r * 3 + 1] * w[1];
-        res[r] -= k[r * 3 + 2] * w[2];
+        double w = p.disp[n + r];
+        if (MODE != kStatic) w += p.dt * p.velo[n + r];
+        if (MODE == kNewmark) w += 0.5 * p.dt * p.dt * p.acc[n + r];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) G[r * 3 + c] += w * d[c];
+      }
+    }
+    const double w = MODE == kStatic ? p.young[e] * vol : vol;
+    double S[6];
+    tet_stress(G, w * p.lam, w * p.myu, S);
+    double2 *o = reinterpret_cast<double2 *>(stress + e * 6);
+    o[0] = make_double2(S[0], S[1]);
+    o[1] = make_double2(S[2], S[3]);
+    o[2] = make_double2(S[4], S[5]);
+  }
+}
+
+// One thread per node: the diagonal block and the right-hand side.
+template <int MODE>
+__global__ void __launch_bounds__(128) k_tet_nodes(unsigned np, const unsigned *__restrict__ noff, unsigned total,
+                                                   const unsigned *__restrict__ nlist,
+                                                   const unsigned *__restrict__ tet, const double *__restrict__ xyz,
+                                                   const double *__restrict__ geo,
+                                                   const double *__restrict__ stress, const TetParam p, double *vdia,
+                                                   double *rhs) {
+  const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= np) return;
+  const unsigned l0 = noff[i], l1 = i + 1 < np ? noff[i + 1] : total;
+  if (l0 == l1) return;
+  double X[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, vsum = 0.0, vmass = 0.0, f[3] = {0, 0, 0}, macc[3] = {0, 0, 0};
+  double skew[3] = {0, 0, 0};
+  double R[9];
+  if (MODE == kWarp) {
+#pragma unroll
+    for (int q = 0; q < 9; ++q) R[q] = p.rot[(size_t)i * 9 + q];
+  }
+  for (unsigned l = l0; l < l1; ++l) {
+    const unsigned code = nlist[l], e = code >> 4, ia = (code >> 2) & 3u, ib = code & 3u;
+    double a[3], vol;
+    tet_grad(geo, e, ia, a, &vol);
+    const double w = MODE == kStatic ? p.young[e] * vol : vol;
+    double b[3] = {a[0], a[1], a[2]};
+    // a tet that names the node twice: K_ab joins the diagonal (kStatic), or the
+    // (a, a) block once more (the dynamic forms), as the reference's Merge does
+    if (ia != ib && MODE == kStatic) tet_grad(geo, e, ib, b, &vol);
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      const double wa = w * a[r];
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+        if (c >= r) X[r * 3 + c] += wa * b[c];
+    }
+    if (MODE == kStatic && ia != ib) {  // the lower part's excess over the upper one
+      skew[0] += w * (a[1] * b[0] - a[0] * b[1]);
+      skew[1] += w * (a[2] * b[0] - a[0] * b[2]);
+      skew[2] += w * (a[2] * b[1] - a[1] * b[2]);
+    }
+    vmass += vol;
+    if (ia != ib) continue;
+    vsum += vol;
+    if (MODE == kWarp) {
+      double G[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll
+      for (unsigned q = 0; q < 4; ++q) {
+        const size_t n = (size_t)tet[(size_t)e * 4 + q] * 3;
+        double d[3], v, x[3], P[3];
+        tet_grad(geo, e, q, d, &v);
+#pragma unroll
+        for (int r = 0; r < 3; ++r) P[r] = xyz[n + r];
+#pragma unroll
+        for (int r = 0; r < 3; ++r)
+          x[r] = P[r] + p.disp[n + r] + p.dt * p.velo[n + r] -
+                 (R[r * 3] * P[0] + R[r * 3 + 1] * P[1] + R[r * 3 + 2] * P[2]);
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+          const double y = R[r] * x[0] + R[3 + r] * x[1] + R[6 + r] * x[2];  // R^T (P + u + dt v - R P)
+#pragma unroll
+          for (int c = 0; c < 3; ++c) G[r * 3 + c] += y * d[c];
+        }
+      }
+      double S[6];
+      tet_stress(G, vol * p.lam, vol * p.myu, S);
+      f[0] += S[0] * a[0] + S[3] * a[1] + S[5] * a[2];
+      f[1] += S[3] * a[0] + S[1] * a[1] + S[4] * a[2];
+      f[2] += S[5] * a[0] + S[4] * a[1] + S[2] * a[2];
+    } else if (stress) {
+      const double2 *o = reinterpret_cast<const double2 *>(stress + (size_t)e * 6);
+      const double2 s0 = __ldg(o), s1 = __ldg(o + 1), s2 = __ldg(o + 2);
+      f[0] += s0.x * a[0] + s1.y * a[1] + s2.y * a[2];
+      f[1] += s1.y * a[0] + s0.y * a[1] + s2.x * a[2];
+      f[2] += s2.y * a[0] + s2.x * a[1] + s1.x * a[2];
+    }
+    if (MODE == kNewmark) {
+#pragma unroll
+      for (unsigned q = 0; q < 4; ++q) {
+        const double *x = p.acc + (size_t)tet[(size_t)e * 4 + q] * 3;
+        const double m = q == ia ? 2.0 * vol : vol;
+#pragma unroll
+        for (int r = 0; r < 3; ++r) macc[r] += m * x[r];
       }
     }
   }
+  X[3] = X[1] + skew[0];
+  X[6] = X[2] + skew[1];
+  X[7] = X[5] + skew[2];
+  double k[9];
+  tet_block(X, p.lam, p.myu, k);
+  if (MODE == kWarp) rotate_block(R, k);
+  double m = 0.0;
+  if (MODE == kBEuler || MODE == kWarp) m = p.rho * vmass * 0.25 / (p.dt * p.dt);
+  if (MODE == kNewmark) {
+    const double s = p.beta * p.dt * p.dt;
 #pragma unroll
-  for (int b = 0; b < 4; ++b) {
-    const unsigned s = slot[(size_t)e * 16 + a * 4 + b];
-    double k[9];
-    eblock(s == kDiagSlot ? (int)a : b, k);
-    double *dst = (s == kDiagSlot) ? vdia + (size_t)i * 9 : vcrs + (size_t)s * 9;
+    for (int q = 0; q < 9; ++q) k[q] *= s;
+    m = p.rho * vmass * 0.1;
+  }
+  double *dst = vdia + (size_t)i * 9;
 #pragma unroll
-    for (int q = 0; q < 9; ++q) dst[q] += k[q];
+  for (int q = 0; q < 9; ++q) dst[q] += k[q] + (q % 4 == 0 ? m : 0.0);
+  if (MODE == kWarp) {
+    const double t0 = f[0], t1 = f[1], t2 = f[2];
+#pragma unroll
+    for (int r = 0; r < 3; ++r) f[r] = R[r * 3] * t0 + R[r * 3 + 1] * t1 + R[r * 3 + 2] * t2;
   }
 #pragma unroll
-  for (int r = 0; r < 3; ++r) rhs[(size_t)i * 3 + r] += (MODE == kNewmark) ? res[r] : res[r] / dt;
+  for (int r = 0; r < 3; ++r) {
+    double q = vsum * p.rho * p.g[r] * 0.25 - f[r];
+    if (MODE == kNewmark) q -= p.rho * 0.05 * macc[r];
+    if (MODE == kBEuler || MODE == kWarp) q /= p.dt;
+    rhs[(size_t)i * 3 + r] += q;
+  }
+}
+
+// The scalar matrix of EMat_Poisson_Tet3D (include/delfem2/fem_poisson.cpp:
+// 163-194), K_e[a][b] = alpha vol (dN_a . dN_b): one thread per edge, and per
+// node (b_i += source vol/4 - sum_b K_ab val_b; a pair of a tet that names a
+// node twice adds the (a, a) entry again, as the reference's Merge does).
+__global__ void __launch_bounds__(128) k_poisson_edges(unsigned nedge, const unsigned *__restrict__ eslot,
+                                                       const unsigned *__restrict__ eoff, unsigned total,
+                                                       const unsigned *__restrict__ elist,
+                                                       const unsigned *__restrict__ slot,
+                                                       const double *__restrict__ geo, double alpha, double *vcrs) {
+  const unsigned k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= nedge) return;
+  const unsigned l0 = eoff[k], l1 = k + 1 < nedge ? eoff[k + 1] : total;
+  double x = 0.0;
+  unsigned code = 0;
+  for (unsigned l = l0; l < l1; ++l) {
+    code = elist[l];
+    double a[3], b[3], vol;
+    tet_grad(geo, code >> 4, (code >> 2) & 3u, a, &vol);
+    tet_grad(geo, code >> 4, code & 3u, b, &vol);
+    x += vol * (a[0] * b[0] + a[1] * b[1] + a[2] * b[2]);
+  }
+  x *= alpha;
+  vcrs[eslot[k]] += x;
+  vcrs[slot[(size_t)(code >> 4) * 16 + (code & 3u) * 4 + ((code >> 2) & 3u)]] += x;
+}
+
+__global__ void __launch_bounds__(128) k_poisson_nodes(unsigned np, const unsigned *__restrict__ noff, unsigned total,
+                                                       const unsigned *__restrict__ nlist,
+                                                       const unsigned *__restrict__ tet,
+                                                       const double *__restrict__ geo, double alpha, double source,
+                                                       const double *__restrict__ val, double *vdia, double *rhs) {
+  const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= np) return;
+  const unsigned l0 = noff[i], l1 = i + 1 < np ? noff[i + 1] : total;
+  if (l0 == l1) return;
+  double x = 0.0, res = 0.0, vsum = 0.0;
+  for (unsigned l = l0; l < l1; ++l) {
+    const unsigned code = nlist[l], e = code >> 4, ia = (code >> 2) & 3u;
+    double a[3], vol;
+    tet_grad(geo, e, ia, a, &vol);
+    x += vol * (a[0] * a[0] + a[1] * a[1] + a[2] * a[2]);
+    if (ia != (code & 3u)) continue;
+    vsum += vol;
+    if (val) {
+      double g[3] = {0, 0, 0};
+#pragma unroll
+      for (unsigned q = 0; q < 4; ++q) {
+        const double u = val[tet[(size_t)e * 4 + q]];
+        double d[3], v;
+        tet_grad(geo, e, q, d, &v);
+#pragma unroll
+        for (int r = 0; r < 3; ++r) g[r] += u * d[r];
+      }
+      res += vol * (a[0] * g[0] + a[1] * g[1] + a[2] * g[2]);
+    }
+  }
+  vdia[i] += alpha * x;
+  rhs[i] += source * vsum * 0.25 - alpha * res;
 }
 
 // dL/dE_e = -lam_e^T (K_e / E_e) u_e with G(v)[r][c] = sum_k v_k[r] dN_k[c]:
 // lam^T K_e u = vol (lambda1 tr(GL) tr(GU) + myu1 (tr(GL GU) + GL:GU)),
 // lambda1 = nu/((1+nu)(1-2nu)), myu1 = 1/(2(1+nu)) (the moduli at E = 1).
-__global__ void k_tet_dLdE(size_t ntet, const unsigned *__restrict__ tet, const double *__restrict__ xyz, double nu,
+__global__ void k_tet_dLdE(size_t ntet, const unsigned *__restrict__ tet, const double *__restrict__ geo, double nu,
                            const double *__restrict__ u, const double *__restrict__ lamv, double *__restrict__ out) {
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < ntet; e += (size_t)gridDim.x * blockDim.x) {
     unsigned nd[4];
-    double P[4][3];
+    double dN[4][3], vol = 0.0;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
+      double v;
       nd[k] = tet[e * 4 + k];
-#pragma unroll
-      for (int d = 0; d < 3; ++d) P[k][d] = xyz[(size_t)nd[k] * 3 + d];
+      tet_grad(geo, (unsigned)e, k, dN[k], &v);
+      if (k == 0) vol = v;
     }
-    double dN[4][3];
-    const double vol = tet_geometry(P, dN);
     double GL[3][3] = {{0}}, GU[3][3] = {{0}};
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -327,6 +562,82 @@ __global__ void k_tet_dLdE(size_t ntet, const unsigned *__restrict__ tet, const 
 
 using namespace dfm2g;
 
+static int scan_exclusive(const unsigned *a, unsigned n, int flag, unsigned *out, unsigned *sums, unsigned *total) {
+  const unsigned tiles = (n + kScanTile - 1) / kScanTile;
+  k_scan_tile<<<tiles, 256, 0, stream()>>>(a, n, flag, nullptr, nullptr, sums);
+  k_scan_sums<<<1, 1024, 0, stream()>>>(sums, tiles, total);
+  k_scan_tile<<<tiles, 256, 0, stream()>>>(a, n, flag, sums, out, nullptr);
+  note_launches(3);
+  DFM2G_LAUNCH_CHECK();
+  return DFM2G_OK;
+}
+
+// The gather lists and the tets' geometry (see the top of the file).
+static int tet_lists_build(dfm2g_tetmesh_s *t, const dfm2g_bsr_s *m) {
+  const unsigned np = (unsigned)t->np, nnz = (unsigned)m->nnz;
+  DFM2G_TRY(t->geo.resize(t->ntet * 16 + 2));
+  DFM2G_TRY(t->noff.resize(np + 1));
+  if (t->ntet == 0) return DFM2G_OK;
+  const unsigned grid = ctx().num_sms * 16;
+  k_tet_geo<<<grid, 256, 0, stream()>>>(t->ntet, t->tet.p, t->xyz.p, t->geo.p);
+  // scratch: counts, first entries and ranks of the slots, counts of the nodes, tile sums, three totals
+  const size_t most = std::max((size_t)nnz, (size_t)np);
+  DevBuf<unsigned> tmp;
+  DFM2G_TRY(tmp.resize(3 * (size_t)nnz + np + most / kScanTile + 8));
+  unsigned *count = tmp.p, *ncount = count + nnz, *at = ncount + np, *rank = at + nnz, *totals = rank + nnz,
+           *sums = totals + 3;
+  DFM2G_CUDA(cudaMemsetAsync(count, 0, sizeof(unsigned) * ((size_t)nnz + np), stream()));
+  DFM2G_CUDA(cudaMemsetAsync(totals, 0, sizeof(unsigned) * 3, stream()));
+  k_tet_lists<<<grid, 256, 0, stream()>>>(t->ntet, t->tet.p, t->slot.p, 0, count, ncount, nullptr, nullptr);
+  DFM2G_TRY(scan_exclusive(ncount, np, 0, t->noff.p, sums, totals));
+  if (nnz) {
+    DFM2G_TRY(scan_exclusive(count, nnz, 1, rank, sums, totals + 1));
+    DFM2G_TRY(scan_exclusive(count, nnz, 0, at, sums, totals + 2));
+  }
+  unsigned h[3];
+  DFM2G_CUDA(cudaMemcpyAsync(h, totals, sizeof(h), cudaMemcpyDeviceToHost, stream()));
+  DFM2G_CUDA(cudaStreamSynchronize(stream()));
+  t->nnode_entries = h[0];
+  t->nedge = h[1];
+  t->nedge_entries = h[2];
+  DFM2G_TRY(t->nlist.resize((size_t)h[0] + 1));
+  DFM2G_TRY(t->elist.resize((size_t)h[2] + 1));
+  DFM2G_TRY(t->eslot.resize((size_t)h[1] + 1));
+  DFM2G_TRY(t->eoff.resize((size_t)h[1] + 1));
+  if (nnz) k_tet_edges_compact<<<grid, 256, 0, stream()>>>(nnz, count, at, rank, t->eslot.p, t->eoff.p);
+  // the fill advances the slots' first entries and a copy of the nodes'
+  DFM2G_CUDA(cudaMemcpyAsync(ncount, t->noff.p, sizeof(unsigned) * np, cudaMemcpyDeviceToDevice, stream()));
+  k_tet_lists<<<grid, 256, 0, stream()>>>(t->ntet, t->tet.p, t->slot.p, 1, at, ncount, t->elist.p, t->nlist.p);
+  k_sort_lists<<<grid, 128, 0, stream()>>>(np, t->noff.p, t->nnode_entries, t->nlist.p);
+  if (t->nedge) k_sort_lists<<<grid, 128, 0, stream()>>>(t->nedge, t->eoff.p, t->nedge_entries, t->elist.p);
+  note_launches(6);
+  DFM2G_LAUNCH_CHECK();
+  DFM2G_CUDA(cudaStreamSynchronize(stream()));
+  return DFM2G_OK;
+}
+
+template <int MODE>
+static int tet_assemble(dfm2g_tetmesh_s *t, dfm2g_bsr_s *m, const TetParam &p, double *b) {
+  if (t->ntet == 0) return DFM2G_OK;
+  const double *stress = nullptr;
+  if (MODE != kWarp && p.disp) {
+    DFM2G_TRY(t->stress.ensure(t->ntet * 6 + 2));
+    k_tet_stress<MODE><<<blocks_for(t->ntet, 128), 128, 0, stream()>>>(t->ntet, t->tet.p, t->geo.p, p, t->stress.p);
+    stress = t->stress.p;
+  }
+  if (t->nedge)
+    k_tet_edges<MODE><<<blocks_for(t->nedge, 128), 128, 0, stream()>>>(t->nedge, t->eslot.p, t->eoff.p,
+                                                                      t->nedge_entries, t->elist.p, t->slot.p,
+                                                                      t->tet.p, t->geo.p, p, m->vcrs.p);
+  k_tet_nodes<MODE><<<blocks_for(t->np, 128), 128, 0, stream()>>>((unsigned)t->np, t->noff.p, t->nnode_entries,
+                                                                 t->nlist.p, t->tet.p, t->xyz.p, t->geo.p, stress, p,
+                                                                 m->vdia.p, b);
+  note_launches(stress ? 3 : 2);
+  DFM2G_LAUNCH_CHECK();
+  m->f32_valid = false;
+  return DFM2G_OK;
+}
+
 extern "C" {
 
 int dfm2g_tetmesh_create(dfm2g_tetmesh *out, dfm2g_bsr m, const double *xyz, size_t np, const unsigned *tet,
@@ -349,16 +660,14 @@ int dfm2g_tetmesh_create(dfm2g_tetmesh *out, dfm2g_bsr m, const double *xyz, siz
   if (s == DFM2G_OK) s = t->xyz.resize(np * 3 + 1);
   if (s == DFM2G_OK) s = t->tet.resize(ntet * 4 + 1);
   if (s == DFM2G_OK) s = t->slot.resize(ntet * 16 + 1);
-  if (s == DFM2G_OK) s = t->by_color.resize(ntet + 1);
   if (s == DFM2G_OK && np &&
       cudaMemcpyAsync(t->xyz.p, xyz, sizeof(double) * np * 3, cudaMemcpyHostToDevice, stream()) != cudaSuccess)
     s = fail(DFM2G_ERR_CUDA, "tetmesh_create: copy xyz");
   if (s == DFM2G_OK && ntet &&
-      (cudaMemcpyAsync(t->tet.p, tet, sizeof(unsigned) * ntet * 4, cudaMemcpyHostToDevice, stream()) != cudaSuccess ||
-       cudaMemcpyAsync(t->by_color.p, by_color.data(), sizeof(unsigned) * ntet, cudaMemcpyHostToDevice, stream()) !=
-           cudaSuccess))
+      cudaMemcpyAsync(t->tet.p, tet, sizeof(unsigned) * ntet * 4, cudaMemcpyHostToDevice, stream()) != cudaSuccess)
     s = fail(DFM2G_ERR_CUDA, "tetmesh_create: copy tets");
   if (s == DFM2G_OK) s = build_slot_map(t->tet.p, ntet, 4, m, t->slot.p);
+  if (s == DFM2G_OK) s = tet_lists_build(t, m);
   if (s != DFM2G_OK) {
     delete t;
     return s;
@@ -399,14 +708,14 @@ int dfm2g_tetmesh_assemble_linear(dfm2g_tetmesh t, dfm2g_bsr m, const double *yo
   DFM2G_TRY(ay.in(young, t->ntet, mem, true));
   if (disp) DFM2G_TRY(ad.in(disp, t->np * 3, mem, true));
   DFM2G_TRY(ab.in(b, t->np * 3, mem, true));
-  for (size_t c = 0; c + 1 < t->color_start.size(); ++c) {
-    const unsigned n = t->color_start[c + 1] - t->color_start[c];
-    k_tet_assemble<<<blocks_for((size_t)n * 4, 128), 128, 0, stream()>>>(
-        n, t->by_color.p + t->color_start[c], t->tet.p, t->slot.p, t->xyz.p, ay.dev(), nu, rho, g[0], g[1], g[2],
-        disp ? ad.dev() : nullptr, m->vcrs.p, m->vdia.p, ab.dev());
-  }
-  DFM2G_LAUNCH_CHECK();
-  m->f32_valid = false;
+  TetParam p{};
+  p.lam = nu / ((1.0 + nu) * (1.0 - 2.0 * nu));
+  p.myu = 1.0 / (2.0 * (1.0 + nu));
+  p.rho = rho;
+  for (int d = 0; d < 3; ++d) p.g[d] = g[d];
+  p.young = ay.dev();
+  p.disp = disp ? ad.dev() : nullptr;
+  DFM2G_TRY(tet_assemble<kStatic>(t, m, p, ab.dev()));
   return ab.copy_back();
 } catch (...) {
   return host_failure();
@@ -422,14 +731,17 @@ int dfm2g_tetmesh_assemble_poisson(dfm2g_tetmesh t, dfm2g_bsr m, double alpha, d
   VecArg<double> av, ab;
   if (val) DFM2G_TRY(av.in(val, t->np, mem, true));
   DFM2G_TRY(ab.in(b, t->np, mem, true));
-  for (size_t c = 0; c + 1 < t->color_start.size(); ++c) {
-    const unsigned n = t->color_start[c + 1] - t->color_start[c];
-    k_tet_poisson<<<blocks_for((size_t)n * 4, 128), 128, 0, stream()>>>(
-        n, t->by_color.p + t->color_start[c], t->tet.p, t->slot.p, t->xyz.p, alpha, source, val ? av.dev() : nullptr,
-        m->vcrs.p, m->vdia.p, ab.dev());
+  if (t->ntet) {
+    if (t->nedge)
+      k_poisson_edges<<<blocks_for(t->nedge, 128), 128, 0, stream()>>>(t->nedge, t->eslot.p, t->eoff.p,
+                                                                      t->nedge_entries, t->elist.p, t->slot.p,
+                                                                      t->geo.p, alpha, m->vcrs.p);
+    k_poisson_nodes<<<blocks_for(t->np, 128), 128, 0, stream()>>>((unsigned)t->np, t->noff.p, t->nnode_entries,
+                                                                 t->nlist.p, t->tet.p, t->geo.p, alpha, source,
+                                                                 val ? av.dev() : nullptr, m->vdia.p, ab.dev());
+    note_launches(2);
+    DFM2G_LAUNCH_CHECK();
   }
-  note_launches((unsigned)(t->color_start.empty() ? 0 : t->color_start.size() - 1));
-  DFM2G_LAUNCH_CHECK();
   m->f32_valid = false;
   return ab.copy_back();
 } catch (...) {
@@ -450,25 +762,23 @@ static int tet_dynamic(dfm2g_tetmesh t, dfm2g_bsr m, int mode, double myu, doubl
   DFM2G_TRY(av.in(velo, t->np * 3, mem, true));
   if (mode != kBEuler) DFM2G_TRY(a3.in(third, t->np * (mode == kWarp ? 9 : 3), mem, true));
   DFM2G_TRY(ab.in(b, t->np * 3, mem, true));
-  for (size_t c = 0; c + 1 < t->color_start.size(); ++c) {
-    const unsigned n = t->color_start[c + 1] - t->color_start[c];
-    const unsigned *list = t->by_color.p + t->color_start[c];
-    const unsigned grid = blocks_for((size_t)n * 4, 128);
-#define DFM2G_TET_DYN(M)                                                                                            \
-  k_tet_dynamic<M><<<grid, 128, 0, stream()>>>(n, list, t->tet.p, t->slot.p, t->xyz.p, myu, lambda, rho, g[0], g[1], \
-                                               g[2], dt, beta, ad.dev(), av.dev(),                                  \
-                                               mode == kBEuler ? nullptr : a3.dev(), m->vcrs.p, m->vdia.p, ab.dev())
-    if (mode == kBEuler)
-      DFM2G_TET_DYN(kBEuler);
-    else if (mode == kWarp)
-      DFM2G_TET_DYN(kWarp);
-    else
-      DFM2G_TET_DYN(kNewmark);
-#undef DFM2G_TET_DYN
-  }
-  note_launches((unsigned)(t->color_start.empty() ? 0 : t->color_start.size() - 1));
-  DFM2G_LAUNCH_CHECK();
-  m->f32_valid = false;
+  TetParam p{};
+  p.lam = lambda;
+  p.myu = myu;
+  p.rho = rho;
+  for (int d = 0; d < 3; ++d) p.g[d] = g[d];
+  p.dt = dt;
+  p.beta = beta;
+  p.disp = ad.dev();
+  p.velo = av.dev();
+  if (mode == kWarp) p.rot = a3.dev();
+  if (mode == kNewmark) p.acc = a3.dev();
+  if (mode == kBEuler)
+    DFM2G_TRY(tet_assemble<kBEuler>(t, m, p, ab.dev()));
+  else if (mode == kWarp)
+    DFM2G_TRY(tet_assemble<kWarp>(t, m, p, ab.dev()));
+  else
+    DFM2G_TRY(tet_assemble<kNewmark>(t, m, p, ab.dev()));
   return ab.copy_back();
 }
 
@@ -501,7 +811,7 @@ int dfm2g_tetmesh_dLdE(dfm2g_tetmesh t, const double *young, double nu, const do
   DFM2G_TRY(al.in(lam, t->np * 3, mem, true));
   DFM2G_TRY(ao.in(dLdE, t->ntet, mem, false));
   if (t->ntet)
-    k_tet_dLdE<<<blocks_for(t->ntet, 128, ctx().num_sms * 32), 128, 0, stream()>>>(t->ntet, t->tet.p, t->xyz.p, nu,
+    k_tet_dLdE<<<blocks_for(t->ntet, 128, ctx().num_sms * 32), 128, 0, stream()>>>(t->ntet, t->tet.p, t->geo.p, nu,
                                                                                   au.dev(), al.dev(), ao.dev());
   DFM2G_LAUNCH_CHECK();
   return ao.copy_back();
