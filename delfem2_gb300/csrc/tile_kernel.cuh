@@ -334,6 +334,8 @@ __global__ void __launch_bounds__(32 * (NW + HW + 1), 1)
         };
         if (pending()) {
           // not written yet (this tile runs close behind another): polled in L2
+          // (all pending values at each poll: polling one a lane and reading the
+          // others after it, or two staggered reads of each, measured 0-5% slower)
           unsigned long long t0 = 0;
           unsigned spins = 0;
           do {
@@ -382,28 +384,21 @@ __global__ void __launch_bounds__(32 * (NW + HW + 1), 1)
   constexpr unsigned kDeps = kLast ? MS - 1 : MS;
   const unsigned pos = warp * L::kG + q;  // the lane's row among the step's
 
-  // Warps without a group in a step: FP32 skips (shared-memory bandwidth bounds
-  // its steps), FP64 works on group 0 and stores nothing, so that the step is one
-  // straight piece of code and the next step's loads go out between the
-  // FP64 instructions (each of its warps has an SM quarter to itself).
-  constexpr bool kSkip = sizeof(T) == 4;
+  // A warp without a group in a step works on group 0 and stores nothing: the
+  // step stays one straight piece of code, the next step's loads between its
+  // products (skipping such warps' work measured 2-8% slower in FP32).
   struct Step {
-    bool work;
     unsigned row, local, area;
     unsigned at[kMsc];  // operand offsets: codes until place(), then from ti_smem
     T v[(kNv + kPer - 1) / kPer * kPer];
   };
   // codes and values of the step in `slot`; false: the CTA is done
-  auto load = [&](Step &N, unsigned slot) -> bool {
-    const uint4 meta = smeta[slot];
-    const int stop = sstop[slot];
+  auto load = [&](Step &N, unsigned slot, const uint4 meta, int stop) -> bool {
     const unsigned ng = meta.x & 0xFFu;
     const bool more = meta.w != kTiEnd && stop == 0;
-    N.work = warp < ng;
-    if (kSkip && !(more && N.work)) return more;
     const unsigned so = slot * A.slot_bytes;
     N.area = A.ring_off + so + A.area_off;
-    const unsigned char *gp = ring + so + (N.work ? warp * A.gbytes : 0u);
+    const unsigned char *gp = ring + so + (warp < ng ? warp * A.gbytes : 0u);
     const uint4 *cw = reinterpret_cast<const uint4 *>(gp + (q * S + h) * kMsc * 4u);
 #pragma unroll
     for (unsigned k = 0; k < kMsc / 4; ++k) {
@@ -450,62 +445,60 @@ __global__ void __launch_bounds__(32 * (NW + HW + 1), 1)
     // their reads before this store; a fence would cost 120 cycles)
     if (threadIdx.x == 0) *sdone = done;
     ++done;
-    const bool busy = !kSkip || C.work;
+    // the next step's descriptor first: shared memory answers in order
+    const uint4 meta = smeta[s1];
+    const int stop = sstop[s1];
     T x[MS * B], c = T(0);
-    if (busy) {
 #pragma unroll
-      for (unsigned j = 0; j < MS; ++j)  // (the slot of D^-1 holds a dependency on the other half)
-        if (j < kDeps || S > 1) tile_row<T, B>(ti_smem + C.at[j], x + j * B);
-      if constexpr (!FWD || kLast) c = reinterpret_cast<const T *>(ti_smem + C.area + (C.row != ~0u ? pos : 0u) * kRow)[a];
+    for (unsigned j = 0; j < MS; ++j)  // (the slot of D^-1 holds a dependency on the other half)
+      if (j < kDeps || S > 1) tile_row<T, B>(ti_smem + C.at[j], x + j * B);
+    if constexpr (!FWD || kLast) c = reinterpret_cast<const T *>(ti_smem + C.area + (C.row != ~0u ? pos : 0u) * kRow)[a];
+    const bool more = load(N, s1, meta, stop);
+    T acc[kAcc];
+#pragma unroll
+    for (unsigned k = 0; k < kAcc; ++k) acc[k] = T(0);
+    if constexpr (!FWD && sizeof(T) == 8) acc[0] = h == 0 ? -c : T(0);
+#pragma unroll
+    for (unsigned j = 0; j < MS; ++j) {
+      if (j < kDeps || (S > 1 && h != S - 1)) {
+#pragma unroll
+        for (unsigned k = 0; k < B; ++k) acc[k % kAcc] += C.v[j * B + k] * x[j * B + k];
+      }
     }
-    const bool more = load(N, s1);
-    if (busy) {
-      T acc[kAcc];
+    T z = acc[0];
 #pragma unroll
-      for (unsigned k = 0; k < kAcc; ++k) acc[k] = T(0);
-      if constexpr (!FWD && sizeof(T) == 8) acc[0] = h == 0 ? -c : T(0);
+    for (unsigned k = 1; k < kAcc; ++k) z += acc[k];
+    if constexpr (S == 2) z += __shfl_sync(0xffffffffu, z, lane_ok ? (h == 0 ? lane + B : lane - B) : lane);
+    // FP32 subtracts the finished sum: started from the right-hand side, the
+    // chain would round at its magnitude in every product (1.2e-7 against 8.2e-8)
+    if constexpr (sizeof(T) == 4)
+      z = c - z;
+    else
+      z = -z;
+    if constexpr (kLast) {
+      T t = T(0);
 #pragma unroll
-      for (unsigned j = 0; j < MS; ++j) {
-        if (j < kDeps || (S > 1 && h != S - 1)) {
-#pragma unroll
-          for (unsigned k = 0; k < B; ++k) acc[k % kAcc] += C.v[j * B + k] * x[j * B + k];
-        }
-      }
-      T z = acc[0];
-#pragma unroll
-      for (unsigned k = 1; k < kAcc; ++k) z += acc[k];
-      if constexpr (S == 2) z += __shfl_sync(0xffffffffu, z, lane_ok ? (h == 0 ? lane + B : lane - B) : lane);
-      // FP32 subtracts the finished sum: started from the right-hand side, the
-      // chain would round at its magnitude in every product (1.2e-7 against 8.2e-8)
-      if constexpr (sizeof(T) == 4)
-        z = c - z;
-      else
-        z = -z;
-      if constexpr (kLast) {
-        T t = T(0);
-#pragma unroll
-        for (unsigned k = 0; k < B; ++k)
-          t += C.v[(MS - 1) * B + k] * (B == 1 ? z : __shfl_sync(0xffffffffu, z, half0 + k));
-        z = t;
-      }
-      if (C.row != ~0u && h == kOut) {
-        reinterpret_cast<T *>(xs + (size_t)C.local * kRow)[a] = z;
-        st_relaxed(out + (size_t)C.row * B + a, z);
-      }
+      for (unsigned k = 0; k < B; ++k)
+        t += C.v[(MS - 1) * B + k] * (B == 1 ? z : __shfl_sync(0xffffffffu, z, half0 + k));
+      z = t;
+    }
+    if (C.row != ~0u && h == kOut) {
+      reinterpret_cast<T *>(xs + (size_t)C.local * kRow)[a] = z;
+      st_relaxed(out + (size_t)C.row * B + a, z);
     }
     if (!more) {
       // the end markers need this slot too (they touch only its descriptor)
       if (threadIdx.x == 0) *sdone = done - 1u + A.nslots;
       return false;
     }
-    if (!kSkip || N.work) place(N);
+    place(N);
     s0 = s1;
     return true;
   };
   Step P0, P1;
   asm volatile("bar.sync %0, %1;" ::"n"(kFirst), "n"(32 * (NW + 1)) : "memory");
-  if (!load(P0, 0)) return;
-  if (!kSkip || P0.work) place(P0);
+  if (!load(P0, 0, smeta[0], sstop[0])) return;
+  place(P0);
   while (step(P0, P1) && step(P1, P0)) {
   }
 }

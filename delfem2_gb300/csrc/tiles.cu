@@ -228,7 +228,7 @@ struct TileHost {
 struct TileShape {
   unsigned B, S, rows, segs, width;  // block size, lanes split, limits of a tile and of a step
   unsigned row_bytes, vs;            // bytes of a row in shared memory, of a value
-  unsigned ms[3];                    // slots per lane the kernels are compiled for, ascending (0: none)
+  unsigned ms[4];                    // slots per lane the kernels are compiled for, ascending (0: none)
 };
 
 // Codes and slot sources from the partition. Slots of a row: its dependencies
@@ -359,7 +359,7 @@ void tile_host_build(unsigned n, const std::vector<unsigned> &rs, const std::vec
   out.ok = true;
 }
 
-unsigned tile_max_slots(const TileShape &sh) { return *std::max_element(sh.ms, sh.ms + 3); }
+unsigned tile_max_slots(const TileShape &sh) { return *std::max_element(sh.ms, sh.ms + 4); }
 
 template <typename V>
 int tile_to_host(std::vector<V> &h, const V *d, size_t n) {
@@ -545,7 +545,7 @@ void *tile_kernel(bool forward) {
                  : (void *)k_sweep_tiles<T, B, S, NW, HW, MS, false>;
 }
 
-template <typename T, int B, int S, int NW, int HW, int MSA, int MSB>
+template <typename T, int B, int S, int NW, int HW, int MSA, int MSB, int MSC, int MSD>
 int tile_launch(dfm2g_ilu_s *p, TileSched &ts, bool forward, const T *in, T *out, const int *skip,
                 unsigned long long timeout, bool *usable) {
   constexpr unsigned kRow = kTiXw<T, B> * (unsigned)sizeof(T);
@@ -591,8 +591,10 @@ int tile_launch(dfm2g_ilu_s *p, TileSched &ts, bool forward, const T *in, T *out
     note_launches(1);
     ts.ver = p->factor_version;
   }
-  void *kernel = ts.ms == MSA ? tile_kernel<T, B, S, NW, HW, MSA>(forward)
-                              : tile_kernel<T, B, S, NW, HW, MSB>(forward);
+  void *kernel = ts.ms == MSA   ? tile_kernel<T, B, S, NW, HW, MSA>(forward)
+                 : ts.ms == MSB ? tile_kernel<T, B, S, NW, HW, MSB>(forward)
+                 : ts.ms == MSC ? tile_kernel<T, B, S, NW, HW, MSC>(forward)
+                                : tile_kernel<T, B, S, NW, HW, MSD>(forward);
   DFM2G_TRY(tile_allow_smem(kernel, smem));
   if (ts.coop <= 0) {
     int per_sm = 0;
@@ -618,14 +620,14 @@ int tile_launch(dfm2g_ilu_s *p, TileSched &ts, bool forward, const T *in, T *out
 // Prepares `pair` (both directions) and sweeps; nothing is done (*usable
 // stays false) when the pattern's rows are too long, or when !may_alloc and
 // the records do not exist yet.
-template <typename T, int B, int S, int NW, int HW, int MSA, int MSB>
+template <typename T, int B, int S, int NW, int HW, int MSA, int MSB, int MSC, int MSD>
 int tile_run(dfm2g_ilu_s *p, TileSched *pair, const TileShape &sh, bool forward, const T *in, T *out, const int *skip,
              unsigned long long timeout, bool may_alloc, bool force, bool *usable) {
   TileSched &ts = pair[forward ? 0 : 1];
   if (!may_alloc && (!ts.built || !ts.ok || !ts.bytes.p)) return DFM2G_OK;
   if (!ts.built || (force && ts.thin)) DFM2G_TRY(tile_build(p, pair, sh, force));
   if (!ts.ok) return DFM2G_OK;
-  return tile_launch<T, B, S, NW, HW, MSA, MSB>(p, ts, forward, in, out, skip, timeout, usable);
+  return tile_launch<T, B, S, NW, HW, MSA, MSB, MSC, MSD>(p, ts, forward, in, out, skip, timeout, usable);
 }
 
 // Shapes. The tiles are squares of z lines on the voxel grids (a row's offers
@@ -636,12 +638,12 @@ int tile_run(dfm2g_ilu_s *p, TileSched *pair, const TileShape &sh, bool forward,
 // small tiles hop sooner: 65^3 nodes 200 us a sweep, 285 with 6 x 6 lines on
 // eight warps). 1x1 and 2x2: two lane groups per row.
 constexpr int kHw = 3, kHwNd = 4;  // fetch warps
-constexpr TileShape kShape32{3, 1, 36 * 65, 36, 40, 16, 4, {8, 16, 0}};
-constexpr TileShape kShape64{3, 2, 16 * 65, 16, 20, 24, 8, {4, 8, 0}};
+constexpr TileShape kShape32{3, 1, 36 * 65, 36, 40, 16, 4, {7, 8, 14, 16}};
+constexpr TileShape kShape64{3, 2, 16 * 65, 16, 20, 24, 8, {3, 4, 7, 8}};
 template <typename T>
-constexpr TileShape kShapeNd2{2, 2, 32 * 65, 32, 32, 2 * sizeof(T), sizeof(T), {4, 8, 0}};
+constexpr TileShape kShapeNd2{2, 2, 32 * 65, 32, 32, 2 * sizeof(T), sizeof(T), {4, 8, 0, 0}};
 template <typename T>
-constexpr TileShape kShapeNd1{1, 2, 64 * 65, 64, 64, sizeof(T), sizeof(T), {4, 8, 0}};
+constexpr TileShape kShapeNd1{1, 2, 64 * 65, 64, 64, sizeof(T), sizeof(T), {4, 8, 0, 0}};
 
 }  // namespace
 
@@ -657,16 +659,16 @@ int tile_sweep(dfm2g_ilu_s *p, bool forward, const T *in, T *out, const int *ski
   TileSched *pair = p->tiles[f64 ? 1 : 0];
   *usable = *full = false;
   if (p->ndim == 1)
-    return tile_run<T, 1, 2, 4, kHwNd, 4, 8>(p, pair, kShapeNd1<T>, forward, in, out, skip, timeout, may_alloc,
+    return tile_run<T, 1, 2, 4, kHwNd, 4, 8, 8, 8>(p, pair, kShapeNd1<T>, forward, in, out, skip, timeout, may_alloc,
                                              force, usable);
   if (p->ndim == 2)
-    return tile_run<T, 2, 2, 4, kHwNd, 4, 8>(p, pair, kShapeNd2<T>, forward, in, out, skip, timeout, may_alloc,
+    return tile_run<T, 2, 2, 4, kHwNd, 4, 8, 8, 8>(p, pair, kShapeNd2<T>, forward, in, out, skip, timeout, may_alloc,
                                              force, usable);
   constexpr TileShape sh = f64 ? kShape64 : kShape32;
   if constexpr (f64)
-    DFM2G_TRY((tile_run<T, 3, 2, 4, kHw, 4, 8>(p, pair, sh, forward, in, out, skip, timeout, may_alloc, force, usable)));
+    DFM2G_TRY((tile_run<T, 3, 2, 4, kHw, 3, 4, 7, 8>(p, pair, sh, forward, in, out, skip, timeout, may_alloc, force, usable)));
   else
-    DFM2G_TRY((tile_run<T, 3, 1, 4, kHw, 8, 16>(p, pair, sh, forward, in, out, skip, timeout, may_alloc, force, usable)));
+    DFM2G_TRY((tile_run<T, 3, 1, 4, kHw, 7, 8, 14, 16>(p, pair, sh, forward, in, out, skip, timeout, may_alloc, force, usable)));
   *full = *usable && (forward ? p->max_lower : p->max_upper) <= kTiAutoDeps &&
           2.0 * pair[forward ? 0 : 1].rows_per_step >= sh.segs && (!f64 || p->nblk >= kTi64MinRows);
   return DFM2G_OK;
