@@ -90,9 +90,16 @@ static bool make_tiles(const std::vector<unsigned> &rs, unsigned nblk, unsigned 
 int bsr_tiles_build(dfm2g_bsr_s *m) {
   m->tiles_ok = false;
   std::vector<unsigned> t32, t64;
+  // Fewer rows than fill the machine at full tiles: shorter tiles, down to one
+  // consumer warp for each quarter of an SM, so that a tile's rows (a latency
+  // chain of their own each) run on more SMs at once.
+  constexpr unsigned kLeast = 40;
+  const unsigned share = (m->nblk / (unsigned)ctx().num_sms + 10) / 10 * 10;
   if (m->nblk == 0 ||
-      !make_tiles(m->h_row_start, m->nblk, TileCfgC<float>::kBlocks, TileCfgC<float>::kRows, t32) ||
-      !make_tiles(m->h_row_start, m->nblk, TileCfgC<double>::kBlocks, TileCfgC<double>::kRows, t64))
+      !make_tiles(m->h_row_start, m->nblk, TileCfgC<float>::kBlocks,
+                  std::min(std::max(share, kLeast), TileCfgC<float>::kRows), t32) ||
+      !make_tiles(m->h_row_start, m->nblk, TileCfgC<double>::kBlocks,
+                  std::min(std::max(share, kLeast), TileCfgC<double>::kRows), t64))
     return DFM2G_OK;
   DFM2G_TRY(m->tiles32.resize(t32.size()));
   DFM2G_TRY(m->tiles64.resize(t64.size()));

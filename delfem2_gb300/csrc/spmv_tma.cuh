@@ -27,13 +27,21 @@ __device__ __forceinline__ void round16(size_t off, size_t end, size_t &a, unsig
 // ---------------------------------------------------------------------------
 // Component layout: lane 3q + a of a consumer warp computes component a of
 // row q of the warp's ten rows, summing K_b[a][0..2] x_b over the row's
-// blocks with no cross-lane reduction. A warp instruction then serves ten rows
-// (the lane layout above: one row per 27 lanes plus a 7-shuffle reduction), so
-// the kernel issues a fraction of the instructions per row (and, in FP64, of
-// the FP64 instructions). Tiles hold ten rows per consumer warp and are
-// double-buffered; the tile's row offsets are staged with its values, block
-// columns and diagonal blocks. FP32: 15 consumer warps (150-row tiles), FP64:
-// 7 (70-row tiles), one CTA per SM.
+// blocks with no cross-lane reduction. A warp instruction then serves ten rows,
+// so the kernel issues a fraction of the instructions per row (and, in FP64, of
+// the FP64 instructions) of a layout with a warp per row. Tiles hold ten rows
+// per consumer warp and are double-buffered; the tile's row offsets are staged
+// with its values, block columns and diagonal blocks. FP32: 15 consumer warps
+// (150-row tiles), one CTA per SM.
+//
+// FP64: a quarter of an SM issues one FP64 warp instruction per 64 cycles, so
+// the product is bound by their number and by how evenly the warps cover the
+// four quarters: eight consumer warps (80-row tiles), two per quarter, and three
+// fused multiply-adds a block into six sums (component x block parity; two
+// sums over whole blocks take a fourth instruction, the addition, per block).
+// The rounding error is no larger: root mean square 0.299 against 0.305 units
+// of 1e-16 |K||x| over 14-block rows that cancel, 0.180 against 0.212 on smooth
+// vectors.
 #ifndef DFM2G_SPMV_F32_CONSUMERS
 #define DFM2G_SPMV_F32_CONSUMERS 15u  // FP32 tile: consumer warps (ten rows each)
 #endif
@@ -45,10 +53,10 @@ __device__ __forceinline__ void round16(size_t off, size_t end, size_t &a, unsig
 #endif
 template <typename T>
 struct TileCfgC {
-  static constexpr unsigned kConsumers = sizeof(T) == 8 ? 7u : DFM2G_SPMV_F32_CONSUMERS;
+  static constexpr unsigned kConsumers = sizeof(T) == 8 ? 8u : DFM2G_SPMV_F32_CONSUMERS;
   static constexpr unsigned kThreads = 32u * (kConsumers + 1u);
   static constexpr unsigned kRows = kConsumers * 10u;
-  static constexpr unsigned kBlocks = sizeof(T) == 8 ? 1152u : DFM2G_SPMV_F32_BLOCKS;
+  static constexpr unsigned kBlocks = sizeof(T) == 8 ? 1424u : DFM2G_SPMV_F32_BLOCKS;
   static constexpr unsigned kStages = sizeof(T) == 8 ? 2u : DFM2G_SPMV_F32_STAGES;
   static constexpr unsigned kValBytes = kBlocks * 9 * sizeof(T) + 32;
   static constexpr unsigned kColBytes = kBlocks * 4 + 32;
@@ -59,7 +67,7 @@ struct TileCfgC {
   static constexpr size_t kSmem = kBarBytes + (size_t)kStages * kStageBytes;
   static_assert(kValBytes % 16 == 0 && kColBytes % 16 == 0 && kDiaBytes % 16 == 0 && kRsBytes % 16 == 0,
                 "16-byte stage layout");
-  static_assert(kSmem <= 227u * 1024u, "fits one CTA's shared memory");
+  static_assert(kSmem + 1024u <= 227u * 1024u, "fits one CTA's shared memory beside the reductions' words");
 };
 
 // Runs the pipeline over all tiles; epi(row, a, v) is called by the lane that
@@ -136,22 +144,50 @@ __device__ __forceinline__ void spmv_tma_rows_c(const unsigned *__restrict__ til
     const unsigned i = r0 + warp * 10u + q;
     if (lane < 30 && i < r1) {
       const unsigned s0 = rsv[i - r0] - b0, s1 = rsv[i - r0 + 1] - b0;
-      T acc0 = T(0), acc1 = T(0);
-      unsigned u = s0;
-      for (; u + 1 < s1; u += 2) {  // two blocks per step: both x gathers in flight
-        const unsigned j0 = cv[u], j1 = cv[u + 1];
-        const T *v0 = vv + (size_t)u * 9 + a * 3, *v1 = v0 + 9;
-        const T *x0 = x + (size_t)j0 * 3, *x1 = x + (size_t)j1 * 3;
-        acc0 += v0[0] * __ldg(x0) + v0[1] * __ldg(x0 + 1) + v0[2] * __ldg(x0 + 2);
-        acc1 += v1[0] * __ldg(x1) + v1[1] * __ldg(x1 + 1) + v1[2] * __ldg(x1 + 2);
-      }
-      if (u < s1) {
-        const T *v0 = vv + (size_t)u * 9 + a * 3, *x0 = x + (size_t)cv[u] * 3;
-        acc0 += v0[0] * __ldg(x0) + v0[1] * __ldg(x0 + 1) + v0[2] * __ldg(x0 + 2);
-      }
       const T *d = dv + (size_t)(i - r0) * 9 + a * 3, *xi = x + (size_t)i * 3;
-      acc1 += d[0] * __ldg(xi) + d[1] * __ldg(xi + 1) + d[2] * __ldg(xi + 2);
-      epi(i, a, acc0 + acc1);
+      unsigned u = s0;
+      if constexpr (sizeof(T) == 8) {
+        T e0 = T(0), e1 = T(0), e2 = T(0), o0 = T(0), o1 = T(0), o2 = T(0);
+        if ((s1 - u) & 1u) {
+          const T *v0 = vv + (size_t)u * 9 + a * 3, *x0 = x + (size_t)cv[u] * 3;
+          e0 = v0[0] * __ldg(x0), e1 = v0[1] * __ldg(x0 + 1), e2 = v0[2] * __ldg(x0 + 2);
+          ++u;
+        }
+        // two blocks per step, the next two's x gathered under this step's products
+        T g[6] = {};
+        auto gather = [&](unsigned k) {
+          const T *x0 = x + (size_t)cv[k] * 3, *x1 = x + (size_t)cv[k + 1] * 3;
+#pragma unroll
+          for (int c = 0; c < 3; ++c) g[c] = __ldg(x0 + c), g[3 + c] = __ldg(x1 + c);
+        };
+        if (u < s1) gather(u);
+        while (u < s1) {
+          const T *v0 = vv + (size_t)u * 9 + a * 3, *v1 = v0 + 9;
+          const T h[6] = {g[0], g[1], g[2], g[3], g[4], g[5]};
+          u += 2;
+          if (u < s1) gather(u);
+          e0 += v0[0] * h[0], e1 += v0[1] * h[1], e2 += v0[2] * h[2];
+          o0 += v1[0] * h[3], o1 += v1[1] * h[4], o2 += v1[2] * h[5];
+        }
+        // the diagonal block, the largest terms, last: fewer sums are rounded at its size
+        o0 += d[0] * __ldg(xi), o1 += d[1] * __ldg(xi + 1), o2 += d[2] * __ldg(xi + 2);
+        epi(i, a, ((e0 + e1) + e2) + ((o0 + o1) + o2));
+      } else {
+        T acc0 = T(0), acc1 = T(0);
+        for (; u + 1 < s1; u += 2) {
+          const unsigned j0 = cv[u], j1 = cv[u + 1];
+          const T *v0 = vv + (size_t)u * 9 + a * 3, *v1 = v0 + 9;
+          const T *x0 = x + (size_t)j0 * 3, *x1 = x + (size_t)j1 * 3;
+          acc0 += v0[0] * __ldg(x0) + v0[1] * __ldg(x0 + 1) + v0[2] * __ldg(x0 + 2);
+          acc1 += v1[0] * __ldg(x1) + v1[1] * __ldg(x1 + 1) + v1[2] * __ldg(x1 + 2);
+        }
+        if (u < s1) {
+          const T *v0 = vv + (size_t)u * 9 + a * 3, *x0 = x + (size_t)cv[u] * 3;
+          acc0 += v0[0] * __ldg(x0) + v0[1] * __ldg(x0 + 1) + v0[2] * __ldg(x0 + 2);
+        }
+        acc1 += d[0] * __ldg(xi) + d[1] * __ldg(xi + 1) + d[2] * __ldg(xi + 2);
+        epi(i, a, acc0 + acc1);
+      }
     }
     __syncwarp();
     if (lane == 0) mbar_arrive(&empty[s]);
