@@ -205,6 +205,19 @@ __device__ __forceinline__ double block_sum(double v, double *sh) {
   return v;
 }
 
+// Sum over the block's threads of partials[0, nparts) in a fixed order; valid
+// in thread 0. Up to 32 partials are one warp's work: the other warps' shuffle
+// trees (an FP64 warp instruction takes an SM quarter 64 cycles) are left out.
+__device__ __forceinline__ double sum_partials(const double *partials, unsigned nparts, double *sh) {
+  double s = 0.0;
+  if (nparts <= 32) {
+    if (threadIdx.x < 32) s = warp_sum(threadIdx.x < nparts ? ld_relaxed(partials + threadIdx.x) : 0.0);
+    return s;
+  }
+  for (unsigned b = threadIdx.x; b < nparts; b += blockDim.x) s += ld_relaxed(partials + b);
+  return block_sum(s, sh);
+}
+
 // Deterministic grid reduction: every block writes its partial sum, the last
 // block to arrive (ticket) adds the partials in block order. Returns true in
 // thread 0 of the last block, with *total set; the ticket is reset there.
@@ -212,6 +225,10 @@ __device__ __forceinline__ bool grid_sum_last(double partial, double *partials,
                                               unsigned *ticket, double *sh, double *total) {
   __shared__ bool am_last;
   double v = block_sum(partial, sh);
+  if (gridDim.x == 1) {
+    if (threadIdx.x == 0) *total = v;
+    return threadIdx.x == 0;
+  }
   if (threadIdx.x == 0) {
     partials[blockIdx.x] = v;
     __threadfence();
@@ -221,10 +238,7 @@ __device__ __forceinline__ bool grid_sum_last(double partial, double *partials,
   __syncthreads();
   if (!am_last) return false;
   __threadfence();
-  double s = 0.0;
-  for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x) s += ld_relaxed(partials + b);
-  // fixed-order combination: per-thread strided sums then a fixed tree
-  s = block_sum(s, sh);
+  const double s = sum_partials(partials, gridDim.x, sh);
   if (threadIdx.x == 0) {
     *total = s;
     *ticket = 0;
@@ -232,26 +246,29 @@ __device__ __forceinline__ bool grid_sum_last(double partial, double *partials,
   return threadIdx.x == 0;
 }
 
-// Barrier of all CTAs of a cooperative launch: bar[0] counts arrivals, bar[1]
-// is the generation the last arrival advances (both start at 0 and the count
-// returns to 0, so one pair serves any number of barriers of successive
-// launches on a stream). Bounded: false, with DFM2G_ERR_WAIT_TIMEOUT in
-// *err, when the other CTAs do not all arrive within timeout_ns.
+// Barrier of all CTAs of a cooperative launch over one word (*bar, 0 at the
+// start): its low 16 bits count arrivals, its high 16 bits the barriers passed.
+// An arrival adds 1 and learns the generation it waits out from the old value;
+// the last one adds what takes the count back to 0 and the generation on by one
+// (so the word serves any number of barriers of successive launches on a
+// stream; at most 65,535 CTAs). One atomic each and one poll are on the way from
+// the last arrival to the others' leaving. Bounded: false, with
+// DFM2G_ERR_WAIT_TIMEOUT in *err, when the other CTAs do not all arrive within
+// timeout_ns.
 __device__ __forceinline__ bool grid_barrier(unsigned *bar, int *err, unsigned long long timeout_ns) {
   __shared__ int ok_s;
   __syncthreads();
+  if (gridDim.x == 1) return true;
   if (threadIdx.x == 0) {
     int ok = 1;
-    volatile unsigned *gen = bar + 1;
-    const unsigned g = *gen;
     __threadfence();
-    if (atomicAdd(bar, 1u) == gridDim.x - 1) {
-      atomicExch(bar, 0u);
+    const unsigned old = atomicAdd(bar, 1u);
+    if ((old & 0xffffu) == gridDim.x - 1) {
       __threadfence();
-      atomicAdd(bar + 1, 1u);
+      atomicAdd(bar, 0x10000u - gridDim.x);
     } else {
       const unsigned long long t0 = globaltimer_ns();
-      while (*gen == g) {
+      while ((ld_acquire(bar) ^ old) >> 16 == 0u) {
         if (globaltimer_ns() - t0 > timeout_ns) {
           atomicCAS(err, 0, DFM2G_ERR_WAIT_TIMEOUT);
           ok = 0;
@@ -270,9 +287,7 @@ __device__ __forceinline__ bool grid_barrier(unsigned *bar, int *err, unsigned l
 // calls it (all threads of the CTA receive it).
 __device__ __forceinline__ double sum_partials_all(const double *partials, unsigned nparts, double *sh) {
   __shared__ double total_s;
-  double s = 0.0;
-  for (unsigned b = threadIdx.x; b < nparts; b += blockDim.x) s += ld_relaxed(partials + b);
-  s = block_sum(s, sh);
+  const double s = sum_partials(partials, nparts, sh);
   if (threadIdx.x == 0) total_s = s;
   __syncthreads();
   return total_s;

@@ -617,7 +617,14 @@ struct Workspace {
 };
 static Workspace g_ws;
 
-static unsigned reduce_blocks() { return (unsigned)ctx().num_sms * 4; }
+// CTAs of a pass over n elements with a reduction: one per pass of four
+// elements a thread, at most four per SM. Up to kOneCta elements are one CTA's:
+// its few more passes are shorter than the meeting of several CTAs.
+static unsigned reduce_blocks(size_t n) {
+  constexpr size_t kOneCta = 4096;
+  if (n <= kOneCta) return 1;
+  return (unsigned)std::min<size_t>((n + 4 * kThreads - 1) / (4 * kThreads), (size_t)ctx().num_sms * 4);
+}
 
 static int ws_prepare(size_t n, unsigned hist_cap, bool need32) {
   DFM2G_TRY(g_ws.st.ensure(1));
@@ -641,10 +648,10 @@ static int dot_dev(size_t n, const void *a, const void *b, int prec, double *out
   DFM2G_CUDA(cudaMemsetAsync(g_ws.tickets.p, 0, sizeof(unsigned), stream()));
   note_launches(1);
   if (prec == DFM2G_F64)
-    k_dot<double><<<reduce_blocks(), kThreads, 0, stream()>>>(n, (const double *)a, (const double *)b,
+    k_dot<double><<<reduce_blocks(n), kThreads, 0, stream()>>>(n, (const double *)a, (const double *)b,
                                                              g_ws.partials.p, g_ws.tickets.p, out_dev);
   else
-    k_dot<float><<<reduce_blocks(), kThreads, 0, stream()>>>(n, (const float *)a, (const float *)b, g_ws.partials.p,
+    k_dot<float><<<reduce_blocks(n), kThreads, 0, stream()>>>(n, (const float *)a, (const float *)b, g_ws.partials.p,
                                                             g_ws.tickets.p, out_dev);
   DFM2G_LAUNCH_CHECK();
   return DFM2G_OK;
@@ -676,19 +683,16 @@ static int allow_tma_smem(K kernel, size_t smem, int &attr_device) {
   return DFM2G_OK;
 }
 
-#ifndef DFM2G_DOT_CTAS_PER_SM
-#define DFM2G_DOT_CTAS_PER_SM 4u  // CTAs per SM of k_dot_pupdate
-#endif
-// CTAs of k_dot_pupdate<T>: DFM2G_DOT_CTAS_PER_SM per SM, or as many as are resident at once.
+// CTAs of k_dot_pupdate<T>: reduce_blocks(n), or as many as are resident at once.
 template <typename T>
-static int dot_pupdate_blocks(unsigned *grid) {
+static int dot_pupdate_blocks(size_t n, unsigned *grid) {
   static int per_sm_dev = -1, per_sm = 0;
   if (per_sm_dev != ctx().device) {
     DFM2G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_dot_pupdate<T>, kThreads, 0));
     per_sm_dev = ctx().device;
   }
   if (per_sm <= 0) return fail(DFM2G_ERR_CUDA, "k_dot_pupdate cannot be resident");
-  *grid = std::min<unsigned>(DFM2G_DOT_CTAS_PER_SM * (unsigned)ctx().num_sms, (unsigned)per_sm * (unsigned)ctx().num_sms);
+  *grid = std::min(reduce_blocks(n), (unsigned)per_sm * (unsigned)ctx().num_sms);
   return DFM2G_OK;
 }
 
@@ -746,7 +750,7 @@ static int pcg_core(dfm2g_bsr_s *m, dfm2g_ilu_s *p, T *r, T *x, T *w0, T *w1, T 
   note_launches(1);
   DFM2G_LAUNCH_CHECK();
   const unsigned spmv_blocks = blocks_for((size_t)nblk * 32, kThreads, (unsigned)ctx().num_sms * 8);
-  const unsigned vec_blocks = reduce_blocks();
+  const unsigned vec_blocks = reduce_blocks(n);
   const int chunk = 16;
   // 3x3 patterns with SpMV tiles: two cooperative launches besides the SpMV
   // and the sweeps per iteration (k_spmv_update_tma_c, k_dot_pupdate) and the
@@ -762,7 +766,7 @@ static int pcg_core(dfm2g_bsr_s *m, dfm2g_ilu_s *p, T *r, T *x, T *w0, T *w1, T 
     static int attr_a = -1, attr_r = -1;
     DFM2G_TRY(allow_tma_smem(k_spmv_update_tma_c<T>, CT::kSmem, attr_a));
     DFM2G_TRY(allow_tma_smem(k_refresh_tma, C64::kSmem, attr_r));
-    DFM2G_TRY(dot_pupdate_blocks<T>(&dp_grid));
+    DFM2G_TRY(dot_pupdate_blocks<T>(n, &dp_grid));
   }
   for (;;) {
     for (int k = 0; k < chunk; ++k) {
@@ -1002,7 +1006,7 @@ int dfm2g_solve_pcg_mixed_reliable(dfm2g_bsr m, dfm2g_ilu p, const double *b, do
   if (bnorm > 0) {
     {
       ProfScope ps(DFM2G_PROF_OUTER, 1);
-      k_scale_convert<float><<<reduce_blocks(), kThreads, 0, stream()>>>(n, ab.dev(), 1.0 / bnorm, r32);
+      k_scale_convert<float><<<reduce_blocks(n), kThreads, 0, stream()>>>(n, ab.dev(), 1.0 / bnorm, r32);
     }
     DFM2G_LAUNCH_CHECK();
     Refine rf;
@@ -1058,7 +1062,7 @@ int dfm2g_solve_pcg_mixed(dfm2g_bsr m, dfm2g_ilu p, const double *b, double *x, 
   unsigned total_it = 0, outer = 0;
   double rel = bnorm > 0 ? 1.0 : 0.0;
   int status = DFM2G_OK;
-  const unsigned vb = reduce_blocks();
+  const unsigned vb = reduce_blocks(n);
   while (bnorm > 0) {
     double rr = 0;
     DFM2G_TRY(dot_host(n, r64, r64, DFM2G_F64, &rr));
