@@ -56,18 +56,18 @@ __global__ void __launch_bounds__(256) k_bsr_spmv(unsigned nblk, const unsigned 
 }
 
 // Same product in the component layout (spmv_tma_rows_c).
-template <typename T>
-__global__ void __launch_bounds__(TileCfgC<T>::kThreads, 1)
+template <typename T, int B>
+__global__ void __launch_bounds__(TileCfgC<T, B>::kThreads, 1)
     k_bsr_spmv_tma_c(const unsigned *__restrict__ tiles, unsigned ntiles, const unsigned *__restrict__ row_start,
                      const unsigned *__restrict__ col, const T *__restrict__ vcrs, const T *__restrict__ vdia,
                      T *__restrict__ y, T alpha, const T *__restrict__ x, T beta, int *err,
                      unsigned long long timeout_ns) {
   extern __shared__ __align__(128) unsigned char tma_smem[];
-  spmv_tma_rows_c<T>(tiles, ntiles, row_start, col, vcrs, vdia, x, err, timeout_ns, tma_smem,
-                     [&](unsigned row, unsigned a, T v) {
-                       T *py = y + (size_t)row * 3 + a;
-                       *py = beta * *py + alpha * v;
-                     });
+  spmv_tma_rows_c<T, B>(tiles, ntiles, row_start, col, vcrs, vdia, x, err, timeout_ns, tma_smem,
+                        [&](unsigned row, unsigned a, T v) {
+                          T *py = y + (size_t)row * B + a;
+                          *py = beta * *py + alpha * v;
+                        });
 }
 
 // Tiles of consecutive rows with at most `maxb` off-diagonal blocks and `maxr`
@@ -87,19 +87,19 @@ static bool make_tiles(const std::vector<unsigned> &rs, unsigned nblk, unsigned 
   return true;
 }
 
-int bsr_tiles_build(dfm2g_bsr_s *m) {
-  m->tiles_ok = false;
+template <int B>
+static int tiles_build(dfm2g_bsr_s *m) {
+  using C32 = TileCfgC<float, B>;
+  using C64 = TileCfgC<double, B>;
   std::vector<unsigned> t32, t64;
   // Fewer rows than fill the machine at full tiles: shorter tiles, down to one
   // consumer warp for each quarter of an SM, so that a tile's rows (a latency
   // chain of their own each) run on more SMs at once.
-  constexpr unsigned kLeast = 40;
-  const unsigned share = (m->nblk / (unsigned)ctx().num_sms + 10) / 10 * 10;
-  if (m->nblk == 0 ||
-      !make_tiles(m->h_row_start, m->nblk, TileCfgC<float>::kBlocks,
-                  std::min(std::max(share, kLeast), TileCfgC<float>::kRows), t32) ||
-      !make_tiles(m->h_row_start, m->nblk, TileCfgC<double>::kBlocks,
-                  std::min(std::max(share, kLeast), TileCfgC<double>::kRows), t64))
+  constexpr unsigned kWarpRows = C64::kWarpRows;
+  const unsigned share = (m->nblk / (unsigned)ctx().num_sms + kWarpRows) / kWarpRows * kWarpRows;
+  const unsigned least = std::max(share, 4 * kWarpRows);
+  if (!make_tiles(m->h_row_start, m->nblk, C32::kBlocks, std::min(least, C32::kRows), t32) ||
+      !make_tiles(m->h_row_start, m->nblk, C64::kBlocks, std::min(least, C64::kRows), t64))
     return DFM2G_OK;
   DFM2G_TRY(m->tiles32.resize(t32.size()));
   DFM2G_TRY(m->tiles64.resize(t64.size()));
@@ -111,16 +111,22 @@ int bsr_tiles_build(dfm2g_bsr_s *m) {
   DFM2G_CUDA(cudaMemsetAsync(m->err.p, 0, sizeof(int), stream()));
   static int attr_device = -1;  // opt the kernels in to their shared memory once per device
   if (attr_device != ctx().device) {
-    DFM2G_CUDA(cudaFuncSetAttribute(k_bsr_spmv_tma_c<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)TileCfgC<float>::kSmem));
-    DFM2G_CUDA(cudaFuncSetAttribute(k_bsr_spmv_tma_c<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)TileCfgC<double>::kSmem));
+    DFM2G_CUDA(cudaFuncSetAttribute(k_bsr_spmv_tma_c<float, B>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)C32::kSmem));
+    DFM2G_CUDA(cudaFuncSetAttribute(k_bsr_spmv_tma_c<double, B>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)C64::kSmem));
     attr_device = ctx().device;
   }
   m->ntiles32 = (unsigned)t32.size() - 1;
   m->ntiles64 = (unsigned)t64.size() - 1;
   m->tiles_ok = true;
   return DFM2G_OK;
+}
+
+int bsr_tiles_build(dfm2g_bsr_s *m) {
+  m->tiles_ok = false;
+  if (m->nblk == 0) return DFM2G_OK;
+  return m->ndim == 1 ? tiles_build<1>(m) : m->ndim == 2 ? tiles_build<2>(m) : tiles_build<3>(m);
 }
 
 // Reads and clears the SpMV error word (a bounded wait that gave up).
@@ -136,56 +142,39 @@ int bsr_check_err(dfm2g_bsr_s *m) {
   return DFM2G_OK;
 }
 
-template <typename T>
-static void nd_spmv_launch(dfm2g_bsr_s *m, const T *vcrs, const T *vdia, T *y, T alpha, const T *x, T beta) {
+template <typename T, int B>
+static void spmv_launch(dfm2g_bsr_s *m, const T *vcrs, const T *vdia, T *y, T alpha, const T *x, T beta) {
+  if (m->tiles_ok) {
+    using C = TileCfgC<T, B>;
+    const unsigned nt = sizeof(T) == 8 ? m->ntiles64 : m->ntiles32;
+    const unsigned *tiles = sizeof(T) == 8 ? m->tiles64.p : m->tiles32.p;
+    k_bsr_spmv_tma_c<T, B><<<std::min(nt, (unsigned)ctx().num_sms), C::kThreads, C::kSmem, stream()>>>(
+        tiles, nt, m->row_start.p, m->col.p, vcrs, vdia, y, alpha, x, beta, m->err.p, kWaitTimeoutNs);
+    return;
+  }
   const unsigned blocks = blocks_for((size_t)m->nblk * 32, 256, (unsigned)ctx().num_sms * 16);
-  if (m->ndim == 1)
-    k_nd_spmv<T, 1><<<blocks, 256, 0, stream()>>>(m->nblk, m->row_start.p, m->col.p, vcrs, vdia, y, alpha, x, beta);
+  if constexpr (B == 3)
+    k_bsr_spmv<T><<<blocks, 256, 0, stream()>>>(m->nblk, m->row_start.p, m->col.p, vcrs, vdia, y, alpha, x, beta);
   else
-    k_nd_spmv<T, 2><<<blocks, 256, 0, stream()>>>(m->nblk, m->row_start.p, m->col.p, vcrs, vdia, y, alpha, x, beta);
+    k_nd_spmv<T, B><<<blocks, 256, 0, stream()>>>(m->nblk, m->row_start.p, m->col.p, vcrs, vdia, y, alpha, x, beta);
+}
+
+template <typename T>
+static void spmv_launch(dfm2g_bsr_s *m, const T *vcrs, const T *vdia, T *y, T alpha, const T *x, T beta) {
+  if (m->ndim == 1)
+    spmv_launch<T, 1>(m, vcrs, vdia, y, alpha, x, beta);
+  else if (m->ndim == 2)
+    spmv_launch<T, 2>(m, vcrs, vdia, y, alpha, x, beta);
+  else
+    spmv_launch<T, 3>(m, vcrs, vdia, y, alpha, x, beta);
 }
 
 int bsr_spmv(dfm2g_bsr_s *m, int prec, void *y, double alpha, const void *x, double beta) {
-  if (m->ndim != 3) {
-    if (prec == DFM2G_F64) {
-      nd_spmv_launch<double>(m, m->vcrs.p, m->vdia.p, (double *)y, alpha, (const double *)x, beta);
-    } else if (prec == DFM2G_F32) {
-      DFM2G_TRY(bsr_ensure_f32(m));
-      nd_spmv_launch<float>(m, m->vcrs32.p, m->vdia32.p, (float *)y, (float)alpha, (const float *)x, (float)beta);
-    } else {
-      return fail(DFM2G_ERR_ARG, "matvec: prec must be DFM2G_F64 or DFM2G_F32");
-    }
-    note_launches(1);
-    DFM2G_LAUNCH_CHECK();
-    return DFM2G_OK;
-  }
-  if (m->tiles_ok && (prec == DFM2G_F64 || prec == DFM2G_F32)) {
-    const unsigned long long timeout = kWaitTimeoutNs;
-    if (prec == DFM2G_F64) {
-      const unsigned grid = std::min(m->ntiles64, (unsigned)ctx().num_sms);
-      k_bsr_spmv_tma_c<double><<<grid, TileCfgC<double>::kThreads, TileCfgC<double>::kSmem, stream()>>>(
-          m->tiles64.p, m->ntiles64, m->row_start.p, m->col.p, m->vcrs.p, m->vdia.p, (double *)y, alpha,
-          (const double *)x, beta, m->err.p, timeout);
-    } else {
-      DFM2G_TRY(bsr_ensure_f32(m));
-      const unsigned grid = std::min(m->ntiles32, (unsigned)ctx().num_sms);
-      k_bsr_spmv_tma_c<float><<<grid, TileCfgC<float>::kThreads, TileCfgC<float>::kSmem, stream()>>>(
-          m->tiles32.p, m->ntiles32, m->row_start.p, m->col.p, m->vcrs32.p, m->vdia32.p, (float *)y, (float)alpha,
-          (const float *)x, (float)beta, m->err.p, timeout);
-    }
-    note_launches(1);
-    DFM2G_LAUNCH_CHECK();
-    return DFM2G_OK;
-  }
-  const unsigned blocks = blocks_for((size_t)m->nblk * 32, 256, (unsigned)ctx().num_sms * 16);
   if (prec == DFM2G_F64) {
-    k_bsr_spmv<double><<<blocks, 256, 0, stream()>>>(m->nblk, m->row_start.p, m->col.p, m->vcrs.p,
-                                                    m->vdia.p, (double *)y, alpha, (const double *)x, beta);
+    spmv_launch<double>(m, m->vcrs.p, m->vdia.p, (double *)y, alpha, (const double *)x, beta);
   } else if (prec == DFM2G_F32) {
     DFM2G_TRY(bsr_ensure_f32(m));
-    k_bsr_spmv<float><<<blocks, 256, 0, stream()>>>(m->nblk, m->row_start.p, m->col.p, m->vcrs32.p,
-                                                   m->vdia32.p, (float *)y, (float)alpha,
-                                                   (const float *)x, (float)beta);
+    spmv_launch<float>(m, m->vcrs32.p, m->vdia32.p, (float *)y, (float)alpha, (const float *)x, (float)beta);
   } else {
     return fail(DFM2G_ERR_ARG, "matvec: prec must be DFM2G_F64 or DFM2G_F32");
   }
@@ -466,7 +455,7 @@ int dfm2g_bsr_set_pattern(dfm2g_bsr m, const unsigned *row_start, size_t n_row_s
   m->f32_valid = false;
   m->pattern_version++;
   m->tiles_ok = false;
-  if (m->ndim == 3) DFM2G_TRY(bsr_tiles_build(m));
+  DFM2G_TRY(bsr_tiles_build(m));
   DFM2G_CUDA(cudaStreamSynchronize(stream()));
   return DFM2G_OK;
 } catch (...) {

@@ -82,29 +82,6 @@ __global__ void __launch_bounds__(kThreads) k_spmv_pAp(IterState *st, unsigned n
   }
 }
 
-// The same in the component layout of spmv_tma_rows_c (the default when the
-// pattern has tiles).
-template <typename T>
-__global__ void __launch_bounds__(TileCfgC<T>::kThreads, 1)
-    k_spmv_pAp_tma_c(IterState *st, const unsigned *__restrict__ tiles, unsigned ntiles,
-                     const unsigned *__restrict__ row_start, const unsigned *__restrict__ col,
-                     const T *__restrict__ vcrs, const T *__restrict__ vdia, const T *__restrict__ p,
-                     T *__restrict__ Ap, double *partials, int *err, unsigned long long timeout_ns) {
-  extern __shared__ __align__(128) unsigned char tma_smem[];
-  __shared__ double sh[32];
-  if (st->done) return;
-  double dot = 0.0;
-  spmv_tma_rows_c<T>(tiles, ntiles, row_start, col, vcrs, vdia, p, err, timeout_ns, tma_smem,
-                     [&](unsigned row, unsigned a, T v) {
-                       Ap[(size_t)row * 3 + a] = v;
-                       dot += (double)(v * p[(size_t)row * 3 + a]);
-                     });
-  double total;
-  if (grid_sum_last(dot, partials, &st->ticket[0], sh, &total)) {
-    st->alpha = st->rPr / total;
-  }
-}
-
 // The same for 1x1 and 2x2 blocks (nd.cuh).
 template <typename T, int B>
 __global__ void __launch_bounds__(kThreads) k_spmv_pAp_nd(IterState *st, unsigned nblk,
@@ -137,20 +114,6 @@ static int launch_spmv_pAp(dfm2g_bsr_s *m, IterState *st, const T *vcrs, const T
   } else if (m->ndim == 2) {
     k_spmv_pAp_nd<T, 2><<<spmv_blocks, kThreads, 0, stream()>>>(st, m->nblk, m->row_start.p, m->col.p, vcrs, vdia, pv,
                                                                Ap, partials);
-  } else if (m->tiles_ok) {
-    using C = TileCfgC<T>;
-    static int attr_device = -1;  // per instantiation, once per device
-    if (attr_device != ctx().device) {
-      DFM2G_CUDA(cudaFuncSetAttribute(k_spmv_pAp_tma_c<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)C::kSmem));
-      attr_device = ctx().device;
-    }
-    const unsigned nt = sizeof(T) == 8 ? m->ntiles64 : m->ntiles32;
-    const unsigned *tiles = sizeof(T) == 8 ? m->tiles64.p : m->tiles32.p;
-    const unsigned grid = std::min(nt, (unsigned)ctx().num_sms);
-    k_spmv_pAp_tma_c<T><<<grid, C::kThreads, C::kSmem, stream()>>>(st, tiles, nt, m->row_start.p, m->col.p, vcrs,
-                                                                     vdia, pv, Ap, partials, m->err.p,
-                                                                     kWaitTimeoutNs);
   } else {
     k_spmv_pAp<T><<<spmv_blocks, kThreads, 0, stream()>>>(st, m->nblk, m->row_start.p, m->col.p, vcrs, vdia, pv, Ap,
                                                          partials);
@@ -235,11 +198,12 @@ __global__ void __launch_bounds__(kThreads) k_true_residual(IterState *st, unsig
 }
 
 // Both parts of the reliable update in one cooperative launch (k_flush_x,
-// k_true_residual) for 3x3 patterns with SpMV tiles, only when a refresh is
+// k_true_residual) for patterns with SpMV tiles, only when a refresh is
 // due: x64 += x32 / scale and x32 = 0 over the CTA's grid-stride share, a
 // meeting of all CTAs, then r64 = b - K64 x64 through the TMA-staged
-// component-layout product (spmv_tma_rows_c<double>).
-__global__ void __launch_bounds__(TileCfgC<double>::kThreads, 1)
+// component-layout product (spmv_tma_rows_c<double, B>).
+template <int B>
+__global__ void __launch_bounds__(TileCfgC<double, B>::kThreads, 1)
     k_refresh_tma(IterState *st, const unsigned *__restrict__ tiles, unsigned ntiles,
                   const unsigned *__restrict__ row_start, const unsigned *__restrict__ col,
                   const double *__restrict__ vcrs, const double *__restrict__ vdia, double *x64, float *x32,
@@ -259,15 +223,15 @@ __global__ void __launch_bounds__(TileCfgC<double>::kThreads, 1)
     return;
   }
   double rr = 0.0, dd = 0.0;
-  spmv_tma_rows_c<double>(tiles, ntiles, row_start, col, vcrs, vdia, x64, err, timeout_ns, tma_smem,
-                          [&](unsigned row, unsigned a, double v) {
-                            const size_t k = (size_t)row * 3 + a;
-                            const double r = b[k] - v;
-                            const double gap = r - (double)r32[k] * inv_old;  // true minus recursive residual
-                            r32[k] = (float)(r * sc);
-                            rr += r * r;
-                            dd += gap * gap;
-                          });
+  spmv_tma_rows_c<double, B>(tiles, ntiles, row_start, col, vcrs, vdia, x64, err, timeout_ns, tma_smem,
+                             [&](unsigned row, unsigned a, double v) {
+                               const size_t k = (size_t)row * B + a;
+                               const double r = b[k] - v;
+                               const double gap = r - (double)r32[k] * inv_old;  // true minus recursive residual
+                               r32[k] = (float)(r * sc);
+                               rr += r * r;
+                               dd += gap * gap;
+                             });
   refresh_tail(st, rr, dd, partials, sh, sh2);
 }
 
@@ -394,13 +358,13 @@ __global__ void __launch_bounds__(kThreads) k_update(IterState *st, size_t n, T 
   if (grid_sum_last(rr, partials, &st->ticket[1], sh, &total)) update_tail(st, total, hist);
 }
 
-// The SpMV with p.Ap (component layout, k_spmv_pAp_tma_c) and the update
+// The SpMV with p.Ap (component layout, spmv_tma_rows_c) and the update
 // (k_update) in one cooperative launch: the CTAs meet once to add the p.Ap
 // partials (each CTA adds them in the same order, so every CTA has the same
 // alpha), then update their grid-stride share of r and x. The |r|^2 partials
 // go to partials[gridDim.x, 2 gridDim.x).
-template <typename T>
-__global__ void __launch_bounds__(TileCfgC<T>::kThreads, 1)
+template <typename T, int B>
+__global__ void __launch_bounds__(TileCfgC<T, B>::kThreads, 1)
     k_spmv_update_tma_c(IterState *st, const unsigned *__restrict__ tiles, unsigned ntiles,
                         const unsigned *__restrict__ row_start, const unsigned *__restrict__ col,
                         const T *__restrict__ vcrs, const T *__restrict__ vdia, const T *p, T *Ap, T *r, T *x,
@@ -410,11 +374,11 @@ __global__ void __launch_bounds__(TileCfgC<T>::kThreads, 1)
   __shared__ double sh[32];
   if (st->done) return;
   double dot = 0.0;
-  spmv_tma_rows_c<T>(tiles, ntiles, row_start, col, vcrs, vdia, p, err, timeout_ns, tma_smem,
-                     [&](unsigned row, unsigned a, T v) {
-                       Ap[(size_t)row * 3 + a] = v;
-                       dot += (double)(v * p[(size_t)row * 3 + a]);
-                     });
+  spmv_tma_rows_c<T, B>(tiles, ntiles, row_start, col, vcrs, vdia, p, err, timeout_ns, tma_smem,
+                        [&](unsigned row, unsigned a, T v) {
+                          Ap[(size_t)row * B + a] = v;
+                          dot += (double)(v * p[(size_t)row * B + a]);
+                        });
   dot = block_sum(dot, sh);
   if (threadIdx.x == 0) partials[blockIdx.x] = dot;
   if (!grid_barrier(bar, err, timeout_ns)) {
@@ -683,6 +647,14 @@ static int allow_tma_smem(K kernel, size_t smem, int &attr_device) {
   return DFM2G_OK;
 }
 
+// Shared memory of the tiled row products (their CTAs have as many threads for every block size).
+template <typename T>
+static size_t tile_smem(unsigned ndim) {
+  static_assert(TileCfgC<T, 1>::kThreads == TileCfgC<T, 3>::kThreads, "one CTA size");
+  static_assert(TileCfgC<T, 2>::kThreads == TileCfgC<T, 3>::kThreads, "one CTA size");
+  return ndim == 1 ? TileCfgC<T, 1>::kSmem : ndim == 2 ? TileCfgC<T, 2>::kSmem : TileCfgC<T, 3>::kSmem;
+}
+
 // CTAs of k_dot_pupdate<T>: reduce_blocks(n), or as many as are resident at once.
 template <typename T>
 static int dot_pupdate_blocks(size_t n, unsigned *grid) {
@@ -752,20 +724,24 @@ static int pcg_core(dfm2g_bsr_s *m, dfm2g_ilu_s *p, T *r, T *x, T *w0, T *w1, T 
   const unsigned spmv_blocks = blocks_for((size_t)nblk * 32, kThreads, (unsigned)ctx().num_sms * 8);
   const unsigned vec_blocks = reduce_blocks(n);
   const int chunk = 16;
-  // 3x3 patterns with SpMV tiles: two cooperative launches besides the SpMV
-  // and the sweeps per iteration (k_spmv_update_tma_c, k_dot_pupdate) and the
-  // refresh (k_refresh_tma) only does work when one is due; otherwise five
+  // Patterns with SpMV tiles: two cooperative launches besides the sweeps per
+  // iteration (k_spmv_update_tma_c, k_dot_pupdate) and the refresh
+  // (k_refresh_tma) only does work when one is due; otherwise five
   // (k_spmv_pAp*, k_update, k_flush_x + k_true_residual*, k_dot_beta, k_p_update).
-  const bool fused = m->ndim == 3 && m->tiles_ok;
-  using CT = TileCfgC<T>;
-  using C64 = TileCfgC<double>;
+  const bool fused = m->tiles_ok;
+  auto *k_sp = m->ndim == 1   ? k_spmv_update_tma_c<T, 1>
+               : m->ndim == 2 ? k_spmv_update_tma_c<T, 2>
+                              : k_spmv_update_tma_c<T, 3>;
+  auto *k_re = m->ndim == 1 ? k_refresh_tma<1> : m->ndim == 2 ? k_refresh_tma<2> : k_refresh_tma<3>;
+  const size_t smem_T = tile_smem<T>(m->ndim), smem_64 = tile_smem<double>(m->ndim);
+  constexpr unsigned threads_T = TileCfgC<T, 3>::kThreads, threads_64 = TileCfgC<double, 3>::kThreads;
   const unsigned nt_T = sizeof(T) == 8 ? m->ntiles64 : m->ntiles32;
   const unsigned *tiles_T = sizeof(T) == 8 ? m->tiles64.p : m->tiles32.p;
   unsigned dp_grid = 0;
   if (fused) {
-    static int attr_a = -1, attr_r = -1;
-    DFM2G_TRY(allow_tma_smem(k_spmv_update_tma_c<T>, CT::kSmem, attr_a));
-    DFM2G_TRY(allow_tma_smem(k_refresh_tma, C64::kSmem, attr_r));
+    static int attr_a[3] = {-1, -1, -1}, attr_r[3] = {-1, -1, -1};
+    DFM2G_TRY(allow_tma_smem(k_sp, smem_T, attr_a[m->ndim - 1]));
+    DFM2G_TRY(allow_tma_smem(k_re, smem_64, attr_r[m->ndim - 1]));
     DFM2G_TRY(dot_pupdate_blocks<T>(n, &dp_grid));
   }
   for (;;) {
@@ -776,10 +752,10 @@ static int pcg_core(dfm2g_bsr_s *m, dfm2g_ilu_s *p, T *r, T *x, T *w0, T *w1, T 
       T *fa = fill ? mid : nullptr, *fb = fill ? Pr : nullptr;
       if (fused) {
         ProfScope ps(DFM2G_PROF_SPMV, 1);
-        DFM2G_TRY(coop_launch(k_spmv_update_tma_c<T>, std::min(nt_T, (unsigned)ctx().num_sms), CT::kThreads,
-                              CT::kSmem, st, tiles_T, nt_T, (const unsigned *)m->row_start.p,
-                              (const unsigned *)m->col.p, vcrs, vdia, (const T *)pv, Ap, r, x, n, g_ws.partials.p,
-                              g_ws.hist.p, fa, fb, g_ws.bar.p, m->err.p, kWaitTimeoutNs));
+        DFM2G_TRY(coop_launch(k_sp, std::min(nt_T, (unsigned)ctx().num_sms), threads_T, smem_T, st, tiles_T, nt_T,
+                              (const unsigned *)m->row_start.p, (const unsigned *)m->col.p, vcrs, vdia,
+                              (const T *)pv, Ap, r, x, n, g_ws.partials.p, g_ws.hist.p, fa, fb, g_ws.bar.p, m->err.p,
+                              kWaitTimeoutNs));
       } else {
         {
           ProfScope ps(DFM2G_PROF_SPMV, 1);
@@ -794,11 +770,11 @@ static int pcg_core(dfm2g_bsr_s *m, dfm2g_ilu_s *p, T *r, T *x, T *w0, T *w1, T 
       if constexpr (sizeof(T) == 4) {
         if (mode == 2 && fused) {
           ProfScope ps(DFM2G_PROF_OUTER, 1);
-          DFM2G_TRY(coop_launch(k_refresh_tma, std::min(m->ntiles64, (unsigned)ctx().num_sms), C64::kThreads,
-                                C64::kSmem, st, (const unsigned *)m->tiles64.p, m->ntiles64,
-                                (const unsigned *)m->row_start.p, (const unsigned *)m->col.p,
-                                (const double *)m->vcrs.p, (const double *)m->vdia.p, rf.x64, (float *)x, rf.b64,
-                                (float *)r, n, g_ws.partials.p, g_ws.bar.p, m->err.p, kWaitTimeoutNs));
+          DFM2G_TRY(coop_launch(k_re, std::min(m->ntiles64, (unsigned)ctx().num_sms), threads_64, smem_64, st,
+                                (const unsigned *)m->tiles64.p, m->ntiles64, (const unsigned *)m->row_start.p,
+                                (const unsigned *)m->col.p, (const double *)m->vcrs.p, (const double *)m->vdia.p,
+                                rf.x64, (float *)x, rf.b64, (float *)r, n, g_ws.partials.p, g_ws.bar.p, m->err.p,
+                                kWaitTimeoutNs));
         } else if (mode == 2) {
           ProfScope ps(DFM2G_PROF_OUTER, 2);
           k_flush_x<<<vec_blocks, kThreads, 0, stream()>>>(st, n, rf.x64, (float *)x);

@@ -1,4 +1,4 @@
-// TMA-staged 3x3 block SpMV: warp-specialised, persistent.
+// TMA-staged block SpMV (1x1, 2x2 and 3x3 blocks): warp-specialised, persistent.
 //
 // The block rows are cut into tiles of consecutive rows (at most kBlocks
 // off-diagonal blocks and kRows rows each; tile table built on the host from
@@ -25,14 +25,16 @@ __device__ __forceinline__ void round16(size_t off, size_t end, size_t &a, unsig
 }
 
 // ---------------------------------------------------------------------------
-// Component layout: lane 3q + a of a consumer warp computes component a of
-// row q of the warp's ten rows, summing K_b[a][0..2] x_b over the row's
-// blocks with no cross-lane reduction. A warp instruction then serves ten rows,
-// so the kernel issues a fraction of the instructions per row (and, in FP64, of
-// the FP64 instructions) of a layout with a warp per row. Tiles hold ten rows
-// per consumer warp and are double-buffered; the tile's row offsets are staged
+// Component layout: lane B q + a of a consumer warp computes component a of
+// row q of the warp's 32 / B rows, summing K_b[a][0..B-1] x_b over the row's
+// blocks with no cross-lane reduction. A warp instruction then serves 10 rows of
+// 3x3 blocks (16 of 2x2, 32 of 1x1), so the kernel issues a fraction of the
+// instructions per row (and, in FP64, of the FP64 instructions) of a layout with
+// a warp or eight lanes per row and a shuffle tree. Tiles hold 32 / B rows per
+// consumer warp and are double-buffered; the tile's row offsets are staged
 // with its values, block columns and diagonal blocks. FP32: 15 consumer warps
-// (150-row tiles), one CTA per SM.
+// (150-row tiles of 3x3 blocks), one CTA per SM. Tiles of 1x1 and 2x2 rows are
+// sized for 16 blocks a row, which leaves the L1 cache room for x.
 //
 // FP64: a quarter of an SM issues one FP64 warp instruction per 64 cycles, so
 // the product is bound by their number and by how evenly the warps cover the
@@ -41,7 +43,8 @@ __device__ __forceinline__ void round16(size_t off, size_t end, size_t &a, unsig
 // sums over whole blocks take a fourth instruction, the addition, per block).
 // The rounding error is no larger: root mean square 0.299 against 0.305 units
 // of 1e-16 |K||x| over 14-block rows that cancel, 0.180 against 0.212 on smooth
-// vectors.
+// vectors. 1x1 and 2x2 rows sum the same way in both types: no more error than
+// eight lanes' sums and a tree (0.432 against 0.520 units over 14 random terms).
 #ifndef DFM2G_SPMV_F32_CONSUMERS
 #define DFM2G_SPMV_F32_CONSUMERS 15u  // FP32 tile: consumer warps (ten rows each)
 #endif
@@ -51,16 +54,17 @@ __device__ __forceinline__ void round16(size_t off, size_t end, size_t &a, unsig
 #ifndef DFM2G_SPMV_F32_STAGES
 #define DFM2G_SPMV_F32_STAGES 2u  // FP32 ring stages
 #endif
-template <typename T>
+template <typename T, int B>
 struct TileCfgC {
   static constexpr unsigned kConsumers = sizeof(T) == 8 ? 8u : DFM2G_SPMV_F32_CONSUMERS;
   static constexpr unsigned kThreads = 32u * (kConsumers + 1u);
-  static constexpr unsigned kRows = kConsumers * 10u;
-  static constexpr unsigned kBlocks = sizeof(T) == 8 ? 1424u : DFM2G_SPMV_F32_BLOCKS;
+  static constexpr unsigned kWarpRows = 32u / B;
+  static constexpr unsigned kRows = kConsumers * kWarpRows;
+  static constexpr unsigned kBlocks = B < 3 ? kRows * 16u : sizeof(T) == 8 ? 1424u : DFM2G_SPMV_F32_BLOCKS;
   static constexpr unsigned kStages = sizeof(T) == 8 ? 2u : DFM2G_SPMV_F32_STAGES;
-  static constexpr unsigned kValBytes = kBlocks * 9 * sizeof(T) + 32;
+  static constexpr unsigned kValBytes = kBlocks * B * B * sizeof(T) + 32;
   static constexpr unsigned kColBytes = kBlocks * 4 + 32;
-  static constexpr unsigned kDiaBytes = (kRows * 9 * sizeof(T) + 32 + 15) / 16 * 16;
+  static constexpr unsigned kDiaBytes = (kRows * B * B * sizeof(T) + 32 + 15) / 16 * 16;
   static constexpr unsigned kRsBytes = ((kRows + 1) * 4 + 32 + 15) / 16 * 16;
   static constexpr unsigned kStageBytes = kValBytes + kColBytes + kDiaBytes + kRsBytes;
   static constexpr unsigned kBarBytes = 128;
@@ -71,16 +75,16 @@ struct TileCfgC {
 };
 
 // Runs the pipeline over all tiles; epi(row, a, v) is called by the lane that
-// computed component a of `row` (v = (K x)_{3 row + a}). Must be called by all
-// TileCfgC<T>::kThreads threads of the CTA; `smem` holds TileCfgC<T>::kSmem bytes.
-template <typename T, typename Epi>
+// computed component a of `row` (v = (K x)_{B row + a}). Must be called by all
+// TileCfgC<T, B>::kThreads threads of the CTA; `smem` holds TileCfgC<T, B>::kSmem bytes.
+template <typename T, int B, typename Epi>
 __device__ __forceinline__ void spmv_tma_rows_c(const unsigned *__restrict__ tiles, unsigned ntiles,
                                                 const unsigned *__restrict__ row_start,
                                                 const unsigned *__restrict__ col, const T *__restrict__ vcrs,
                                                 const T *__restrict__ vdia, const T *__restrict__ x, int *err,
                                                 unsigned long long timeout_ns, unsigned char *smem, Epi &&epi) {
-  using C = TileCfgC<T>;
-  constexpr size_t B9 = 9 * sizeof(T);  // bytes of one 3x3 block
+  using C = TileCfgC<T, B>;
+  constexpr size_t BB = B * B, kBlk = BB * sizeof(T);  // values, bytes of one block
   uint64_t *full = reinterpret_cast<uint64_t *>(smem);
   uint64_t *empty = full + C::kStages;
   unsigned char *ring = smem + C::kBarBytes;
@@ -109,9 +113,9 @@ __device__ __forceinline__ void spmv_tma_rows_c(const unsigned *__restrict__ til
       unsigned char *st = ring + (size_t)s * C::kStageBytes;
       size_t av, ac, ad, ar;
       unsigned lv, lc, ld, lr;
-      round16((size_t)b0 * B9, (size_t)b1 * B9, av, lv);
+      round16((size_t)b0 * kBlk, (size_t)b1 * kBlk, av, lv);
       round16((size_t)b0 * 4, (size_t)b1 * 4, ac, lc);
-      round16((size_t)r0 * B9, (size_t)r1 * B9, ad, ld);
+      round16((size_t)r0 * kBlk, (size_t)r1 * kBlk, ad, ld);
       round16((size_t)r0 * 4, (size_t)(r1 + 1) * 4, ar, lr);
       mbar_arrive_expect_tx(&full[s], lv + lc + ld + lr);
       if (lv) tma_load_1d(st, reinterpret_cast<const unsigned char *>(vcrs) + av, lv, &full[s]);
@@ -125,7 +129,7 @@ __device__ __forceinline__ void spmv_tma_rows_c(const unsigned *__restrict__ til
     for (unsigned j = first; j < k; ++j) mbar_wait_bounded(&full[j % C::kStages], (j / C::kStages) & 1u, timeout_ns);
     return;
   }
-  const unsigned q = lane / 3u, a = lane - 3u * q;
+  const unsigned q = lane / B, a = lane - B * q;
   unsigned k = 0;
   for (unsigned t = blockIdx.x; t < ntiles; t += G, ++k) {
     const unsigned s = k % C::kStages;
@@ -138,40 +142,56 @@ __device__ __forceinline__ void spmv_tma_rows_c(const unsigned *__restrict__ til
     const unsigned *rsv = reinterpret_cast<const unsigned *>(st + C::kValBytes + C::kColBytes + C::kDiaBytes +
                                                              (((size_t)r0 * 4) & 15));
     const unsigned b0 = rsv[0];
-    const T *vv = reinterpret_cast<const T *>(st + (((size_t)b0 * B9) & 15));
+    const T *vv = reinterpret_cast<const T *>(st + (((size_t)b0 * kBlk) & 15));
     const unsigned *cv = reinterpret_cast<const unsigned *>(st + C::kValBytes + (((size_t)b0 * 4) & 15));
-    const T *dv = reinterpret_cast<const T *>(st + C::kValBytes + C::kColBytes + (((size_t)r0 * B9) & 15));
-    const unsigned i = r0 + warp * 10u + q;
-    if (lane < 30 && i < r1) {
+    const T *dv = reinterpret_cast<const T *>(st + C::kValBytes + C::kColBytes + (((size_t)r0 * kBlk) & 15));
+    const unsigned i = r0 + warp * C::kWarpRows + q;
+    if (lane < C::kWarpRows * B && i < r1) {
       const unsigned s0 = rsv[i - r0] - b0, s1 = rsv[i - r0 + 1] - b0;
-      const T *d = dv + (size_t)(i - r0) * 9 + a * 3, *xi = x + (size_t)i * 3;
+      const T *d = dv + (size_t)(i - r0) * BB + a * B, *xi = x + (size_t)i * B;
       unsigned u = s0;
-      if constexpr (sizeof(T) == 8) {
-        T e0 = T(0), e1 = T(0), e2 = T(0), o0 = T(0), o1 = T(0), o2 = T(0);
-        if ((s1 - u) & 1u) {
-          const T *v0 = vv + (size_t)u * 9 + a * 3, *x0 = x + (size_t)cv[u] * 3;
-          e0 = v0[0] * __ldg(x0), e1 = v0[1] * __ldg(x0 + 1), e2 = v0[2] * __ldg(x0 + 2);
-          ++u;
-        }
-        // two blocks per step, the next two's x gathered under this step's products
-        T g[6] = {};
+      if constexpr (sizeof(T) == 8 || B < 3) {
+        constexpr unsigned W = B == 3 ? 2 : 4;  // blocks per step
+        T e[B] = {}, o[B] = {};                 // sums over the blocks of either parity
+        // the next step's x gathered under this step's products, the first
+        // step's under the row's remainder
+        T g[W * B] = {};
         auto gather = [&](unsigned k) {
-          const T *x0 = x + (size_t)cv[k] * 3, *x1 = x + (size_t)cv[k + 1] * 3;
 #pragma unroll
-          for (int c = 0; c < 3; ++c) g[c] = __ldg(x0 + c), g[3 + c] = __ldg(x1 + c);
+          for (unsigned w = 0; w < W; ++w)
+#pragma unroll
+            for (unsigned c = 0; c < B; ++c) g[w * B + c] = __ldg(x + (size_t)cv[k + w] * B + c);
         };
-        if (u < s1) gather(u);
+        const unsigned rem = (s1 - s0) % W;
+        if (s0 + rem < s1) gather(s0 + rem);
+#pragma unroll
+        for (unsigned w = 0; w + 1 < W; ++w) {
+          if (w < rem) {
+            const T *v = vv + (size_t)u * BB + a * B, *y = x + (size_t)cv[u] * B;
+#pragma unroll
+            for (unsigned c = 0; c < B; ++c) (w & 1 ? o : e)[c] += v[c] * __ldg(y + c);
+            ++u;
+          }
+        }
         while (u < s1) {
-          const T *v0 = vv + (size_t)u * 9 + a * 3, *v1 = v0 + 9;
-          const T h[6] = {g[0], g[1], g[2], g[3], g[4], g[5]};
-          u += 2;
+          const T *v = vv + (size_t)u * BB + a * B;
+          T h[W * B];
+#pragma unroll
+          for (unsigned k = 0; k < W * B; ++k) h[k] = g[k];
+          u += W;
           if (u < s1) gather(u);
-          e0 += v0[0] * h[0], e1 += v0[1] * h[1], e2 += v0[2] * h[2];
-          o0 += v1[0] * h[3], o1 += v1[1] * h[4], o2 += v1[2] * h[5];
+#pragma unroll
+          for (unsigned w = 0; w < W; ++w)
+#pragma unroll
+            for (unsigned c = 0; c < B; ++c) (w & 1 ? o : e)[c] += v[w * BB + c] * h[w * B + c];
         }
         // the diagonal block, the largest terms, last: fewer sums are rounded at its size
-        o0 += d[0] * __ldg(xi), o1 += d[1] * __ldg(xi + 1), o2 += d[2] * __ldg(xi + 2);
-        epi(i, a, ((e0 + e1) + e2) + ((o0 + o1) + o2));
+#pragma unroll
+        for (unsigned c = 0; c < B; ++c) o[c] += d[c] * __ldg(xi + c);
+        T se = e[0], so = o[0];
+#pragma unroll
+        for (unsigned c = 1; c < B; ++c) se += e[c], so += o[c];
+        epi(i, a, se + so);
       } else {
         T acc0 = T(0), acc1 = T(0);
         for (; u + 1 < s1; u += 2) {

@@ -81,7 +81,7 @@ def test_solves(gpu, n, ndim):
     ind, col, row, val, dia = s
     K = _matrix(ind, col, val, dia, ndim)
     ilu = D.CPreconditionerILU()
-    ilu.Initialize_ILU0(K)
+    ilu.Initialize_ILUk(K, 0)
     ilu.CopyValue(K)
     assert ilu.Decompose()
     b = np.random.default_rng(9).standard_normal(n * ndim)
