@@ -308,7 +308,8 @@ __device__ __forceinline__ void tet_stress(const double G[9], double lam, double
   S[5] = myu * (G[6] + G[2]);
 }
 
-// One thread per tet: S of w = u (kStatic), u + dt v (kBEuler), u + dt v + dt^2/2 acc (kNewmark).
+// One thread per tet: S of w = u (kStatic), u + dt v (kBEuler), u + dt v + dt^2/2 acc (kNewmark);
+// kWarp: G of w = u + dt v itself, nine values, as each node of the tet turns it its own way.
 template <int MODE>
 __global__ void __launch_bounds__(128) k_tet_stress(size_t ntet, const unsigned *__restrict__ tet,
                                                     const double *__restrict__ geo, const TetParam p,
@@ -330,6 +331,11 @@ __global__ void __launch_bounds__(128) k_tet_stress(size_t ntet, const unsigned 
         for (int c = 0; c < 3; ++c) G[r * 3 + c] += w * d[c];
       }
     }
+    if (MODE == kWarp) {
+#pragma unroll
+      for (int q = 0; q < 9; ++q) stress[e * 9 + q] = G[q];
+      continue;
+    }
     const double w = MODE == kStatic ? p.young[e] * vol : vol;
     double S[6];
     tet_stress(G, w * p.lam, w * p.myu, S);
@@ -340,18 +346,21 @@ __global__ void __launch_bounds__(128) k_tet_stress(size_t ntet, const unsigned 
   }
 }
 
-// One thread per node: the diagonal block and the right-hand side.
-template <int MODE>
+// The diagonal block and the right-hand side of a node, summed by LN lanes
+// (each takes every LN-th tet; a shuffle tree adds their sums). A thread per
+// node of a small mesh leaves most of the machine idle while each runs some 24
+// tets of FP64 one after the other: LN doubles until there is a warp for each
+// SM quarter (an FP64 warp instruction takes a quarter 64 cycles, so more warps
+// would not help).
+template <int MODE, int LN>
 __global__ void __launch_bounds__(128) k_tet_nodes(unsigned np, const unsigned *__restrict__ noff, unsigned total,
                                                    const unsigned *__restrict__ nlist,
-                                                   const unsigned *__restrict__ tet, const double *__restrict__ xyz,
-                                                   const double *__restrict__ geo,
+                                                   const unsigned *__restrict__ tet, const double *__restrict__ geo,
                                                    const double *__restrict__ stress, const TetParam p, double *vdia,
                                                    double *rhs) {
-  const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= np) return;
+  const unsigned t = blockIdx.x * blockDim.x + threadIdx.x, sub = t % LN, i0 = t / LN;
+  const unsigned i = i0 < np ? i0 : np - 1;
   const unsigned l0 = noff[i], l1 = i + 1 < np ? noff[i + 1] : total;
-  if (l0 == l1) return;
   double X[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, vsum = 0.0, vmass = 0.0, f[3] = {0, 0, 0}, macc[3] = {0, 0, 0};
   double skew[3] = {0, 0, 0};
   double R[9];
@@ -359,7 +368,7 @@ __global__ void __launch_bounds__(128) k_tet_nodes(unsigned np, const unsigned *
 #pragma unroll
     for (int q = 0; q < 9; ++q) R[q] = p.rot[(size_t)i * 9 + q];
   }
-  for (unsigned l = l0; l < l1; ++l) {
+  for (unsigned l = l0 + sub; l < l1; l += LN) {
     const unsigned code = nlist[l], e = code >> 4, ia = (code >> 2) & 3u, ib = code & 3u;
     double a[3], vol;
     tet_grad(geo, e, ia, a, &vol);
@@ -384,25 +393,15 @@ __global__ void __launch_bounds__(128) k_tet_nodes(unsigned np, const unsigned *
     if (ia != ib) continue;
     vsum += vol;
     if (MODE == kWarp) {
-      double G[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+      // G = sum_q R^T (P_q + u_q + dt v_q - R P_q) dN_q^T = R^T (I + U - R), as
+      // sum_q P_q dN_q^T = I, with U of k_tet_stress: 27 products instead of 130
+      double H[9], G[9];
 #pragma unroll
-      for (unsigned q = 0; q < 4; ++q) {
-        const size_t n = (size_t)tet[(size_t)e * 4 + q] * 3;
-        double d[3], v, x[3], P[3];
-        tet_grad(geo, e, q, d, &v);
+      for (int q = 0; q < 9; ++q) H[q] = __ldg(stress + (size_t)e * 9 + q) + ((q % 4 == 0 ? 1.0 : 0.0) - R[q]);
 #pragma unroll
-        for (int r = 0; r < 3; ++r) P[r] = xyz[n + r];
+      for (int r = 0; r < 3; ++r)
 #pragma unroll
-        for (int r = 0; r < 3; ++r)
-          x[r] = P[r] + p.disp[n + r] + p.dt * p.velo[n + r] -
-                 (R[r * 3] * P[0] + R[r * 3 + 1] * P[1] + R[r * 3 + 2] * P[2]);
-#pragma unroll
-        for (int r = 0; r < 3; ++r) {
-          const double y = R[r] * x[0] + R[3 + r] * x[1] + R[6 + r] * x[2];  // R^T (P + u + dt v - R P)
-#pragma unroll
-          for (int c = 0; c < 3; ++c) G[r * 3 + c] += y * d[c];
-        }
-      }
+        for (int c = 0; c < 3; ++c) G[r * 3 + c] = R[r] * H[c] + R[3 + r] * H[3 + c] + R[6 + r] * H[6 + c];
       double S[6];
       tet_stress(G, vol * p.lam, vol * p.myu, S);
       f[0] += S[0] * a[0] + S[3] * a[1] + S[5] * a[2];
@@ -425,6 +424,23 @@ __global__ void __launch_bounds__(128) k_tet_nodes(unsigned np, const unsigned *
       }
     }
   }
+  if (LN > 1) {
+    auto add = [](double &v) {
+#pragma unroll
+      for (int o = 1; o < LN; o *= 2) v += __shfl_xor_sync(0xffffffffu, v, o);
+    };
+#pragma unroll
+    for (int q = 0; q < 9; ++q)
+      if (q % 3 >= q / 3) add(X[q]);
+    add(vmass), add(vsum);
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      add(f[r]);
+      if (MODE == kStatic) add(skew[r]);
+      if (MODE == kNewmark) add(macc[r]);
+    }
+  }
+  if (sub != 0 || i0 >= np || l0 == l1) return;
   X[3] = X[1] + skew[0];
   X[6] = X[2] + skew[1];
   X[7] = X[5] + skew[2];
@@ -620,8 +636,8 @@ template <int MODE>
 static int tet_assemble(dfm2g_tetmesh_s *t, dfm2g_bsr_s *m, const TetParam &p, double *b) {
   if (t->ntet == 0) return DFM2G_OK;
   const double *stress = nullptr;
-  if (MODE != kWarp && p.disp) {
-    DFM2G_TRY(t->stress.ensure(t->ntet * 6 + 2));
+  if (p.disp) {
+    DFM2G_TRY(t->stress.ensure(t->ntet * (MODE == kWarp ? 9 : 6) + 2));
     k_tet_stress<MODE><<<blocks_for(t->ntet, 128), 128, 0, stream()>>>(t->ntet, t->tet.p, t->geo.p, p, t->stress.p);
     stress = t->stress.p;
   }
@@ -629,9 +645,20 @@ static int tet_assemble(dfm2g_tetmesh_s *t, dfm2g_bsr_s *m, const TetParam &p, d
     k_tet_edges<MODE><<<blocks_for(t->nedge, 128), 128, 0, stream()>>>(t->nedge, t->eslot.p, t->eoff.p,
                                                                       t->nedge_entries, t->elist.p, t->slot.p,
                                                                       t->tet.p, t->geo.p, p, m->vcrs.p);
-  k_tet_nodes<MODE><<<blocks_for(t->np, 128), 128, 0, stream()>>>((unsigned)t->np, t->noff.p, t->nnode_entries,
-                                                                 t->nlist.p, t->tet.p, t->xyz.p, t->geo.p, stress, p,
-                                                                 m->vdia.p, b);
+  const size_t quarters = (size_t)ctx().num_sms * 4 * 32;  // threads at a warp for each SM quarter
+  auto nodes = [&](auto *kernel, unsigned lanes) {
+    kernel<<<blocks_for(t->np * lanes, 128), 128, 0, stream()>>>((unsigned)t->np, t->noff.p, t->nnode_entries,
+                                                                t->nlist.p, t->tet.p, t->geo.p, stress, p, m->vdia.p,
+                                                                b);
+  };
+  if (t->np * 8 <= quarters)
+    nodes(k_tet_nodes<MODE, 8>, 8);
+  else if (t->np * 4 <= quarters)
+    nodes(k_tet_nodes<MODE, 4>, 4);
+  else if (t->np * 2 <= quarters)
+    nodes(k_tet_nodes<MODE, 2>, 2);
+  else
+    nodes(k_tet_nodes<MODE, 1>, 1);
   note_launches(stress ? 3 : 2);
   DFM2G_LAUNCH_CHECK();
   m->f32_valid = false;
