@@ -8,7 +8,7 @@
 // beta = (r, r0*) alpha / ((r, r0*)_old omega), p = beta p + r - beta omega A Mp.
 // The scalars live on the device: each pair of dot products is one
 // deterministic grid reduction whose last block applies the step's scalar
-// update. The host reads the state once per iteration.
+// update; (r, r0*) of the next iteration is the one beta took. The host reads the state once per iteration.
 #include <cmath>
 
 #include "common.cuh"
@@ -25,20 +25,13 @@ struct BiState {
 };
 
 constexpr int kBiThreads = 256;
-enum { kOpInit = 0, kOpRR2 = 1, kOpAlpha = 2, kOpOmega = 3, kOpConvBeta = 4 };
+enum { kOpInit, kOpAlpha, kOpOmega, kOpConvBeta };
 
+// The two sums over the grid (the last block has them) and the step's scalar update.
 template <int OP>
-__global__ void __launch_bounds__(kBiThreads) k_bi_dots(size_t n, const double *__restrict__ a1,
-                                                        const double *__restrict__ b1, const double *__restrict__ a2,
-                                                        const double *__restrict__ b2, double *partials, BiState *st,
-                                                        double *hist) {
+__device__ __forceinline__ void bi_tail(double s1, double s2, double *partials, BiState *st, double *hist) {
   __shared__ double sh[32];
   __shared__ bool last;
-  double s1 = 0.0, s2 = 0.0;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    s1 += a1[i] * b1[i];
-    if (a2) s2 += a2[i] * b2[i];
-  }
   s1 = block_sum(s1, sh);
   s2 = block_sum(s2, sh);
   if (threadIdx.x == 0) {
@@ -66,9 +59,8 @@ __global__ void __launch_bounds__(kBiThreads) k_bi_dots(size_t n, const double *
       st->done = 3;
     } else {
       st->inv0 = 1.0 / t1;
+      st->r_r2 = t1;  // r0* = r
     }
-  } else if (OP == kOpRR2) {
-    st->r_r2 = t1;
   } else if (OP == kOpAlpha) {
     st->alpha = st->r_r2 / t1;
   } else if (OP == kOpOmega) {
@@ -85,7 +77,21 @@ __global__ void __launch_bounds__(kBiThreads) k_bi_dots(size_t n, const double *
     else if (st->it + 1 >= st->max_iter)
       st->done = 2;
     st->beta = t2 * st->alpha / (st->r_r2 * st->omega);
+    st->r_r2 = t2;
   }
+}
+
+template <int OP>
+__global__ void __launch_bounds__(kBiThreads) k_bi_dots(size_t n, const double *__restrict__ a1,
+                                                        const double *__restrict__ b1, const double *__restrict__ a2,
+                                                        const double *__restrict__ b2, double *partials, BiState *st,
+                                                        double *hist) {
+  double s1 = 0.0, s2 = 0.0;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    s1 += a1[i] * b1[i];
+    if (a2) s2 += a2[i] * b2[i];
+  }
+  bi_tail<OP>(s1, s2, partials, st, hist);
 }
 
 // s = r - alpha A Mp
@@ -96,18 +102,26 @@ __global__ void k_bi_s(size_t n, const BiState *st, const double *__restrict__ r
     s[i] = r[i] - a * AMp[i];
 }
 
-// x += alpha Mp; x += omega Ms; r = s - omega A Ms (the reference's order)
-__global__ void k_bi_xr(size_t n, const BiState *st, double *__restrict__ x, double *__restrict__ r,
-                        const double *__restrict__ Mp, const double *__restrict__ Ms, const double *__restrict__ s,
-                        const double *__restrict__ AMs) {
+// x += alpha Mp; x += omega Ms; r = s - omega A Ms (the reference's order),
+// and (r, r), (r, r0*) of the new r while it is in a register.
+__global__ void __launch_bounds__(kBiThreads) k_bi_xr(size_t n, BiState *st, double *__restrict__ x,
+                                                      double *__restrict__ r, const double *__restrict__ Mp,
+                                                      const double *__restrict__ Ms, const double *__restrict__ s,
+                                                      const double *__restrict__ AMs, const double *__restrict__ r0,
+                                                      double *partials, double *hist) {
   const double a = st->alpha, w = st->omega;
+  double s1 = 0.0, s2 = 0.0;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     double xi = x[i];
     xi += a * Mp[i];
     xi += w * Ms[i];
     x[i] = xi;
-    r[i] = s[i] + (-w) * AMs[i];
+    const double ri = s[i] + (-w) * AMs[i];
+    r[i] = ri;
+    s1 += ri * ri;
+    s2 += ri * r0[i];
   }
+  bi_tail<kOpConvBeta>(s1, s2, partials, st, hist);
 }
 
 // p = beta p + r - beta omega A Mp
@@ -149,7 +163,9 @@ int dfm2g_solve_pbicgstab(dfm2g_bsr m, dfm2g_ilu p, double *r, double *x, double
     return DFM2G_OK;
   }
   auto &W = g_bi;
-  const unsigned grid = (unsigned)ctx().num_sms * 4;
+  // one CTA per four elements a thread, at most four per SM (fewer meet in the
+  // reductions of a short vector)
+  const unsigned grid = blocks_for(n, 4 * kBiThreads, (unsigned)ctx().num_sms * 4);
   DFM2G_TRY(W.st.ensure(1));
   DFM2G_TRY(W.partials.ensure(2 * (size_t)grid));
   DFM2G_TRY(W.hist.ensure((size_t)max_iter + 4));
@@ -177,7 +193,7 @@ int dfm2g_solve_pbicgstab(dfm2g_bsr m, dfm2g_ilu p, double *r, double *x, double
   // y (the reference's semantics): start them at zero, as its std::vectors do
   DFM2G_CUDA(cudaMemsetAsync(AMp, 0, sizeof(double) * n, stream()));
   DFM2G_CUDA(cudaMemsetAsync(AMs, 0, sizeof(double) * n, stream()));
-  const unsigned vb = blocks_for(n, kBiThreads, grid);
+  const unsigned vb = blocks_for(n, kBiThreads, (unsigned)ctx().num_sms * 4);
   k_bi_dots<kOpInit><<<grid, kBiThreads, 0, stream()>>>(n, rd, rd, nullptr, nullptr, W.partials.p, W.st.p, W.hist.p);
   note_launches(1);
   DFM2G_LAUNCH_CHECK();
@@ -192,8 +208,6 @@ int dfm2g_solve_pbicgstab(dfm2g_bsr m, dfm2g_ilu p, double *r, double *x, double
   while (!h.done) {
     DFM2G_TRY(ilu_sweep(p, DFM2G_F64, true, pv, tmp));
     DFM2G_TRY(ilu_sweep(p, DFM2G_F64, false, tmp, Mp));
-    k_bi_dots<kOpRR2><<<grid, kBiThreads, 0, stream()>>>(n, rd, r0, nullptr, nullptr, W.partials.p, W.st.p,
-                                                          W.hist.p);
     DFM2G_TRY(bsr_spmv(m, DFM2G_F64, AMp, 1.0, Mp, 0.0));
     k_bi_dots<kOpAlpha><<<grid, kBiThreads, 0, stream()>>>(n, AMp, r0, nullptr, nullptr, W.partials.p, W.st.p,
                                                             W.hist.p);
@@ -202,10 +216,9 @@ int dfm2g_solve_pbicgstab(dfm2g_bsr m, dfm2g_ilu p, double *r, double *x, double
     DFM2G_TRY(ilu_sweep(p, DFM2G_F64, false, tmp, Ms));
     DFM2G_TRY(bsr_spmv(m, DFM2G_F64, AMs, 1.0, Ms, 0.0));
     k_bi_dots<kOpOmega><<<grid, kBiThreads, 0, stream()>>>(n, AMs, AMs, s, AMs, W.partials.p, W.st.p, W.hist.p);
-    k_bi_xr<<<vb, kBiThreads, 0, stream()>>>(n, W.st.p, xd, rd, Mp, Ms, s, AMs);
-    k_bi_dots<kOpConvBeta><<<grid, kBiThreads, 0, stream()>>>(n, rd, rd, rd, r0, W.partials.p, W.st.p, W.hist.p);
+    k_bi_xr<<<grid, kBiThreads, 0, stream()>>>(n, W.st.p, xd, rd, Mp, Ms, s, AMs, r0, W.partials.p, W.hist.p);
     k_bi_p<<<vb, kBiThreads, 0, stream()>>>(n, W.st.p, pv, rd, AMp);
-    note_launches(8);
+    note_launches(5);
     DFM2G_LAUNCH_CHECK();
     DFM2G_CUDA(cudaMemcpyAsync(&h, W.st.p, sizeof(h), cudaMemcpyDeviceToHost, stream()));
     DFM2G_CUDA(cudaStreamSynchronize(stream()));
