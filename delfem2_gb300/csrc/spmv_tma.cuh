@@ -185,13 +185,15 @@ __device__ __forceinline__ void spmv_tma_rows_c(const unsigned *__restrict__ til
 #pragma unroll
             for (unsigned c = 0; c < B; ++c) (w & 1 ? o : e)[c] += v[w * BB + c] * h[w * B + c];
         }
-        // the diagonal block, the largest terms, last: fewer sums are rounded at its size
+        // the diagonal block, the largest terms, summed apart and added late: few
+        // sums are rounded at its size
+        T t = d[0] * __ldg(xi);
 #pragma unroll
-        for (unsigned c = 0; c < B; ++c) o[c] += d[c] * __ldg(xi + c);
+        for (unsigned c = 1; c < B; ++c) t += d[c] * __ldg(xi + c);
         T se = e[0], so = o[0];
 #pragma unroll
         for (unsigned c = 1; c < B; ++c) se += e[c], so += o[c];
-        epi(i, a, se + so);
+        epi(i, a, se + (so + t));
       } else {
         T acc0 = T(0), acc1 = T(0);
         for (; u + 1 < s1; u += 2) {
