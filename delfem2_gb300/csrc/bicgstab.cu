@@ -86,6 +86,7 @@ __global__ void __launch_bounds__(kBiThreads) k_bi_dots(size_t n, const double *
                                                         const double *__restrict__ b1, const double *__restrict__ a2,
                                                         const double *__restrict__ b2, double *partials, BiState *st,
                                                         double *hist) {
+  pdl_wait();
   double s1 = 0.0, s2 = 0.0;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     s1 += a1[i] * b1[i];
@@ -97,6 +98,7 @@ __global__ void __launch_bounds__(kBiThreads) k_bi_dots(size_t n, const double *
 // s = r - alpha A Mp
 __global__ void k_bi_s(size_t n, const BiState *st, const double *__restrict__ r, const double *__restrict__ AMp,
                        double *__restrict__ s) {
+  pdl_wait();
   const double a = st->alpha;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
     s[i] = r[i] - a * AMp[i];
@@ -109,6 +111,7 @@ __global__ void __launch_bounds__(kBiThreads) k_bi_xr(size_t n, BiState *st, dou
                                                       const double *__restrict__ Ms, const double *__restrict__ s,
                                                       const double *__restrict__ AMs, const double *__restrict__ r0,
                                                       double *partials, double *hist) {
+  pdl_wait();
   const double a = st->alpha, w = st->omega;
   double s1 = 0.0, s2 = 0.0;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
@@ -127,6 +130,7 @@ __global__ void __launch_bounds__(kBiThreads) k_bi_xr(size_t n, BiState *st, dou
 // p = beta p + r - beta omega A Mp
 __global__ void k_bi_p(size_t n, const BiState *st, double *__restrict__ p, const double *__restrict__ r,
                        const double *__restrict__ AMp) {
+  pdl_wait();
   if (st->done) return;
   const double b = st->beta, bw = -st->beta * st->omega;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
@@ -209,15 +213,23 @@ int dfm2g_solve_pbicgstab(dfm2g_bsr m, dfm2g_ilu p, double *r, double *x, double
     DFM2G_TRY(ilu_sweep(p, DFM2G_F64, true, pv, tmp));
     DFM2G_TRY(ilu_sweep(p, DFM2G_F64, false, tmp, Mp));
     DFM2G_TRY(bsr_spmv(m, DFM2G_F64, AMp, 1.0, Mp, 0.0));
-    k_bi_dots<kOpAlpha><<<grid, kBiThreads, 0, stream()>>>(n, AMp, r0, nullptr, nullptr, W.partials.p, W.st.p,
-                                                            W.hist.p);
-    k_bi_s<<<vb, kBiThreads, 0, stream()>>>(n, W.st.p, rd, AMp, s);
+    const double *none = nullptr;
+    auto dots = [&](auto *kernel, const double *a1, const double *b1, const double *a2, const double *b2) {
+      return launch_after(false, kernel, grid, (unsigned)kBiThreads, (size_t)0, n, a1, b1, a2, b2, W.partials.p,
+                          W.st.p, W.hist.p);
+    };
+    DFM2G_TRY(dots(k_bi_dots<kOpAlpha>, AMp, r0, none, none));
+    DFM2G_TRY(launch_after(false, k_bi_s, vb, (unsigned)kBiThreads, (size_t)0, n, (const BiState *)W.st.p,
+                           (const double *)rd, (const double *)AMp, s));
     DFM2G_TRY(ilu_sweep(p, DFM2G_F64, true, s, tmp));
     DFM2G_TRY(ilu_sweep(p, DFM2G_F64, false, tmp, Ms));
     DFM2G_TRY(bsr_spmv(m, DFM2G_F64, AMs, 1.0, Ms, 0.0));
-    k_bi_dots<kOpOmega><<<grid, kBiThreads, 0, stream()>>>(n, AMs, AMs, s, AMs, W.partials.p, W.st.p, W.hist.p);
-    k_bi_xr<<<grid, kBiThreads, 0, stream()>>>(n, W.st.p, xd, rd, Mp, Ms, s, AMs, r0, W.partials.p, W.hist.p);
-    k_bi_p<<<vb, kBiThreads, 0, stream()>>>(n, W.st.p, pv, rd, AMp);
+    DFM2G_TRY(dots(k_bi_dots<kOpOmega>, AMs, AMs, s, AMs));
+    DFM2G_TRY(launch_after(false, k_bi_xr, grid, (unsigned)kBiThreads, (size_t)0, n, W.st.p, xd, rd,
+                           (const double *)Mp, (const double *)Ms, (const double *)s, (const double *)AMs,
+                           (const double *)r0, W.partials.p, W.hist.p));
+    DFM2G_TRY(launch_after(false, k_bi_p, vb, (unsigned)kBiThreads, (size_t)0, n, (const BiState *)W.st.p, pv,
+                           (const double *)rd, (const double *)AMp));
     note_launches(5);
     DFM2G_LAUNCH_CHECK();
     DFM2G_CUDA(cudaMemcpyAsync(&h, W.st.p, sizeof(h), cudaMemcpyDeviceToHost, stream()));

