@@ -66,6 +66,7 @@ __global__ void __launch_bounds__(kThreads) k_spmv_pAp(IterState *st, unsigned n
                                                        const T *__restrict__ vdia, const T *__restrict__ p,
                                                        T *__restrict__ Ap, double *partials) {
   __shared__ double sh[32];
+  pdl_wait();
   if (st->done) return;
   const unsigned lane = threadIdx.x & 31;
   double dot = 0.0;
@@ -82,6 +83,30 @@ __global__ void __launch_bounds__(kThreads) k_spmv_pAp(IterState *st, unsigned n
   }
 }
 
+// The same in the component layout of spmv_tma_rows_c (the default when the
+// pattern has tiles).
+template <typename T, int B>
+__global__ void __launch_bounds__(TileCfgC<T, B>::kThreads, 1)
+    k_spmv_pAp_tma_c(IterState *st, const unsigned *__restrict__ tiles, unsigned ntiles,
+                     const unsigned *__restrict__ row_start, const unsigned *__restrict__ col,
+                     const T *__restrict__ vcrs, const T *__restrict__ vdia, const T *__restrict__ p,
+                     T *__restrict__ Ap, double *partials, int *err, unsigned long long timeout_ns) {
+  extern __shared__ __align__(128) unsigned char tma_smem[];
+  __shared__ double sh[32];
+  pdl_wait();
+  if (st->done) return;
+  double dot = 0.0;
+  spmv_tma_rows_c<T, B>(tiles, ntiles, row_start, col, vcrs, vdia, p, err, timeout_ns, tma_smem,
+                        [&](unsigned row, unsigned a, T v) {
+                          Ap[(size_t)row * B + a] = v;
+                          dot += (double)(v * p[(size_t)row * B + a]);
+                        });
+  double total;
+  if (grid_sum_last(dot, partials, &st->ticket[0], sh, &total)) {
+    st->alpha = st->rPr / total;
+  }
+}
+
 // The same for 1x1 and 2x2 blocks (nd.cuh).
 template <typename T, int B>
 __global__ void __launch_bounds__(kThreads) k_spmv_pAp_nd(IterState *st, unsigned nblk,
@@ -90,6 +115,7 @@ __global__ void __launch_bounds__(kThreads) k_spmv_pAp_nd(IterState *st, unsigne
                                                           const T *__restrict__ vdia, const T *__restrict__ p,
                                                           T *__restrict__ Ap, double *partials) {
   __shared__ double sh[32];
+  pdl_wait();
   if (st->done) return;
   double dot = 0.0;
   nd_spmv_rows<T, B>(nblk, row_start, col, vcrs, vdia, p, [&](unsigned row, const T s[B], unsigned sub) {
@@ -105,24 +131,43 @@ __global__ void __launch_bounds__(kThreads) k_spmv_pAp_nd(IterState *st, unsigne
   }
 }
 
-template <typename T>
-static int launch_spmv_pAp(dfm2g_bsr_s *m, IterState *st, const T *vcrs, const T *vdia, const T *pv, T *Ap,
-                           double *partials, unsigned spmv_blocks) {
-  if (m->ndim == 1) {
-    k_spmv_pAp_nd<T, 1><<<spmv_blocks, kThreads, 0, stream()>>>(st, m->nblk, m->row_start.p, m->col.p, vcrs, vdia, pv,
-                                                               Ap, partials);
-  } else if (m->ndim == 2) {
-    k_spmv_pAp_nd<T, 2><<<spmv_blocks, kThreads, 0, stream()>>>(st, m->nblk, m->row_start.p, m->col.p, vcrs, vdia, pv,
-                                                               Ap, partials);
-  } else {
-    k_spmv_pAp<T><<<spmv_blocks, kThreads, 0, stream()>>>(st, m->nblk, m->row_start.p, m->col.p, vcrs, vdia, pv, Ap,
-                                                         partials);
+// Lets a TMA-staged kernel use TileCfgC's shared memory (once per device).
+template <typename K>
+static int allow_tma_smem(K kernel, size_t smem, int &attr_device) {
+  if (attr_device != ctx().device) {
+    DFM2G_CUDA(cudaFuncSetAttribute((const void *)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    attr_device = ctx().device;
   }
   return DFM2G_OK;
 }
 
+template <typename T, int B>
+static int launch_spmv_pAp(dfm2g_bsr_s *m, IterState *st, const T *vcrs, const T *vdia, const T *pv, T *Ap,
+                           double *partials) {
+  const unsigned *rs = m->row_start.p, *col = m->col.p;
+  if (m->tiles_ok) {
+    using C = TileCfgC<T, B>;
+    static int attr_device = -1;
+    DFM2G_TRY(allow_tma_smem(k_spmv_pAp_tma_c<T, B>, C::kSmem, attr_device));
+    const unsigned nt = sizeof(T) == 8 ? m->ntiles64 : m->ntiles32;
+    const unsigned *tiles = sizeof(T) == 8 ? m->tiles64.p : m->tiles32.p;
+    return launch_after(false, k_spmv_pAp_tma_c<T, B>, std::min(nt, (unsigned)ctx().num_sms), C::kThreads, C::kSmem,
+                        st, tiles, nt, rs, col, vcrs, vdia, pv, Ap, partials, m->err.p, kWaitTimeoutNs);
+  }
+  const unsigned blocks = blocks_for((size_t)m->nblk * 32, kThreads, (unsigned)ctx().num_sms * 8);
+  auto *kernel = [] {
+    if constexpr (B == 3)
+      return k_spmv_pAp<T>;
+    else
+      return k_spmv_pAp_nd<T, B>;
+  }();
+  return launch_after(false, kernel, blocks, (unsigned)kThreads, (size_t)0, st, m->nblk, rs, col, vcrs, vdia, pv, Ap,
+                      partials);
+}
+
 // Reliable update, part 1: x64 += x32, x32 = 0 (only when a refresh is due).
 __global__ void k_flush_x(const IterState *st, size_t n, double *__restrict__ x64, float *__restrict__ x32) {
+  pdl_wait();
   if (st->done || !st->update) return;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     x64[i] += (double)x32[i] / st->scale;
@@ -174,6 +219,7 @@ __global__ void __launch_bounds__(kThreads) k_true_residual(IterState *st, unsig
                                                             const double *__restrict__ b, float *__restrict__ r32,
                                                             double *partials) {
   __shared__ double sh[32];
+  pdl_wait();
   if (st->done || !st->update) return;
   __shared__ double sh2[32];
   const unsigned lane = threadIdx.x & 31;
@@ -197,32 +243,21 @@ __global__ void __launch_bounds__(kThreads) k_true_residual(IterState *st, unsig
   refresh_tail(st, rr, dd, partials, sh, sh2);
 }
 
-// Both parts of the reliable update in one cooperative launch (k_flush_x,
-// k_true_residual) for patterns with SpMV tiles, only when a refresh is
-// due: x64 += x32 / scale and x32 = 0 over the CTA's grid-stride share, a
-// meeting of all CTAs, then r64 = b - K64 x64 through the TMA-staged
+// Part 2 for patterns with SpMV tiles, through the TMA-staged
 // component-layout product (spmv_tma_rows_c<double, B>).
 template <int B>
 __global__ void __launch_bounds__(TileCfgC<double, B>::kThreads, 1)
     k_refresh_tma(IterState *st, const unsigned *__restrict__ tiles, unsigned ntiles,
                   const unsigned *__restrict__ row_start, const unsigned *__restrict__ col,
-                  const double *__restrict__ vcrs, const double *__restrict__ vdia, double *x64, float *x32,
-                  const double *__restrict__ b, float *__restrict__ r32, size_t n, double *partials, unsigned *bar,
-                  int *err, unsigned long long timeout_ns) {
+                  const double *__restrict__ vcrs, const double *__restrict__ vdia, const double *__restrict__ x64,
+                  const double *__restrict__ b, float *__restrict__ r32, double *partials, int *err,
+                  unsigned long long timeout_ns) {
   extern __shared__ __align__(128) unsigned char tma_smem[];
   __shared__ double sh[32];
   __shared__ double sh2[32];
   pdl_wait();
   if (st->done || !st->update) return;
-  const double sc = st->scale_next, old = st->scale, inv_old = 1.0 / st->scale;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    x64[i] += (double)x32[i] / old;
-    x32[i] = 0.f;
-  }
-  if (!grid_barrier(bar, err, timeout_ns)) {
-    if (threadIdx.x == 0) st->done = 4;
-    return;
-  }
+  const double sc = st->scale_next, inv_old = 1.0 / st->scale;
   double rr = 0.0, dd = 0.0;
   spmv_tma_rows_c<double, B>(tiles, ntiles, row_start, col, vcrs, vdia, x64, err, timeout_ns, tma_smem,
                              [&](unsigned row, unsigned a, double v) {
@@ -460,102 +495,56 @@ __global__ void __launch_bounds__(kThreads) k_update(IterState *st, size_t n, T 
                                                      const T *p, const T *Ap, double *partials, double *hist,
                                                      T *fill_a, T *fill_b) {
   __shared__ double sh[32];
+  pdl_wait();
   if (st->done) return;
   const double rr = update_pass<T>(n, r, x, p, Ap, st->alpha, fill_a, fill_b);
   double total;
   if (grid_sum_last(rr, partials, &st->ticket[1], sh, &total)) update_tail(st, total, hist);
 }
 
-// The SpMV with p.Ap (component layout, spmv_tma_rows_c) and the update
-// (k_update) in one cooperative launch: the CTAs meet once to add the p.Ap
-// partials (each CTA adds them in the same order, so every CTA has the same
-// alpha), then update their grid-stride share of r and x. The |r|^2 partials
-// go to partials[gridDim.x, 2 gridDim.x).
-template <typename T, int B>
-__global__ void __launch_bounds__(TileCfgC<T, B>::kThreads, 1)
-    k_spmv_update_tma_c(IterState *st, const unsigned *__restrict__ tiles, unsigned ntiles,
-                        const unsigned *__restrict__ row_start, const unsigned *__restrict__ col,
-                        const T *__restrict__ vcrs, const T *__restrict__ vdia, const T *p, T *Ap, T *r, T *x,
-                        size_t n, double *partials, double *hist, T *fill_a, T *fill_b, unsigned *bar, int *err,
-                        unsigned long long timeout_ns) {
-  extern __shared__ __align__(128) unsigned char tma_smem[];
-  __shared__ double sh[32];
-  pdl_wait();
-  if (st->done) return;
-  double dot = 0.0;
-  spmv_tma_rows_c<T, B>(tiles, ntiles, row_start, col, vcrs, vdia, p, err, timeout_ns, tma_smem,
-                        [&](unsigned row, unsigned a, T v) {
-                          Ap[(size_t)row * B + a] = v;
-                          dot += (double)(v * p[(size_t)row * B + a]);
-                        });
-  dot = block_sum(dot, sh);
-  if (threadIdx.x == 0) partials[blockIdx.x] = dot;
-  if (!grid_barrier(bar, err, timeout_ns)) {
-    if (threadIdx.x == 0) st->done = 4;
-    return;
-  }
-  const double alpha = st->rPr / sum_partials_all(partials, gridDim.x, sh);
-  if (blockIdx.x == 0 && threadIdx.x == 0) st->alpha = alpha;
-  const double rr = update_pass<T>(n, r, x, p, Ap, alpha, fill_a, fill_b);
-  double total;
-  if (grid_sum_last(rr, partials + gridDim.x, &st->ticket[1], sh, &total)) update_tail(st, total, hist);
+// rPr1 = (r, Pr) -> beta = rPr1 / rPr and the state (one thread of the grid).
+__device__ __forceinline__ double take_rPr(IterState *st, double total) {
+  // after a rescale of the FP32 vectors, the old p and (r,Pr) are in the old
+  // scale: p_new = z + rPr1/(rPr*ratio^2) * (ratio*p) = z + rPr1/(rPr*ratio) * p
+  const double beta = st->restart_p ? 0.0 : total / (st->rPr * st->ratio);
+  st->beta = beta;
+  st->rPr = total;
+  st->ratio = 1.0;
+  st->restart_p = 0;
+  return beta;
 }
 
-// rPr1 = (r, Pr); beta = rPr1/rPr.
 template <typename T>
 __global__ void __launch_bounds__(kThreads) k_dot_beta(IterState *st, size_t n, const T *__restrict__ r,
                                                        const T *__restrict__ z, double *partials) {
   __shared__ double sh[32];
+  pdl_wait();
   if (st->done) return;
   const double s = dot_pass<T>(n, r, z);
   double total;
-  if (grid_sum_last(s, partials, &st->ticket[2], sh, &total)) {
-    // after a rescale of the FP32 vectors, the old p and (r,Pr) are in the old
-    // scale: p_new = z + rPr1/(rPr*ratio^2) * (ratio*p) = z + rPr1/(rPr*ratio) * p
-    st->beta = st->restart_p ? 0.0 : total / (st->rPr * st->ratio);
-    st->rPr = total;
-    st->ratio = 1.0;
-    st->restart_p = 0;
-  }
+  if (grid_sum_last(s, partials, &st->ticket[2], sh, &total)) take_rPr(st, total);
 }
 
 // p = z + beta p.
 template <typename T>
 __global__ void k_p_update(const IterState *st, size_t n, T *p, const T *__restrict__ z) {
+  pdl_wait();
   if (st->done) return;
   p_pass<T>(n, p, z, (T)st->beta);
 }
 
-// (r, z), beta and p = z + beta p in one cooperative launch (k_dot_beta and
-// k_p_update): the CTAs meet once to add the dot's partials, each in the same
-// order, so every CTA computes the same beta. The state the dot updates
-// (rPr, ratio, restart_p) is read before the meeting and written after it.
+// k_dot_beta and k_p_update in one launch of one CTA, for short vectors.
 template <typename T>
 __global__ void __launch_bounds__(kThreads) k_dot_pupdate(IterState *st, size_t n, const T *__restrict__ r,
-                                                          const T *__restrict__ z, T *p, double *partials,
-                                                          unsigned *bar, int *err, unsigned long long timeout_ns) {
+                                                          const T *__restrict__ z, T *p) {
   __shared__ double sh[32];
+  __shared__ T beta_s;
   pdl_wait();
   if (st->done) return;
-  const double rPr = st->rPr, ratio = st->ratio;
-  const int restart = st->restart_p;
   const double s = block_sum(dot_pass<T>(n, r, z), sh);
-  if (threadIdx.x == 0) partials[blockIdx.x] = s;
-  if (!grid_barrier(bar, err, timeout_ns)) {
-    if (threadIdx.x == 0) st->done = 4;
-    return;
-  }
-  const double total = sum_partials_all(partials, gridDim.x, sh);
-  // after a rescale of the FP32 vectors, the old p and (r,Pr) are in the old
-  // scale: p_new = z + rPr1/(rPr*ratio^2) * (ratio*p) = z + rPr1/(rPr*ratio) * p
-  const double beta = restart ? 0.0 : total / (rPr * ratio);
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    st->beta = beta;
-    st->rPr = total;
-    st->ratio = 1.0;
-    st->restart_p = 0;
-  }
-  p_pass<T>(n, p, z, (T)beta);
+  if (threadIdx.x == 0) beta_s = (T)take_rPr(st, s);
+  __syncthreads();
+  p_pass<T>(n, p, z, beta_s);
 }
 
 // generic deterministic dot into a device scalar
@@ -618,7 +607,6 @@ struct Workspace {
   DevBuf<IterState> st;
   DevBuf<double> partials, scal, hist;
   DevBuf<unsigned> tickets;
-  DevBuf<unsigned> bar;  // grid_barrier words of the cooperative solver kernels
   DevBuf<double> v64[6];
   DevBuf<float> v32[6];
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -639,8 +627,6 @@ static int ws_prepare(size_t n, unsigned hist_cap, bool need32) {
   DFM2G_TRY(g_ws.partials.ensure((size_t)ctx().num_sms * 64));
   DFM2G_TRY(g_ws.scal.ensure(8));
   DFM2G_TRY(g_ws.tickets.ensure(4));
-  DFM2G_TRY(g_ws.bar.ensure(2));
-  DFM2G_CUDA(cudaMemsetAsync(g_ws.bar.p, 0, 2 * sizeof(unsigned), stream()));
   DFM2G_TRY(g_ws.hist.ensure(hist_cap + 4));
   for (auto &b : g_ws.v64) DFM2G_TRY(b.ensure(n + 1));
   if (need32)
@@ -672,37 +658,6 @@ static int dot_host(size_t n, const void *a, const void *b, int prec, double *ou
   return DFM2G_OK;
 }
 
-// Lets a TMA-staged kernel use TileCfgC's shared memory (once per device).
-template <typename K>
-static int allow_tma_smem(K kernel, size_t smem, int &attr_device) {
-  if (attr_device != ctx().device) {
-    DFM2G_CUDA(cudaFuncSetAttribute((const void *)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attr_device = ctx().device;
-  }
-  return DFM2G_OK;
-}
-
-// Shared memory of the tiled row products (their CTAs have as many threads for every block size).
-template <typename T>
-static size_t tile_smem(unsigned ndim) {
-  static_assert(TileCfgC<T, 1>::kThreads == TileCfgC<T, 3>::kThreads, "one CTA size");
-  static_assert(TileCfgC<T, 2>::kThreads == TileCfgC<T, 3>::kThreads, "one CTA size");
-  return ndim == 1 ? TileCfgC<T, 1>::kSmem : ndim == 2 ? TileCfgC<T, 2>::kSmem : TileCfgC<T, 3>::kSmem;
-}
-
-// CTAs of k_dot_pupdate<T>: reduce_blocks(n), or as many as are resident at once.
-template <typename T>
-static int dot_pupdate_blocks(size_t n, unsigned *grid) {
-  static int per_sm_dev = -1, per_sm = 0;
-  if (per_sm_dev != ctx().device) {
-    DFM2G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_dot_pupdate<T>, kThreads, 0));
-    per_sm_dev = ctx().device;
-  }
-  if (per_sm <= 0) return fail(DFM2G_ERR_CUDA, "k_dot_pupdate cannot be resident");
-  *grid = std::min(reduce_blocks(n), (unsigned)per_sm * (unsigned)ctx().num_sms);
-  return DFM2G_OK;
-}
-
 // Core preconditioned CG on device vectors of type T.
 //  r: rhs in, final residual out; x: solution out (starts at 0);
 //  w0..w3: scratch vectors (Pr/Ap share w0 as in the reference, p = w1,
@@ -716,6 +671,26 @@ struct Refine {
   const double *b64 = nullptr;
   double delta = 0, bnorm = 0;
 };
+
+// Both parts of the reliable update (their kernels only work when one is due).
+template <int B>
+static int launch_refresh(dfm2g_bsr_s *m, IterState *st, size_t n, float *x32, float *r32, const Refine &rf) {
+  const unsigned *rs = m->row_start.p, *col = m->col.p;
+  const double *vcrs = m->vcrs.p, *vdia = m->vdia.p, *x64 = rf.x64;
+  DFM2G_TRY(launch_after(false, k_flush_x, reduce_blocks(n), (unsigned)kThreads, (size_t)0, (const IterState *)st, n,
+                         rf.x64, x32));
+  if (m->tiles_ok) {
+    using C = TileCfgC<double, B>;
+    static int attr_device = -1;
+    DFM2G_TRY(allow_tma_smem(k_refresh_tma<B>, C::kSmem, attr_device));
+    return launch_after(false, k_refresh_tma<B>, std::min(m->ntiles64, (unsigned)ctx().num_sms), C::kThreads,
+                        C::kSmem, st, (const unsigned *)m->tiles64.p, m->ntiles64, rs, col, vcrs, vdia, x64, rf.b64,
+                        r32, g_ws.partials.p, m->err.p, kWaitTimeoutNs);
+  }
+  const unsigned blocks = blocks_for((size_t)m->nblk * 32, kThreads, (unsigned)ctx().num_sms * 8);
+  return launch_after(false, k_true_residual<B>, blocks, (unsigned)kThreads, (size_t)0, st, m->nblk, rs, col, vcrs,
+                      vdia, x64, rf.b64, r32, g_ws.partials.p);
+}
 
 template <typename T>
 static int pcg_core(dfm2g_bsr_s *m, dfm2g_ilu_s *p, T *r, T *x, T *w0, T *w1, T *w2, double tol,
@@ -756,75 +731,33 @@ static int pcg_core(dfm2g_bsr_s *m, dfm2g_ilu_s *p, T *r, T *x, T *w0, T *w1, T 
   k_init_state<<<1, 1, 0, stream()>>>(st, g_ws.scal.p, g_ws.hist.p, mode);
   note_launches(1);
   DFM2G_LAUNCH_CHECK();
-  const unsigned spmv_blocks = blocks_for((size_t)nblk * 32, kThreads, (unsigned)ctx().num_sms * 8);
   const unsigned vec_blocks = reduce_blocks(n);
   const int chunk = 16;
-  // Patterns with SpMV tiles: two cooperative launches besides the sweeps per
-  // iteration (k_spmv_update_tma_c, k_dot_pupdate) and the refresh
-  // (k_refresh_tma) only does work when one is due; otherwise five
-  // (k_spmv_pAp*, k_update, k_flush_x + k_true_residual*, k_dot_beta, k_p_update).
-  const bool fused = m->tiles_ok;
-  auto *k_sp = m->ndim == 1   ? k_spmv_update_tma_c<T, 1>
-               : m->ndim == 2 ? k_spmv_update_tma_c<T, 2>
-                              : k_spmv_update_tma_c<T, 3>;
-  auto *k_re = m->ndim == 1 ? k_refresh_tma<1> : m->ndim == 2 ? k_refresh_tma<2> : k_refresh_tma<3>;
-  const size_t smem_T = tile_smem<T>(m->ndim), smem_64 = tile_smem<double>(m->ndim);
-  constexpr unsigned threads_T = TileCfgC<T, 3>::kThreads, threads_64 = TileCfgC<double, 3>::kThreads;
-  const unsigned nt_T = sizeof(T) == 8 ? m->ntiles64 : m->ntiles32;
-  const unsigned *tiles_T = sizeof(T) == 8 ? m->tiles64.p : m->tiles32.p;
-  unsigned dp_grid = 0;
-  if (fused) {
-    static int attr_a[3] = {-1, -1, -1}, attr_r[3] = {-1, -1, -1};
-    DFM2G_TRY(allow_tma_smem(k_sp, smem_T, attr_a[m->ndim - 1]));
-    DFM2G_TRY(allow_tma_smem(k_re, smem_64, attr_r[m->ndim - 1]));
-    DFM2G_TRY(dot_pupdate_blocks<T>(n, &dp_grid));
-  }
+  const unsigned th = kThreads;
+  const size_t none = 0;
   for (;;) {
     for (int k = 0; k < chunk; ++k) {
       T *Ap = Pr;
       // the sweeps' outputs get their pending marker in the update (Ap is Pr: read first, element by element)
       const bool fill = mode != 1 && p->sweep_mode != DFM2G_SWEEP_LEVELS;
       T *fa = fill ? mid : nullptr, *fb = fill ? Pr : nullptr;
-      if (fused) {
+      {
         ProfScope ps(DFM2G_PROF_SPMV, 1);
-        DFM2G_TRY(launch_after(true, k_sp, std::min(nt_T, (unsigned)ctx().num_sms), threads_T, smem_T, st, tiles_T,
-                               nt_T, (const unsigned *)m->row_start.p, (const unsigned *)m->col.p, vcrs, vdia,
-                               (const T *)pv, Ap, r, x, n, g_ws.partials.p, g_ws.hist.p, fa, fb, g_ws.bar.p,
-                               m->err.p, kWaitTimeoutNs));
-      } else {
-        {
-          ProfScope ps(DFM2G_PROF_SPMV, 1);
-          DFM2G_TRY(launch_spmv_pAp<T>(m, st, vcrs, vdia, pv, Ap, g_ws.partials.p, spmv_blocks));
-        }
-        {
-          ProfScope ps(DFM2G_PROF_UPDATE, 1);
-          k_update<T><<<vec_blocks, kThreads, 0, stream()>>>(st, n, r, x, pv, Ap, g_ws.partials.p, g_ws.hist.p, fa,
-                                                             fb);
-        }
+        DFM2G_TRY((m->ndim == 1   ? launch_spmv_pAp<T, 1>(m, st, vcrs, vdia, pv, Ap, g_ws.partials.p)
+                   : m->ndim == 2 ? launch_spmv_pAp<T, 2>(m, st, vcrs, vdia, pv, Ap, g_ws.partials.p)
+                                  : launch_spmv_pAp<T, 3>(m, st, vcrs, vdia, pv, Ap, g_ws.partials.p)));
+      }
+      {
+        ProfScope ps(DFM2G_PROF_UPDATE, 1);
+        DFM2G_TRY(launch_after(false, k_update<T>, vec_blocks, th, none, st, n, r, x, (const T *)pv, (const T *)Ap,
+                               g_ws.partials.p, g_ws.hist.p, fa, fb));
       }
       if constexpr (sizeof(T) == 4) {
-        if (mode == 2 && fused) {
-          ProfScope ps(DFM2G_PROF_OUTER, 1);
-          DFM2G_TRY(launch_after(true, k_re, std::min(m->ntiles64, (unsigned)ctx().num_sms), threads_64, smem_64, st,
-                                (const unsigned *)m->tiles64.p, m->ntiles64, (const unsigned *)m->row_start.p,
-                                (const unsigned *)m->col.p, (const double *)m->vcrs.p, (const double *)m->vdia.p,
-                                rf.x64, (float *)x, rf.b64, (float *)r, n, g_ws.partials.p, g_ws.bar.p, m->err.p,
-                                kWaitTimeoutNs));
-        } else if (mode == 2) {
+        if (mode == 2) {
           ProfScope ps(DFM2G_PROF_OUTER, 2);
-          k_flush_x<<<vec_blocks, kThreads, 0, stream()>>>(st, n, rf.x64, (float *)x);
-          if (m->ndim == 3)
-            k_true_residual<3><<<spmv_blocks, kThreads, 0, stream()>>>(st, nblk, m->row_start.p, m->col.p,
-                                                                       m->vcrs.p, m->vdia.p, rf.x64, rf.b64,
-                                                                       (float *)r, g_ws.partials.p);
-          else if (m->ndim == 2)
-            k_true_residual<2><<<spmv_blocks, kThreads, 0, stream()>>>(st, nblk, m->row_start.p, m->col.p,
-                                                                       m->vcrs.p, m->vdia.p, rf.x64, rf.b64,
-                                                                       (float *)r, g_ws.partials.p);
-          else
-            k_true_residual<1><<<spmv_blocks, kThreads, 0, stream()>>>(st, nblk, m->row_start.p, m->col.p,
-                                                                       m->vcrs.p, m->vdia.p, rf.x64, rf.b64,
-                                                                       (float *)r, g_ws.partials.p);
+          DFM2G_TRY(m->ndim == 1   ? launch_refresh<1>(m, st, n, x, r, rf)
+                    : m->ndim == 2 ? launch_refresh<2>(m, st, n, x, r, rf)
+                                   : launch_refresh<3>(m, st, n, x, r, rf));
         }
       }
       if (mode != 1) {
@@ -836,23 +769,25 @@ static int pcg_core(dfm2g_bsr_s *m, dfm2g_ilu_s *p, T *r, T *x, T *w0, T *w1, T 
           ProfScope ps(DFM2G_PROF_BWD, 0);
           DFM2G_TRY(ilu_sweep_guarded(p, prec, false, mid, Pr, &st->done));
         }
-        if (fused) {
+        if (vec_blocks == 1) {
           ProfScope ps(DFM2G_PROF_DOT, 1);
-          DFM2G_TRY(launch_after(dp_grid > 1, k_dot_pupdate<T>, dp_grid, (unsigned)kThreads, (size_t)0, st, n, (const T *)r,
-                                (const T *)Pr, pv, g_ws.partials.p, g_ws.bar.p, m->err.p, kWaitTimeoutNs));
+          DFM2G_TRY(launch_after(false, k_dot_pupdate<T>, 1u, th, none, st, n, (const T *)r, (const T *)Pr, pv));
         } else {
           {
             ProfScope ps(DFM2G_PROF_DOT, 1);
-            k_dot_beta<T><<<vec_blocks, kThreads, 0, stream()>>>(st, n, r, Pr, g_ws.partials.p);
+            DFM2G_TRY(launch_after(false, k_dot_beta<T>, vec_blocks, th, none, st, n, (const T *)r, (const T *)Pr,
+                                   g_ws.partials.p));
           }
           {
             ProfScope ps(DFM2G_PROF_PUPDATE, 1);
-            k_p_update<T><<<vec_blocks, kThreads, 0, stream()>>>(st, n, pv, Pr);
+            DFM2G_TRY(launch_after(false, k_p_update<T>, vec_blocks, th, none, (const IterState *)st, n, pv,
+                                   (const T *)Pr));
           }
         }
       } else {
         ProfScope ps(DFM2G_PROF_PUPDATE, 1);
-        k_p_update<T><<<vec_blocks, kThreads, 0, stream()>>>(st, n, pv, r);
+        DFM2G_TRY(launch_after(false, k_p_update<T>, vec_blocks, th, none, (const IterState *)st, n, pv,
+                               (const T *)r));
       }
     }
     DFM2G_LAUNCH_CHECK();
