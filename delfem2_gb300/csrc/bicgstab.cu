@@ -215,20 +215,20 @@ int dfm2g_solve_pbicgstab(dfm2g_bsr m, dfm2g_ilu p, double *r, double *x, double
     DFM2G_TRY(bsr_spmv(m, DFM2G_F64, AMp, 1.0, Mp, 0.0));
     const double *none = nullptr;
     auto dots = [&](auto *kernel, const double *a1, const double *b1, const double *a2, const double *b2) {
-      return launch_after(false, kernel, grid, (unsigned)kBiThreads, (size_t)0, n, a1, b1, a2, b2, W.partials.p,
+      return launch_after(kernel, grid, (unsigned)kBiThreads, (size_t)0, n, a1, b1, a2, b2, W.partials.p,
                           W.st.p, W.hist.p);
     };
     DFM2G_TRY(dots(k_bi_dots<kOpAlpha>, AMp, r0, none, none));
-    DFM2G_TRY(launch_after(false, k_bi_s, vb, (unsigned)kBiThreads, (size_t)0, n, (const BiState *)W.st.p,
+    DFM2G_TRY(launch_after(k_bi_s, vb, (unsigned)kBiThreads, (size_t)0, n, (const BiState *)W.st.p,
                            (const double *)rd, (const double *)AMp, s));
     DFM2G_TRY(ilu_sweep(p, DFM2G_F64, true, s, tmp));
     DFM2G_TRY(ilu_sweep(p, DFM2G_F64, false, tmp, Ms));
     DFM2G_TRY(bsr_spmv(m, DFM2G_F64, AMs, 1.0, Ms, 0.0));
     DFM2G_TRY(dots(k_bi_dots<kOpOmega>, AMs, AMs, s, AMs));
-    DFM2G_TRY(launch_after(false, k_bi_xr, grid, (unsigned)kBiThreads, (size_t)0, n, W.st.p, xd, rd,
+    DFM2G_TRY(launch_after(k_bi_xr, grid, (unsigned)kBiThreads, (size_t)0, n, W.st.p, xd, rd,
                            (const double *)Mp, (const double *)Ms, (const double *)s, (const double *)AMs,
                            (const double *)r0, W.partials.p, W.hist.p));
-    DFM2G_TRY(launch_after(false, k_bi_p, vb, (unsigned)kBiThreads, (size_t)0, n, (const BiState *)W.st.p, pv,
+    DFM2G_TRY(launch_after(k_bi_p, vb, (unsigned)kBiThreads, (size_t)0, n, (const BiState *)W.st.p, pv,
                            (const double *)rd, (const double *)AMp));
     note_launches(5);
     DFM2G_LAUNCH_CHECK();

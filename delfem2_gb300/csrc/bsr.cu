@@ -150,7 +150,7 @@ static int spmv_launch(dfm2g_bsr_s *m, const T *vcrs, const T *vdia, T *y, T alp
     const unsigned nt = sizeof(T) == 8 ? m->ntiles64 : m->ntiles32;
     const unsigned *tiles = sizeof(T) == 8 ? m->tiles64.p : m->tiles32.p;
     const unsigned grid = std::min(nt, (unsigned)ctx().num_sms);
-    return launch_after(false, k_bsr_spmv_tma_c<T, B>, grid, C::kThreads, C::kSmem, tiles, nt,
+    return launch_after(k_bsr_spmv_tma_c<T, B>, grid, C::kThreads, C::kSmem, tiles, nt,
                         (const unsigned *)m->row_start.p, (const unsigned *)m->col.p, vcrs, vdia, y, alpha, x, beta,
                         m->err.p, kWaitTimeoutNs);
   }

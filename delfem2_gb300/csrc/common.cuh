@@ -126,30 +126,27 @@ struct VecArg {
 // (programmatic stream serialisation). A kernel launched so starts with
 // pdl_wait(), which returns when that kernel has ended and its writes are
 // visible, so the order is the stream's as ever; it saves the set-up between two
-// kernels (1.4 us from one to the next instead of 4.1). Cooperative where the
-// CTAs meet.
-inline int launch_after(const void *kernel, unsigned grid, unsigned threads, size_t smem, void **args,
-                        bool cooperative) {
-  cudaLaunchAttribute at[2] = {};
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  at[1].id = cudaLaunchAttributeCooperative;
-  at[1].val.cooperative = 1;
+// kernels (1.4 us from one to the next instead of 4.1; a cooperative kernel, and
+// the one after it, gain nothing).
+inline int launch_after(const void *kernel, unsigned grid, unsigned threads, size_t smem, void **args) {
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t c = {};
   c.gridDim = dim3(grid);
   c.blockDim = dim3(threads);
   c.dynamicSmemBytes = smem;
   c.stream = stream();
-  c.attrs = at;
-  c.numAttrs = cooperative ? 2 : 1;
+  c.attrs = &at;
+  c.numAttrs = 1;
   DFM2G_CUDA(cudaLaunchKernelExC(&c, kernel, args));
   return DFM2G_OK;
 }
 // The same with typed arguments (each must have the kernel parameter's exact type).
 template <typename... A>
-int launch_after(bool cooperative, void (*kernel)(A...), unsigned grid, unsigned threads, size_t smem, A... args) {
+int launch_after(void (*kernel)(A...), unsigned grid, unsigned threads, size_t smem, A... args) {
   void *argv[] = {(void *)&args...};
-  return launch_after((const void *)kernel, grid, threads, smem, argv, cooperative);
+  return launch_after((const void *)kernel, grid, threads, smem, argv);
 }
 
 inline unsigned blocks_for(size_t work, unsigned per_block, unsigned cap = 0xFFFFFFFFu) {
@@ -313,16 +310,6 @@ __device__ __forceinline__ bool grid_barrier(unsigned *bar, int *err, unsigned l
   }
   __syncthreads();
   return ok_s != 0;
-}
-
-// Sum of partials[0, nparts) in a fixed order, the same in every CTA that
-// calls it (all threads of the CTA receive it).
-__device__ __forceinline__ double sum_partials_all(const double *partials, unsigned nparts, double *sh) {
-  __shared__ double total_s;
-  const double s = sum_partials(partials, nparts, sh);
-  if (threadIdx.x == 0) total_s = s;
-  __syncthreads();
-  return total_s;
 }
 
 }  // namespace dfm2g

@@ -1019,6 +1019,25 @@ static int coop_blocks(const void *kernel, int *cache) {
   return DFM2G_OK;
 }
 
+// Every word of `out` (a multiple of four bytes, on four) to the sweeps' pending
+// marker: a kernel, as a kernel can be set up behind it and a memset's successor
+// not.
+__global__ void __launch_bounds__(256) k_fill_pending(unsigned *__restrict__ out, size_t words) {
+  pdl_wait();
+  const size_t S = (size_t)gridDim.x * blockDim.x, t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  const size_t lead = min(words, (16 - ((size_t)out & 15)) % 16 / 4), wide = (words - lead) / 4;
+  uint4 *v = reinterpret_cast<uint4 *>(out + lead);
+  for (size_t i = t; i < wide; i += S) v[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
+  if (t < lead) out[t] = ~0u;
+  if (lead + 4 * wide + t < words) out[lead + 4 * wide + t] = ~0u;
+}
+static int fill_pending(void *out, size_t bytes) {
+  const size_t words = bytes / 4;
+  note_launches(1);
+  return launch_after(k_fill_pending, blocks_for(words, 4 * 256, (unsigned)ctx().num_sms * 4), 256u, (size_t)0,
+                      (unsigned *)out, words);
+}
+
 template <typename T, int B>
 static int nd_sweep_impl(dfm2g_ilu_s *p, bool forward, const T *in, T *out, const T *vcrs, const T *vdia,
                          const int *skip, bool prefilled, bool may_alloc) {
@@ -1048,7 +1067,7 @@ static int nd_sweep_impl(dfm2g_ilu_s *p, bool forward, const T *in, T *out, cons
     return DFM2G_OK;
   }
   if ((const void *)in == (const void *)out) return fail(DFM2G_ERR_ARG, "sync-free sweep needs in != out");
-  if (!prefilled) DFM2G_CUDA(cudaMemsetAsync(out, 0xFF, sizeof(T) * n * B, stream()));
+  if (!prefilled) DFM2G_TRY(fill_pending(out, sizeof(T) * n * B));
   if (p->sweep_mode == DFM2G_SWEEP_CHAINS || p->sweep_mode == DFM2G_SWEEP_AUTO) {
     const unsigned long long timeout = kWaitTimeoutNs + 20000ull * (forward ? p->nlev_f : p->nlev_b);
     bool usable = false, full = false;
@@ -1126,13 +1145,13 @@ static int sweep_impl(dfm2g_ilu_s *p, bool forward, const T *in, T *out, const T
     }  // else (a row too long for a unit, or not built): the sync-free schedule below
   }
   if (p->sweep_mode == DFM2G_SWEEP_PARTS && p->parts_ok) {
-    if (!prefilled) DFM2G_CUDA(cudaMemsetAsync(out, 0xFF, sizeof(T) * n * 3, stream()));
+    if (!prefilled) DFM2G_TRY(fill_pending(out, sizeof(T) * n * 3));
     const unsigned nlev = forward ? p->nlev_f : p->nlev_b;
     ran = DFM2G_SWEEP_PARTS;
     return part_sweep<T>(p, forward, in, out, vcrs, vdia, skip, kWaitTimeoutNs + 20000ull * nlev);
   }
   // sync-free, tile, chain and blob schedules: `out` is filled with the pending marker
-  if (!prefilled) DFM2G_CUDA(cudaMemsetAsync(out, 0xFF, sizeof(T) * n * 3, stream()));
+  if (!prefilled) DFM2G_TRY(fill_pending(out, sizeof(T) * n * 3));
   const bool auto_pick = p->sweep_mode == DFM2G_SWEEP_AUTO || p->sweep_mode == DFM2G_SWEEP_CLUSTER;
   if (p->sweep_mode == DFM2G_SWEEP_CHAINS || p->sweep_mode == DFM2G_SWEEP_TILES || auto_pick) {
     const unsigned nlev = forward ? p->nlev_f : p->nlev_b;
@@ -1543,6 +1562,13 @@ static int precond_host(dfm2g_ilu p, int prec, void *vec, int mem, int which /*1
   const size_t es = prec == DFM2G_F64 ? 8 : 4;
   void *a = prec == DFM2G_F64 ? (void *)p->tmp64a.p : (void *)p->tmp32a.p;
   void *b = prec == DFM2G_F64 ? (void *)p->tmp64b.p : (void *)p->tmp32b.p;
+  if (which == 3 && mem != DFM2G_MEM_HOST && ((size_t)vec & 15) == 0) {
+    // straight from the vector and back into it (each sweep fills its own output
+    // first); others go through aligned copies
+    DFM2G_TRY(ilu_sweep(p, prec, true, vec, b));
+    DFM2G_TRY(ilu_sweep(p, prec, false, b, vec));
+    return read_err(p);
+  }
   if (mem == DFM2G_MEM_HOST) {
     DFM2G_CUDA(cudaMemcpyAsync(a, vec, n * es, cudaMemcpyHostToDevice, stream()));
   } else {

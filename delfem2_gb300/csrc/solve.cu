@@ -51,11 +51,11 @@ constexpr int kThreads = 256;
 
 // Reliable updates ask for the deciding FP64 residual once the FP32 one is
 // below this share of the tolerance. Asked for at the tolerance itself, the
-// true residual stops anywhere near it and the solution's error with it (7e-10
-// to 1.2e-9 in the 48^3 gradients at a tolerance of 2e-11, by the summation
-// order alone); at half of it the answer is inside the tolerance at the first
-// refresh, for about 2% more iterations.
-constexpr double kFinalRefresh = 0.5;
+// true residual stops anywhere near it and the solution's error with it, by the
+// summation order alone (48^3 gradients at a tolerance of 2e-11, 14 seeds: 1.2e-11
+// to 2.0e-9; at 0.7 of it 1.1e-11 to 2.0e-9 with fewer above 5e-10, 1 against
+// 3), for about 1% more iterations.
+constexpr double kFinalRefresh = 0.7;
 
 // p.Ap fused into the SpMV Ap = K p (warp per block row); the last block sets
 // alpha = (r, Pr) / (p, Ap).
@@ -151,7 +151,7 @@ static int launch_spmv_pAp(dfm2g_bsr_s *m, IterState *st, const T *vcrs, const T
     DFM2G_TRY(allow_tma_smem(k_spmv_pAp_tma_c<T, B>, C::kSmem, attr_device));
     const unsigned nt = sizeof(T) == 8 ? m->ntiles64 : m->ntiles32;
     const unsigned *tiles = sizeof(T) == 8 ? m->tiles64.p : m->tiles32.p;
-    return launch_after(false, k_spmv_pAp_tma_c<T, B>, std::min(nt, (unsigned)ctx().num_sms), C::kThreads, C::kSmem,
+    return launch_after(k_spmv_pAp_tma_c<T, B>, std::min(nt, (unsigned)ctx().num_sms), C::kThreads, C::kSmem,
                         st, tiles, nt, rs, col, vcrs, vdia, pv, Ap, partials, m->err.p, kWaitTimeoutNs);
   }
   const unsigned blocks = blocks_for((size_t)m->nblk * 32, kThreads, (unsigned)ctx().num_sms * 8);
@@ -161,7 +161,7 @@ static int launch_spmv_pAp(dfm2g_bsr_s *m, IterState *st, const T *vcrs, const T
     else
       return k_spmv_pAp_nd<T, B>;
   }();
-  return launch_after(false, kernel, blocks, (unsigned)kThreads, (size_t)0, st, m->nblk, rs, col, vcrs, vdia, pv, Ap,
+  return launch_after(kernel, blocks, (unsigned)kThreads, (size_t)0, st, m->nblk, rs, col, vcrs, vdia, pv, Ap,
                       partials);
 }
 
@@ -677,18 +677,18 @@ template <int B>
 static int launch_refresh(dfm2g_bsr_s *m, IterState *st, size_t n, float *x32, float *r32, const Refine &rf) {
   const unsigned *rs = m->row_start.p, *col = m->col.p;
   const double *vcrs = m->vcrs.p, *vdia = m->vdia.p, *x64 = rf.x64;
-  DFM2G_TRY(launch_after(false, k_flush_x, reduce_blocks(n), (unsigned)kThreads, (size_t)0, (const IterState *)st, n,
+  DFM2G_TRY(launch_after(k_flush_x, reduce_blocks(n), (unsigned)kThreads, (size_t)0, (const IterState *)st, n,
                          rf.x64, x32));
   if (m->tiles_ok) {
     using C = TileCfgC<double, B>;
     static int attr_device = -1;
     DFM2G_TRY(allow_tma_smem(k_refresh_tma<B>, C::kSmem, attr_device));
-    return launch_after(false, k_refresh_tma<B>, std::min(m->ntiles64, (unsigned)ctx().num_sms), C::kThreads,
+    return launch_after(k_refresh_tma<B>, std::min(m->ntiles64, (unsigned)ctx().num_sms), C::kThreads,
                         C::kSmem, st, (const unsigned *)m->tiles64.p, m->ntiles64, rs, col, vcrs, vdia, x64, rf.b64,
                         r32, g_ws.partials.p, m->err.p, kWaitTimeoutNs);
   }
   const unsigned blocks = blocks_for((size_t)m->nblk * 32, kThreads, (unsigned)ctx().num_sms * 8);
-  return launch_after(false, k_true_residual<B>, blocks, (unsigned)kThreads, (size_t)0, st, m->nblk, rs, col, vcrs,
+  return launch_after(k_true_residual<B>, blocks, (unsigned)kThreads, (size_t)0, st, m->nblk, rs, col, vcrs,
                       vdia, x64, rf.b64, r32, g_ws.partials.p);
 }
 
@@ -749,7 +749,7 @@ static int pcg_core(dfm2g_bsr_s *m, dfm2g_ilu_s *p, T *r, T *x, T *w0, T *w1, T 
       }
       {
         ProfScope ps(DFM2G_PROF_UPDATE, 1);
-        DFM2G_TRY(launch_after(false, k_update<T>, vec_blocks, th, none, st, n, r, x, (const T *)pv, (const T *)Ap,
+        DFM2G_TRY(launch_after(k_update<T>, vec_blocks, th, none, st, n, r, x, (const T *)pv, (const T *)Ap,
                                g_ws.partials.p, g_ws.hist.p, fa, fb));
       }
       if constexpr (sizeof(T) == 4) {
@@ -771,22 +771,22 @@ static int pcg_core(dfm2g_bsr_s *m, dfm2g_ilu_s *p, T *r, T *x, T *w0, T *w1, T 
         }
         if (vec_blocks == 1) {
           ProfScope ps(DFM2G_PROF_DOT, 1);
-          DFM2G_TRY(launch_after(false, k_dot_pupdate<T>, 1u, th, none, st, n, (const T *)r, (const T *)Pr, pv));
+          DFM2G_TRY(launch_after(k_dot_pupdate<T>, 1u, th, none, st, n, (const T *)r, (const T *)Pr, pv));
         } else {
           {
             ProfScope ps(DFM2G_PROF_DOT, 1);
-            DFM2G_TRY(launch_after(false, k_dot_beta<T>, vec_blocks, th, none, st, n, (const T *)r, (const T *)Pr,
+            DFM2G_TRY(launch_after(k_dot_beta<T>, vec_blocks, th, none, st, n, (const T *)r, (const T *)Pr,
                                    g_ws.partials.p));
           }
           {
             ProfScope ps(DFM2G_PROF_PUPDATE, 1);
-            DFM2G_TRY(launch_after(false, k_p_update<T>, vec_blocks, th, none, (const IterState *)st, n, pv,
+            DFM2G_TRY(launch_after(k_p_update<T>, vec_blocks, th, none, (const IterState *)st, n, pv,
                                    (const T *)Pr));
           }
         }
       } else {
         ProfScope ps(DFM2G_PROF_PUPDATE, 1);
-        DFM2G_TRY(launch_after(false, k_p_update<T>, vec_blocks, th, none, (const IterState *)st, n, pv,
+        DFM2G_TRY(launch_after(k_p_update<T>, vec_blocks, th, none, (const IterState *)st, n, pv,
                                (const T *)r));
       }
     }

@@ -611,7 +611,7 @@ int tile_launch(dfm2g_ilu_s *p, TileSched &ts, bool forward, const T *in, T *out
   A.timeout_ns = timeout;
   A.skip = skip;
   void *args[] = {(void *)&A, (void *)&in, (void *)&out};
-  DFM2G_TRY(launch_after(kernel, blocks, kThreads, smem, args, false));
+  DFM2G_TRY(launch_after(kernel, blocks, kThreads, smem, args));
   note_launches(1);
   *usable = true;
   return DFM2G_OK;

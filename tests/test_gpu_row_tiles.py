@@ -101,3 +101,29 @@ def test_solves(gpu, n, ndim):
     x = np.zeros(n * ndim)
     D.Solve_PCG_Mixed(b.copy(), x, 1e-11, K, ilu, method="reliable")
     assert rel(x) < 1e-10
+
+
+@pytest.mark.parametrize("n", [1, 41, 1366])
+@pytest.mark.parametrize("ndim", [1, 2, 3])
+@pytest.mark.parametrize("offset", [0, 1, 2, 3])
+def test_precond_of_a_device_vector(gpu, n, ndim, offset):
+    """SolvePrecond works straight in a device vector that starts on 16 bytes and through a copy in one that does not:
+    the same bits as the host vector's call either way, and nothing written beside the vector."""
+    torch = pytest.importorskip("torch")
+    import delfem2_gb300 as D
+    ind, col, row, val, dia = _system(n, ndim)
+    ilu = D.CPreconditionerILU()
+    K = _matrix(ind, col, val, dia, ndim)
+    ilu.Initialize_ILUk(K, 0)
+    ilu.CopyValue(K)
+    assert ilu.Decompose()
+    for dt in (np.float64, np.float32):
+        b = np.random.default_rng(4).standard_normal(n * ndim).astype(dt)
+        want = b.copy()
+        ilu.SolvePrecond(want)
+        room = torch.full((n * ndim + 8,), 7.0, dtype=getattr(torch, dt.__name__), device="cuda")
+        vec = room[offset:offset + n * ndim]
+        vec.copy_(torch.from_numpy(b))
+        ilu.SolvePrecond(vec)
+        assert np.array_equal(vec.cpu().numpy(), want)
+        assert (room[:offset] == 7.0).all() and (room[offset + n * ndim:] == 7.0).all()
