@@ -107,9 +107,9 @@ def algorithmic_bytes(kind: str, nb: int, nz: int, s: int, fused: bool = False) 
     """Bytes one launch of a kernel class must move (each array once per pass).
 
     nb block rows, nz off-diagonal blocks, s = bytes per value; index arrays u32.
-    nz/2 blocks lie in each triangle (the pattern is symmetric). fused: the
-    solver's cooperative kernels, where the SpMV launch also runs the update
-    pass and the dot launch the p update."""
+    nz/2 blocks lie in each triangle (the pattern is symmetric). fused: a solve
+    whose SpMV launch also runs the update pass and whose dot launch the p update
+    (no "update" class in its profile)."""
     v3 = 3 * s * nb
     if kind == "spmv":      # K values + col + row_start, p read, Ap written (+ the update pass)
         return 9 * s * (nz + nb) + 4 * nz + 4 * (nb + 1) + 2 * v3 + (8 * v3 if fused else 0)

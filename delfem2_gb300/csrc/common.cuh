@@ -194,6 +194,8 @@ __device__ __forceinline__ void st_release(unsigned *p, unsigned v) {
   asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 // First statement of a kernel launched by launch_after (no effect otherwise).
+// (Letting the next kernel's blocks in from here on, instead of at the end,
+// gained nothing and cost the scalar solves 6%: they hold registers and slots.)
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ unsigned long long globaltimer_ns() {
   unsigned long long t;

@@ -14,13 +14,13 @@
 // voxel meshes), and a dependency path crosses a tile boundary once per tile
 // instead of once per row or pencil of rows.
 //
-// Progress: tiles are handed out in increasing number (the first by CTA
-// index, later ones from a counter), every CTA is resident (cooperative
-// launch), and every dependency of a tile's row lies in a lower-numbered tile
-// or in an earlier step of the same tile. The lowest-numbered unfinished tile
-// is the current tile of some CTA (a CTA's next tile is numbered above its
-// current one), and all its outside dependencies are finished, so the sweep
-// cannot deadlock. Every wait is bounded (DFM2G_ERR_WAIT_TIMEOUT); a CTA that
+// Progress: tiles are handed out in increasing number from a counter, to CTAs
+// that are running, and every dependency of a tile's row lies in a
+// lower-numbered tile or in an earlier step of the same tile. The
+// lowest-numbered unfinished tile is the current tile of some running CTA (a
+// CTA's next tile is numbered above its current one), and all its outside
+// dependencies are finished, so the sweep cannot deadlock, wherever and whenever
+// the CTAs are placed. Every wait is bounded (DFM2G_ERR_WAIT_TIMEOUT); a CTA that
 // stops early first waits (bounded) for the copies it issued.
 #include <algorithm>
 #include <atomic>

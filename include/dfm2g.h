@@ -471,15 +471,14 @@ DFM2G_API int dfm2g_vec_set_zero(double *x, size_t n, int mem);
 /* Kernel classes timed when profiling is on (CUDA events around every launch
  * of the solver loops; adds a little overhead, so off by default). */
 enum dfm2g_prof_kind {
-  DFM2G_PROF_SPMV = 0,     /* Ap = K p fused with p.Ap (3x3 patterns with
-                              SpMV tiles: and the update, in one launch)       */
+  DFM2G_PROF_SPMV = 0,     /* Ap = K p fused with p.Ap                         */
   DFM2G_PROF_UPDATE = 1,   /* r -= a Ap, x += a p, |r|^2, and the pending-
                               marker fill of the sweep outputs                 */
   DFM2G_PROF_FILL = 2,     /* (unused: the fill is part of the update)        */
   DFM2G_PROF_FWD = 3,      /* forward sweep                                    */
   DFM2G_PROF_BWD = 4,      /* backward sweep                                   */
-  DFM2G_PROF_DOT = 5,      /* (r, z) and beta (3x3 patterns with SpMV tiles:
-                              and p = z + beta p, in one launch)              */
+  DFM2G_PROF_DOT = 5,      /* (r, z) and beta (vectors of up to 4,096
+                              elements: and p = z + beta p, in one launch)     */
   DFM2G_PROF_PUPDATE = 6,  /* p = z + beta p                                   */
   DFM2G_PROF_OUTER = 7,    /* FP64 residual / refinement kernels               */
   DFM2G_PROF_NKIND = 8
@@ -497,7 +496,7 @@ DFM2G_API int dfm2g_alloc_count(unsigned long long *count);
 /* Launches one tiny kernel that waits on a value nothing ever writes, bounded
  * by `timeout_ms`; must return DFM2G_ERR_WAIT_TIMEOUT with the context usable. */
 DFM2G_API int dfm2g_debug_wait_timeout(unsigned timeout_ms);
-/* Two rounds of the solver kernels' bounded grid barrier over 4 cooperative
+/* Two rounds of a bounded grid barrier over 4 cooperative
  * CTAs: DFM2G_OK when every CTA arrives; with one_block_absent one CTA returns
  * without arriving and the call must return DFM2G_ERR_WAIT_TIMEOUT after about
  * `timeout_ms`, with the context usable. */
