@@ -4,10 +4,11 @@
 //   forward, FP64      z_i = D_i^-1 in_i - sum_j (D_i^-1 L_ij) z_j
 //   forward, FP32      z_i = D_i^-1 (in_i - sum_j L_ij z_j)
 // In FP64 D^-1 is multiplied into the records when they are written (in FP64),
-// which leaves three FP64 instructions out of a step's chain; its error against
-// 64 bits is the unfolded one's (1.5e-15 and 2e-15 at 40 x 37 x 43 and
-// 63 x 64 x 61 voxels). In FP32 the same would round D^-1 L and D^-1 apart and
-// cost 16% in accuracy (9.5e-8 against 8.2e-8), so D^-1 is applied last there.
+// which leaves three FP64 instructions out of a step's chain; the sweep's error
+// is the unfolded one's (1.03e-16 against 1.04e-16 of quad precision at
+// 40 x 37 x 43 voxels, within 1% either way for random 1x1 to 3x3 blocks). In
+// FP32 the same would round D^-1 L and D^-1 apart and cost 16% in accuracy
+// (9.5e-8 against 8.2e-8), so D^-1 is applied last there.
 //
 // One CTA sweeps one tile at a time, step by step (a step: the tile's rows of
 // one local level). Its warps have three jobs:
@@ -36,7 +37,8 @@
 //
 // FP64 on GB300 issues one warp instruction per 64 cycles and SM quarter
 // whatever the number of active lanes, so an FP64 step is split over four
-// warps, one per quarter, six lanes a row: 13 FP64 instructions a step.
+// warps, one per quarter, six lanes a row: 13 FP64 instructions a step (14
+// backward, which adds the right-hand side last).
 #pragma once
 
 #include "common.cuh"
@@ -461,7 +463,6 @@ __global__ void __launch_bounds__(32 * (NW + HW + 1), 1)
     T acc[kAcc];
 #pragma unroll
     for (unsigned k = 0; k < kAcc; ++k) acc[k] = T(0);
-    if constexpr (!FWD && sizeof(T) == 8) acc[0] = h == 0 ? -c : T(0);
 #pragma unroll
     for (unsigned j = 0; j < MS; ++j) {
       if (j < kDeps || (S > 1 && h != S - 1)) {
@@ -473,9 +474,10 @@ __global__ void __launch_bounds__(32 * (NW + HW + 1), 1)
 #pragma unroll
     for (unsigned k = 1; k < kAcc; ++k) z += acc[k];
     if constexpr (S == 2) z += __shfl_sync(0xffffffffu, z, lane_ok ? (h == 0 ? lane + B : lane - B) : lane);
-    // FP32 subtracts the finished sum: started from the right-hand side, the
-    // chain would round at its magnitude in every product (1.2e-7 against 8.2e-8)
-    if constexpr (sizeof(T) == 4)
+    // the finished sum is subtracted: started from the right-hand side, the
+    // chain would round at its magnitude in every product (forward FP32 1.2e-7
+    // against 8.2e-8, backward FP64 1.8e-16 against 0.9e-16)
+    if constexpr (sizeof(T) == 4 || !FWD)
       z = c - z;
     else
       z = -z;

@@ -634,7 +634,7 @@ int tile_run(dfm2g_ilu_s *p, TileSched *pair, const TileShape &sh, bool forward,
 // spread over its neighbours' lines, diagonals included, so other segment
 // counts grow ragged tiles: 16 lines swept 20% faster than 20). FP32 3x3: 6 x 6
 // lines, three lanes a row. FP64 3x3: 4 x 4, six lanes a row on four warps (the
-// step's 13 FP64 instructions per warp are its time, whatever the rows, so
+// step's 13 or 14 FP64 instructions per warp are its time, whatever the rows, so
 // small tiles hop sooner: 65^3 nodes 200 us a sweep, 285 with 6 x 6 lines on
 // eight warps). 1x1 and 2x2: two lane groups per row.
 constexpr int kHw = 3, kHwNd = 4;  // fetch warps
