@@ -317,6 +317,20 @@ __device__ __forceinline__ void st_chunk(T *p, const Chunk<T> &c, bool wide) {
 }
 __device__ __forceinline__ bool on_16(const void *p) { return ((size_t)p & 15u) == 0; }
 
+// s += the chunk's products (FP32: as one FP32 run, or one by one).
+template <typename T>
+__device__ __forceinline__ void add_chunk(double &s, const Chunk<T> &a, const Chunk<T> &b, bool run) {
+  if (sizeof(T) == 4 && run) {
+    T acc = T(0);
+#pragma unroll
+    for (unsigned e = 0; e < Chunk<T>::V; ++e) acc += a.v[e] * b.v[e];
+    s += (double)acc;
+  } else {
+#pragma unroll
+    for (unsigned e = 0; e < Chunk<T>::V; ++e) s += (double)a.v[e] * (double)b.v[e];
+  }
+}
+
 // The CTA's grid-stride share of [0, n): many(k) for kUnroll chunks, the u-th at
 // element k + u * stride; one(k) for a chunk; last(k) for an element of the end.
 template <typename T, typename Many, typename One, typename Last>
@@ -329,13 +343,24 @@ __device__ __forceinline__ void chunk_pass(size_t n, Many &&many, One &&one, Las
   if (nv * V + t < n) last(nv * V + t);
 }
 
+// FP32 vectors: the products of the first fp32_runs(n) elements are added in
+// FP32 four at a time (a chunk), those of the others one by one in FP64. All of
+// them in FP64 would bound the pass by its FP64 instructions (3.2 M elements:
+// some 16 us of them beside 21 us of memory); a vector that does not fill the
+// machine with chunks has the time, and every FP32 run costs up to 1.2e-7 of
+// its sum.
+static size_t fp32_runs(size_t n) {
+  const size_t fill = (size_t)ctx().num_sms * 4 * kThreads * Chunk<float>::V;
+  return n / fill * fill;
+}
+
 // r -= alpha Ap; x += alpha p over the CTA's grid-stride share of the
-// vectors; returns the share of |r|^2 (FP32: a run of one chunk, accumulated
-// in FP64). When fill_a and fill_b are given, both are set to the sweeps'
-// pending marker chunk by chunk after Ap is read (Ap may alias fill_a).
+// vectors; returns the share of |r|^2 (FP32: in runs below element `runs`).
+// When fill_a and fill_b are given, both are set to the sweeps' pending marker
+// chunk by chunk after Ap is read (Ap may alias fill_a).
 template <typename T>
-__device__ __forceinline__ double update_pass(size_t n, T *r, T *x, const T *p, const T *Ap, double alpha, T *fill_a,
-                                              T *fill_b) {
+__device__ __forceinline__ double update_pass(size_t n, size_t runs, T *r, T *x, const T *p, const T *Ap,
+                                              double alpha, T *fill_a, T *fill_b) {
   using C = Chunk<T>;
   const bool wr = on_16(r), wx = on_16(x), wp = on_16(p), wa = on_16(Ap);  // fill_a, fill_b: workspace
   const T al = (T)alpha, pend = pending_marker<T>();
@@ -344,23 +369,18 @@ __device__ __forceinline__ double update_pass(size_t n, T *r, T *x, const T *p, 
   for (unsigned k = 0; k < C::V; ++k) mark.v[k] = pend;
   double rr = 0.0;
   auto finish = [&](size_t k, C rv, C xv, const C &pv, const C &av) {
-    [[maybe_unused]] T acc = T(0);
 #pragma unroll
     for (unsigned e = 0; e < C::V; ++e) {
       rv.v[e] += -al * av.v[e];
       xv.v[e] += al * pv.v[e];
-      if constexpr (sizeof(T) == 8)
-        rr += rv.v[e] * rv.v[e];
-      else
-        acc += rv.v[e] * rv.v[e];
     }
+    add_chunk(rr, rv, rv, k < runs);
     st_chunk(r + k, rv, wr);
     st_chunk(x + k, xv, wx);
     if (fill_a) {
       st_chunk(fill_a + k, mark, true);
       st_chunk(fill_b + k, mark, true);
     }
-    if constexpr (sizeof(T) == 4) rr += (double)acc;
   };
   chunk_pass<T>(
       n,
@@ -390,23 +410,12 @@ __device__ __forceinline__ double update_pass(size_t n, T *r, T *x, const T *p, 
   return rr;
 }
 
-// (r, z) over the CTA's share (FP32: a run of one chunk, accumulated in FP64).
+// (r, z) over the CTA's share (FP32: in runs below element `runs`).
 template <typename T>
-__device__ __forceinline__ double dot_pass(size_t n, const T *r, const T *z) {
+__device__ __forceinline__ double dot_pass(size_t n, size_t runs, const T *r, const T *z) {
   using C = Chunk<T>;
   const bool wr = on_16(r), wz = on_16(z);
   double s = 0.0;
-  auto add = [&](const C &a, const C &b) {
-    if constexpr (sizeof(T) == 8) {
-      s += a.v[0] * b.v[0];
-      s += a.v[1] * b.v[1];
-    } else {
-      T acc = T(0);
-#pragma unroll
-      for (unsigned e = 0; e < C::V; ++e) acc += a.v[e] * b.v[e];
-      s += (double)acc;
-    }
-  };
   chunk_pass<T>(
       n,
       [&](size_t k, size_t S) {
@@ -417,9 +426,9 @@ __device__ __forceinline__ double dot_pass(size_t n, const T *r, const T *z) {
           b[u] = ld_chunk(z + k + u * S, wz);
         }
 #pragma unroll
-        for (int u = 0; u < kUnroll; ++u) add(a[u], b[u]);
+        for (int u = 0; u < kUnroll; ++u) add_chunk(s, a[u], b[u], k + u * S < runs);
       },
-      [&](size_t k) { add(ld_chunk(r + k, wr), ld_chunk(z + k, wz)); },
+      [&](size_t k) { add_chunk(s, ld_chunk(r + k, wr), ld_chunk(z + k, wz), k < runs); },
       [&](size_t k) { s += (double)r[k] * (double)z[k]; });
   return s;
 }
@@ -491,13 +500,13 @@ __device__ __forceinline__ void update_tail(IterState *st, double total, double 
 // r -= alpha Ap; x += alpha p; |r|^2 -> history and the stop test
 // (update_pass, update_tail).
 template <typename T>
-__global__ void __launch_bounds__(kThreads) k_update(IterState *st, size_t n, T *__restrict__ r, T *__restrict__ x,
-                                                     const T *p, const T *Ap, double *partials, double *hist,
-                                                     T *fill_a, T *fill_b) {
+__global__ void __launch_bounds__(kThreads) k_update(IterState *st, size_t n, size_t runs, T *__restrict__ r,
+                                                     T *__restrict__ x, const T *p, const T *Ap, double *partials,
+                                                     double *hist, T *fill_a, T *fill_b) {
   __shared__ double sh[32];
   pdl_wait();
   if (st->done) return;
-  const double rr = update_pass<T>(n, r, x, p, Ap, st->alpha, fill_a, fill_b);
+  const double rr = update_pass<T>(n, runs, r, x, p, Ap, st->alpha, fill_a, fill_b);
   double total;
   if (grid_sum_last(rr, partials, &st->ticket[1], sh, &total)) update_tail(st, total, hist);
 }
@@ -515,12 +524,12 @@ __device__ __forceinline__ double take_rPr(IterState *st, double total) {
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kThreads) k_dot_beta(IterState *st, size_t n, const T *__restrict__ r,
+__global__ void __launch_bounds__(kThreads) k_dot_beta(IterState *st, size_t n, size_t runs, const T *__restrict__ r,
                                                        const T *__restrict__ z, double *partials) {
   __shared__ double sh[32];
   pdl_wait();
   if (st->done) return;
-  const double s = dot_pass<T>(n, r, z);
+  const double s = dot_pass<T>(n, runs, r, z);
   double total;
   if (grid_sum_last(s, partials, &st->ticket[2], sh, &total)) take_rPr(st, total);
 }
@@ -541,7 +550,7 @@ __global__ void __launch_bounds__(kThreads) k_dot_pupdate(IterState *st, size_t 
   __shared__ T beta_s;
   pdl_wait();
   if (st->done) return;
-  const double s = block_sum(dot_pass<T>(n, r, z), sh);
+  const double s = block_sum(dot_pass<T>(n, 0, r, z), sh);
   if (threadIdx.x == 0) beta_s = (T)take_rPr(st, s);
   __syncthreads();
   p_pass<T>(n, p, z, beta_s);
@@ -732,6 +741,7 @@ static int pcg_core(dfm2g_bsr_s *m, dfm2g_ilu_s *p, T *r, T *x, T *w0, T *w1, T 
   note_launches(1);
   DFM2G_LAUNCH_CHECK();
   const unsigned vec_blocks = reduce_blocks(n);
+  const size_t runs = fp32_runs(n);
   const int chunk = 16;
   const unsigned th = kThreads;
   const size_t none = 0;
@@ -749,7 +759,7 @@ static int pcg_core(dfm2g_bsr_s *m, dfm2g_ilu_s *p, T *r, T *x, T *w0, T *w1, T 
       }
       {
         ProfScope ps(DFM2G_PROF_UPDATE, 1);
-        DFM2G_TRY(launch_after(k_update<T>, vec_blocks, th, none, st, n, r, x, (const T *)pv, (const T *)Ap,
+        DFM2G_TRY(launch_after(k_update<T>, vec_blocks, th, none, st, n, runs, r, x, (const T *)pv, (const T *)Ap,
                                g_ws.partials.p, g_ws.hist.p, fa, fb));
       }
       if constexpr (sizeof(T) == 4) {
@@ -775,7 +785,7 @@ static int pcg_core(dfm2g_bsr_s *m, dfm2g_ilu_s *p, T *r, T *x, T *w0, T *w1, T 
         } else {
           {
             ProfScope ps(DFM2G_PROF_DOT, 1);
-            DFM2G_TRY(launch_after(k_dot_beta<T>, vec_blocks, th, none, st, n, (const T *)r, (const T *)Pr,
+            DFM2G_TRY(launch_after(k_dot_beta<T>, vec_blocks, th, none, st, n, runs, (const T *)r, (const T *)Pr,
                                    g_ws.partials.p));
           }
           {
