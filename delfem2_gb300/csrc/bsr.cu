@@ -93,6 +93,8 @@ static int tiles_build(dfm2g_bsr_s *m) {
   using C32 = TileCfgC<float, B>;
   using C64 = TileCfgC<double, B>;
   std::vector<unsigned> t32, t64;
+  for (unsigned i = 0; i < m->nblk; ++i)
+    if (m->h_row_start[i + 1] - m->h_row_start[i] > C64::kLongest) return DFM2G_OK;
   // Fewer rows than fill the machine at full tiles: shorter tiles, down to one
   // consumer warp for each quarter of an SM, so that a tile's rows (a latency
   // chain of their own each) run on more SMs at once.

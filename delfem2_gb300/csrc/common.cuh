@@ -329,7 +329,7 @@ struct dfm2g_bsr_s {
   bool f32_valid = false;
   unsigned pattern_version = 0;
   // row tiles of the TMA-staged SpMV (TileCfgC<float, ndim>, TileCfgC<double, ndim>); tiles_ok is
-  // false when a row alone exceeds a tile
+  // false when a row is longer than TileCfgC::kLongest
   dfm2g::DevBuf<unsigned> tiles32, tiles64;
   unsigned ntiles32 = 0, ntiles64 = 0;
   bool tiles_ok = false;
