@@ -56,6 +56,7 @@ struct Context {
   cudaStream_t own = nullptr;
   int device = -1;
   int num_sms = 0;
+  int *err_word = nullptr;  // pinned: an error word on its way to the host
 };
 Context &ctx();
 int ensure_context();

@@ -68,6 +68,7 @@ int ensure_context() {
     DFM2G_CUDA(cudaStreamCreateWithFlags(&g_ctx.own, cudaStreamNonBlocking));
     g_ctx.stream = g_ctx.own;
   }
+  if (!g_ctx.err_word) DFM2G_CUDA(cudaMallocHost(&g_ctx.err_word, sizeof(int)));
   g_ctx.num_sms = sms;
   g_ctx.device = dev;
   return DFM2G_OK;

@@ -169,7 +169,9 @@ DFM2G_API int dfm2g_bsr_add_dia(dfm2g_bsr m, double eps);
 /* MatVec: y = alpha*K*x + beta*y, ls_block_sparse.cpp:213-273 (y is scaled by
  * beta first, so a NaN in y survives beta == 0; the 1x1 / 2x2 / 3x3 loops of
  * 59-133). prec DFM2G_F32 uses the FP32
- * mirror of the values (refreshed by dfm2g_bsr_update_f32) and float vectors. */
+ * mirror of the values (refreshed by dfm2g_bsr_update_f32) and float vectors.
+ * A 1x1 or 2x2 product of device vectors is queued without waiting for it (and
+ * may be captured into a graph; FP32 once the mirror exists). */
 DFM2G_API int dfm2g_bsr_matvec(dfm2g_bsr m, int prec, void *y, double alpha, const void *x,
                                double beta, int mem);
 /* Refresh the FP32 mirror of the values from the FP64 values. */
