@@ -459,7 +459,7 @@ struct dfm2g_tetmesh_s {
   dfm2g::DevBuf<unsigned> slot;       // ntet*16 slot ids (diagonal: 0xffffffff)
   std::vector<unsigned> color_start;  // ncolor+1 (of the node colouring, reported only)
   dfm2g::DevBuf<double> geo;          // ntet*16: shape-function gradients, volume
-  dfm2g::DevBuf<double> stress;       // ntet*6, grown on demand
+  dfm2g::DevBuf<double> stress;       // 3x3 blocks: ntet*9 (6 in use, stiffness warping 9)
   // gather lists (fem.cu): edges with their tets, nodes with theirs
   unsigned nedge = 0, nedge_entries = 0, nnode_entries = 0;
   dfm2g::DevBuf<unsigned> eslot, eoff, elist, noff, nlist;

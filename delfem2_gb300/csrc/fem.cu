@@ -592,6 +592,9 @@ static int scan_exclusive(const unsigned *a, unsigned n, int flag, unsigned *out
 static int tet_lists_build(dfm2g_tetmesh_s *t, const dfm2g_bsr_s *m) {
   const unsigned np = (unsigned)t->np, nnz = (unsigned)m->nnz;
   DFM2G_TRY(t->geo.resize(t->ntet * 16 + 2));
+  // the stresses' workspace for every mode, so that no assembly allocates (it may
+  // be captured) and none moves a buffer that a captured one still writes
+  if (m->ndim == 3) DFM2G_TRY(t->stress.resize(t->ntet * 9 + 2));
   DFM2G_TRY(t->noff.resize(np + 1));
   if (t->ntet == 0) return DFM2G_OK;
   const unsigned grid = ctx().num_sms * 16;
@@ -637,7 +640,6 @@ static int tet_assemble(dfm2g_tetmesh_s *t, dfm2g_bsr_s *m, const TetParam &p, d
   if (t->ntet == 0) return DFM2G_OK;
   const double *stress = nullptr;
   if (p.disp) {
-    DFM2G_TRY(t->stress.ensure(t->ntet * (MODE == kWarp ? 9 : 6) + 2));
     k_tet_stress<MODE><<<blocks_for(t->ntet, 128), 128, 0, stream()>>>(t->ntet, t->tet.p, t->geo.p, p, t->stress.p);
     stress = t->stress.p;
   }
