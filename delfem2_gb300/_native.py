@@ -149,6 +149,7 @@ SIGNATURES = {
     "dfm2g_debug_wait_timeout": [_u],
     "dfm2g_debug_grid_barrier": [_u, _i],
     "dfm2g_debug_host_failure": [_i],
+    "dfm2g_debug_fail_alloc": [_u],
 }
 
 PROF_KINDS = ["spmv", "update", "fill", "fwd", "bwd", "dot", "pupdate", "outer"]

@@ -39,6 +39,7 @@ int host_failure() noexcept;
 // ---- instrumentation -----------------------------------------------------------
 void note_launches(unsigned n);
 void note_alloc();  // one device allocation (cudaMalloc) made by the library
+bool alloc_denied();  // this allocation is the one dfm2g_debug_fail_alloc asked to fail
 // Times the launches between construction and destruction as one `kind`
 // sample when profiling is on; counts them always.
 struct ProfScope {
@@ -81,9 +82,10 @@ struct DevBuf {
     release();
     if (count == 0) return DFM2G_OK;
     note_alloc();
-    cudaError_t e = cudaMalloc(&p, count * sizeof(T));
+    cudaError_t e = alloc_denied() ? cudaErrorMemoryAllocation : cudaMalloc(&p, count * sizeof(T));
     if (e != cudaSuccess) {
       p = nullptr;
+      cudaGetLastError();  // reported here, not by the next launch's check
       return fail(DFM2G_ERR_CUDA, "cudaMalloc(%zu bytes): %s", count * sizeof(T),
                   cudaGetErrorString(e));
     }
@@ -446,6 +448,7 @@ struct dfm2g_ilu_s {
   dfm2g::DevBuf<unsigned short> flow_tab;  // one-launch factorisation: update targets,
   dfm2g::DevBuf<unsigned> flow_flags;      // and the decomposition each row was last finished in
   unsigned flow_epoch = 0;
+  bool flow_ready = false;                 // both are there and filled
   int last_sched[2][2] = {{-1, -1}, {-1, -1}};  // schedule of the last sweep [f64][backward]
 };
 

@@ -91,6 +91,9 @@ static std::atomic<unsigned long long> g_allocs{0};
 void note_launches(unsigned n) { g_launches += n; }
 void note_alloc() { g_allocs += 1; }
 
+static std::atomic<unsigned> g_deny_alloc{0};  // allocations up to the one that fails; 0: none does
+bool alloc_denied() { return g_deny_alloc.load() != 0 && g_deny_alloc.fetch_sub(1) == 1; }
+
 static cudaEvent_t take_event() {
   if (!g_event_pool.empty()) {
     cudaEvent_t e = g_event_pool.back();
@@ -183,6 +186,13 @@ int dfm2g_launch_count(unsigned long long *count) try {
 int dfm2g_alloc_count(unsigned long long *count) try {
   if (!count) return fail(DFM2G_ERR_ARG, "null count");
   *count = g_allocs.load();
+  return DFM2G_OK;
+} catch (...) {
+  return host_failure();
+}
+
+int dfm2g_debug_fail_alloc(unsigned nth) try {
+  g_deny_alloc = nth;
   return DFM2G_OK;
 } catch (...) {
   return host_failure();

@@ -1341,6 +1341,7 @@ static int ilu_install_pattern(dfm2g_ilu p, unsigned n, unsigned ndim, size_t nn
   stream_schedules_reset(p);
   chain_schedules_reset(p);
   tile_schedules_reset(p);
+  p->flow_ready = false;
   p->flow_tab.release();
   p->flow_flags.release();
   if (ndim == 3) {  // the blob and row-range schedules are written for 3x3 blocks
@@ -1366,8 +1367,9 @@ static int ilu_install_pattern(dfm2g_ilu p, unsigned n, unsigned ndim, size_t nn
 }
 
 // The factorisation in one launch (k_ilu_factor_flow); *flowed stays false
-// when a row does not fit shared memory or the target table would exceed
-// kFlowTabMax bytes (then one launch per level).
+// when a row does not fit shared memory, the target table would exceed
+// kFlowTabMax bytes or there is no device memory for it (then one launch per
+// level, which needs none).
 constexpr size_t kFlowTabMax = size_t(1) << 30;
 
 template <int B, int R>
@@ -1409,15 +1411,19 @@ static int factor_flow(dfm2g_ilu p, bool *flowed) {
   const size_t warp_bytes = ((size_t)(maxnb + 1) * B * B * 8 + (size_t)p->max_lower * maxu * 2 + 15) / 16 * 16;
   const size_t tab = p->nnz * maxu;
   if (warp_bytes * kFlowWarps > 200u * 1024u || tab * 2 > kFlowTabMax) return DFM2G_OK;
-  if (!p->flow_tab.p) {
-    DFM2G_TRY(p->flow_tab.resize(tab + 1));
-    DFM2G_TRY(p->flow_flags.resize(p->nblk));
+  if (!p->flow_ready) {
+    if (p->flow_tab.resize(tab + 1) != DFM2G_OK || p->flow_flags.resize(p->nblk) != DFM2G_OK) {
+      p->flow_tab.release();
+      p->flow_flags.release();
+      return DFM2G_OK;
+    }
     DFM2G_CUDA(cudaMemsetAsync(p->flow_flags.p, 0, sizeof(unsigned) * p->nblk, stream()));
     p->flow_epoch = 0;
     k_ilu_targets<<<blocks_for((size_t)p->nblk * 32, 256, ctx().num_sms * 16), 256, 0, stream()>>>(
         p->nblk, p->row_start.p, p->col.p, p->dia_ind.p, maxu, p->flow_tab.p);
     note_launches(1);
     DFM2G_LAUNCH_CHECK();
+    p->flow_ready = true;
   }
   if (p->flow_epoch == 0xFFFFFFFEu) {  // the flags' epochs are used up: start over
     DFM2G_CUDA(cudaMemsetAsync(p->flow_flags.p, 0, sizeof(unsigned) * p->nblk, stream()));

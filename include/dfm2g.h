@@ -507,6 +507,9 @@ DFM2G_API int dfm2g_debug_grid_barrier(unsigned timeout_ms, int one_block_absent
  * memory, 1: a standard exception, 2: anything else); must return
  * DFM2G_ERR_HOST with a message for dfm2g_last_error(). */
 DFM2G_API int dfm2g_debug_host_failure(int kind);
+/* Host only: the nth device allocation from now on fails as if the device were
+ * out of memory (0: none does). */
+DFM2G_API int dfm2g_debug_fail_alloc(unsigned nth);
 
 #ifdef __cplusplus
 }
