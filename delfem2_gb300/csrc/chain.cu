@@ -631,12 +631,13 @@ DevBuf<unsigned char> &chain_bytes(ChainSched &cs, float) { return cs.bytes32; }
 }  // namespace
 
 // Builds the chains of one direction (first use), rewrites the records of the
-// value type after each decomposition, and launches the sweep; false in
+// value type after each decomposition, sets `fill` bytes of `out` to the pending
+// marker and launches the sweep; false in
 // *usable when the pattern's records do not fit the shared-memory ring, or
 // when !may_alloc and the chains or records do not exist yet.
 template <typename T>
-int chain_sweep(dfm2g_ilu_s *p, bool forward, const T *in, T *out, const T *vcrs, const T *vdia, const int *skip,
-                unsigned long long timeout, bool may_alloc, bool *usable) {
+int chain_sweep(dfm2g_ilu_s *p, bool forward, const T *in, T *out, size_t fill, const T *vcrs, const T *vdia,
+                const int *skip, unsigned long long timeout, bool may_alloc, bool *usable) {
   ChainSched &cs = forward ? p->cs_f : p->cs_b;
   *usable = false;
   if (!may_alloc && (!cs.built || !cs.ok || !chain_bytes(cs, T(0)).p)) return DFM2G_OK;
@@ -687,15 +688,16 @@ int chain_sweep(dfm2g_ilu_s *p, bool forward, const T *in, T *out, const T *vcrs
   int *err = p->err.p;
   void *args[] = {(void *)&nchain, (void *)&chains, (void *)&bp, (void *)&rec, (void *)&m, (void *)&vo,
                   (void *)&in, (void *)&out, (void *)&ctr, (void *)&err, (void *)&timeout, (void *)&skip};
+  DFM2G_TRY(fill_pending(out, fill));
   DFM2G_CUDA(cudaLaunchCooperativeKernel(kernel, dim3(blocks), dim3(kChThreads), args, smem, stream()));
   note_launches(1);
   *usable = true;
   return DFM2G_OK;
 }
 
-template int chain_sweep<float>(dfm2g_ilu_s *, bool, const float *, float *, const float *, const float *,
+template int chain_sweep<float>(dfm2g_ilu_s *, bool, const float *, float *, size_t, const float *, const float *,
                                 const int *, unsigned long long, bool, bool *);
-template int chain_sweep<double>(dfm2g_ilu_s *, bool, const double *, double *, const double *, const double *,
+template int chain_sweep<double>(dfm2g_ilu_s *, bool, const double *, double *, size_t, const double *, const double *,
                                  const int *, unsigned long long, bool, bool *);
 
 // Drops the chains and records (a new pattern); rebuilt on first use.

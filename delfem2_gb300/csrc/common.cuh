@@ -470,6 +470,7 @@ struct dfm2g_tetmesh_s {
 
 namespace dfm2g {
 // cross-file internals
+int fill_pending(void *out, size_t bytes);  // `bytes` of `out` to the sweeps' pending marker
 int ilu_sweep(dfm2g_ilu_s *p, int prec, bool forward, const void *in, void *out);
 int ilu_sweep_guarded(dfm2g_ilu_s *p, int prec, bool forward, const void *in, void *out, const int *skip);
 int color_elements(const unsigned *elem, size_t nelem, unsigned nno, size_t np, std::vector<unsigned> &by_color,
@@ -485,12 +486,12 @@ int stream_sweep(dfm2g_ilu_s *p, bool forward, const T *in, T *out, const T *vcr
                  unsigned long long timeout, bool may_alloc, bool *usable);
 void stream_schedules_reset(dfm2g_ilu_s *p);
 template <typename T>
-int chain_sweep(dfm2g_ilu_s *p, bool forward, const T *in, T *out, const T *vcrs, const T *vdia, const int *skip,
-                unsigned long long timeout, bool may_alloc, bool *usable);
+int chain_sweep(dfm2g_ilu_s *p, bool forward, const T *in, T *out, size_t fill, const T *vcrs, const T *vdia,
+                const int *skip, unsigned long long timeout, bool may_alloc, bool *usable);
 void chain_schedules_reset(dfm2g_ilu_s *p);
 template <typename T>
-int tile_sweep(dfm2g_ilu_s *p, bool forward, const T *in, T *out, const int *skip, unsigned long long timeout,
-               bool may_alloc, bool force, bool *usable, bool *full);
+int tile_sweep(dfm2g_ilu_s *p, bool forward, const T *in, T *out, size_t fill, const int *skip,
+               unsigned long long timeout, bool may_alloc, bool force, bool *usable, bool *full);
 void tile_schedules_reset(dfm2g_ilu_s *p);
 template <typename T>
 int cluster_sweep(dfm2g_ilu_s *p, bool forward, const T *in, T *out, const T *vcrs, const T *vdia, const int *skip,

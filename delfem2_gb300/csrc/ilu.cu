@@ -1031,7 +1031,8 @@ __global__ void __launch_bounds__(256) k_fill_pending(unsigned *__restrict__ out
   if (t < lead) out[t] = ~0u;
   if (lead + 4 * wide + t < words) out[lead + 4 * wide + t] = ~0u;
 }
-static int fill_pending(void *out, size_t bytes) {
+int fill_pending(void *out, size_t bytes) {
+  if (bytes == 0) return DFM2G_OK;
   const size_t words = bytes / 4;
   note_launches(1);
   return launch_after(k_fill_pending, blocks_for(words, 4 * 256, (unsigned)ctx().num_sms * 4), 256u, (size_t)0,
@@ -1067,12 +1068,14 @@ static int nd_sweep_impl(dfm2g_ilu_s *p, bool forward, const T *in, T *out, cons
     return DFM2G_OK;
   }
   if ((const void *)in == (const void *)out) return fail(DFM2G_ERR_ARG, "sync-free sweep needs in != out");
-  if (!prefilled) DFM2G_TRY(fill_pending(out, sizeof(T) * n * B));
+  // `out` is filled right before a launch, after all that may fail: a vector that
+  // is swept in place is still the caller's when memory for the records is refused
+  const size_t fill = prefilled ? 0 : sizeof(T) * n * B;
   if (p->sweep_mode == DFM2G_SWEEP_CHAINS || p->sweep_mode == DFM2G_SWEEP_AUTO) {
     const unsigned long long timeout = kWaitTimeoutNs + 20000ull * (forward ? p->nlev_f : p->nlev_b);
     bool usable = false, full = false;
-    DFM2G_TRY(tile_sweep<T>(p, forward, in, out, skip, timeout, may_alloc, false, &usable, &full));
-    if (!usable) DFM2G_TRY(chain_sweep<T>(p, forward, in, out, vcrs, vdia, skip, timeout, may_alloc, &usable));
+    DFM2G_TRY(tile_sweep<T>(p, forward, in, out, fill, skip, timeout, may_alloc, false, &usable, &full));
+    if (!usable) DFM2G_TRY(chain_sweep<T>(p, forward, in, out, fill, vcrs, vdia, skip, timeout, may_alloc, &usable));
     if (usable) {
       ran = DFM2G_SWEEP_CHAINS;
       return DFM2G_OK;
@@ -1081,6 +1084,7 @@ static int nd_sweep_impl(dfm2g_ilu_s *p, bool forward, const T *in, T *out, cons
   void *kernel = forward ? (void *)k_sweep_syncfree_nd<T, true, B> : (void *)k_sweep_syncfree_nd<T, false, B>;
   int *cache = &p->coop_cache[sizeof(T) == 8 ? 1 : 0][forward ? 1 : 0][0];
   DFM2G_TRY(coop_blocks<T>(kernel, cache));
+  DFM2G_TRY(fill_pending(out, fill));
   const unsigned want = blocks_for((size_t)n * 32, 256);
   const unsigned blocks =
       std::min<unsigned>(std::min<unsigned>(want, (unsigned)*cache), kNdSweepCtasPerSm * (unsigned)ctx().num_sms);
@@ -1150,20 +1154,21 @@ static int sweep_impl(dfm2g_ilu_s *p, bool forward, const T *in, T *out, const T
     ran = DFM2G_SWEEP_PARTS;
     return part_sweep<T>(p, forward, in, out, vcrs, vdia, skip, kWaitTimeoutNs + 20000ull * nlev);
   }
-  // sync-free, tile, chain and blob schedules: `out` is filled with the pending marker
-  if (!prefilled) DFM2G_TRY(fill_pending(out, sizeof(T) * n * 3));
+  // sync-free, tile, chain and blob schedules: `out` is filled with the pending
+  // marker right before the launch (see nd_sweep_impl)
+  const size_t fill = prefilled ? 0 : sizeof(T) * n * 3;
   const bool auto_pick = p->sweep_mode == DFM2G_SWEEP_AUTO || p->sweep_mode == DFM2G_SWEEP_CLUSTER;
   if (p->sweep_mode == DFM2G_SWEEP_CHAINS || p->sweep_mode == DFM2G_SWEEP_TILES || auto_pick) {
     const unsigned nlev = forward ? p->nlev_f : p->nlev_b;
     const unsigned long long timeout = kWaitTimeoutNs + 20000ull * nlev;
     bool usable = false, full = false;
-    DFM2G_TRY(tile_sweep<T>(p, forward, in, out, skip, timeout, may_alloc, p->sweep_mode == DFM2G_SWEEP_TILES,
+    DFM2G_TRY(tile_sweep<T>(p, forward, in, out, fill, skip, timeout, may_alloc, p->sweep_mode == DFM2G_SWEEP_TILES,
                             &usable, &full));
     if (usable) {
       ran = !auto_pick ? p->sweep_mode : full ? DFM2G_SWEEP_TILES : DFM2G_SWEEP_CHAINS;
       return DFM2G_OK;
     }  // else (rows too long for the tiles' records, or not built): one warp per chain
-    DFM2G_TRY(chain_sweep<T>(p, forward, in, out, vcrs, vdia, skip, timeout, may_alloc, &usable));
+    DFM2G_TRY(chain_sweep<T>(p, forward, in, out, fill, vcrs, vdia, skip, timeout, may_alloc, &usable));
     if (usable) {
       ran = DFM2G_SWEEP_CHAINS;
       return DFM2G_OK;
@@ -1173,6 +1178,7 @@ static int sweep_impl(dfm2g_ilu_s *p, bool forward, const T *in, T *out, const T
     const GroupSched &gs = forward ? p->gs_f : p->gs_b;
     if (p->sweep_mode == DFM2G_SWEEP_GROUPS && gs.ok && gs.values_ok) {
       ran = DFM2G_SWEEP_GROUPS;
+      DFM2G_TRY(fill_pending(out, fill));
       return group_sweep(p, forward, (const float *)in, (float *)out, skip);
     }
   }
@@ -1182,6 +1188,7 @@ static int sweep_impl(dfm2g_ilu_s *p, bool forward, const T *in, T *out, const T
                       : (forward ? (void *)k_sweep_syncfree<T, true, 4> : (void *)k_sweep_syncfree<T, false, 4>);
   int *cache = &p->coop_cache[sizeof(T) == 8 ? 1 : 0][forward ? 1 : 0][wide ? 1 : 0];
   DFM2G_TRY(coop_blocks<T>(kernel, cache));
+  DFM2G_TRY(fill_pending(out, fill));
   const unsigned want = blocks_for((size_t)n * 32, 256);
   const unsigned blocks = std::min<unsigned>(want, (unsigned)*cache);
   const uint4 *meta = forward ? p->meta_f.p : p->meta_b.p;

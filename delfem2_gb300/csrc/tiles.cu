@@ -546,7 +546,7 @@ void *tile_kernel(bool forward) {
 }
 
 template <typename T, int B, int S, int NW, int HW, int MSA, int MSB, int MSC, int MSD>
-int tile_launch(dfm2g_ilu_s *p, TileSched &ts, bool forward, const T *in, T *out, const int *skip,
+int tile_launch(dfm2g_ilu_s *p, TileSched &ts, bool forward, const T *in, T *out, size_t fill, const int *skip,
                 unsigned long long timeout, bool *usable) {
   constexpr unsigned kRow = kTiXw<T, B> * (unsigned)sizeof(T);
   constexpr unsigned kThreads = 32 * (NW + HW + 1);
@@ -611,23 +611,25 @@ int tile_launch(dfm2g_ilu_s *p, TileSched &ts, bool forward, const T *in, T *out
   A.timeout_ns = timeout;
   A.skip = skip;
   void *args[] = {(void *)&A, (void *)&in, (void *)&out};
+  DFM2G_TRY(fill_pending(out, fill));
   DFM2G_TRY(launch_after(kernel, blocks, kThreads, smem, args));
   note_launches(1);
   *usable = true;
   return DFM2G_OK;
 }
 
-// Prepares `pair` (both directions) and sweeps; nothing is done (*usable
+// Prepares `pair` (both directions), sets `fill` bytes of `out` to the pending
+// marker and sweeps; nothing is done (*usable
 // stays false) when the pattern's rows are too long, or when !may_alloc and
 // the records do not exist yet.
 template <typename T, int B, int S, int NW, int HW, int MSA, int MSB, int MSC, int MSD>
-int tile_run(dfm2g_ilu_s *p, TileSched *pair, const TileShape &sh, bool forward, const T *in, T *out, const int *skip,
-             unsigned long long timeout, bool may_alloc, bool force, bool *usable) {
+int tile_run(dfm2g_ilu_s *p, TileSched *pair, const TileShape &sh, bool forward, const T *in, T *out, size_t fill,
+             const int *skip, unsigned long long timeout, bool may_alloc, bool force, bool *usable) {
   TileSched &ts = pair[forward ? 0 : 1];
   if (!may_alloc && (!ts.built || !ts.ok || !ts.bytes.p)) return DFM2G_OK;
   if (!ts.built || (force && ts.thin)) DFM2G_TRY(tile_build(p, pair, sh, force));
   if (!ts.ok) return DFM2G_OK;
-  return tile_launch<T, B, S, NW, HW, MSA, MSB, MSC, MSD>(p, ts, forward, in, out, skip, timeout, usable);
+  return tile_launch<T, B, S, NW, HW, MSA, MSB, MSC, MSD>(p, ts, forward, in, out, fill, skip, timeout, usable);
 }
 
 // Shapes. The tiles are squares of z lines on the voxel grids (a row's offers
@@ -653,31 +655,33 @@ constexpr TileShape kShapeNd1{1, 2, 64 * 65, 64, 64, sizeof(T), sizeof(T), {4, 8
 // reports as tiles; the same sweep over thinner patterns (cloth sheets, fill-in,
 // 1x1 and 2x2 blocks, small FP64 systems) it reports as chains.
 template <typename T>
-int tile_sweep(dfm2g_ilu_s *p, bool forward, const T *in, T *out, const int *skip, unsigned long long timeout,
-               bool may_alloc, bool force, bool *usable, bool *full) {
+int tile_sweep(dfm2g_ilu_s *p, bool forward, const T *in, T *out, size_t fill, const int *skip,
+               unsigned long long timeout, bool may_alloc, bool force, bool *usable, bool *full) {
   constexpr bool f64 = sizeof(T) == 8;
   TileSched *pair = p->tiles[f64 ? 1 : 0];
   *usable = *full = false;
   if (p->ndim == 1)
-    return tile_run<T, 1, 2, 4, kHwNd, 4, 8, 8, 8>(p, pair, kShapeNd1<T>, forward, in, out, skip, timeout, may_alloc,
-                                             force, usable);
+    return tile_run<T, 1, 2, 4, kHwNd, 4, 8, 8, 8>(p, pair, kShapeNd1<T>, forward, in, out, fill, skip, timeout,
+                                             may_alloc, force, usable);
   if (p->ndim == 2)
-    return tile_run<T, 2, 2, 4, kHwNd, 4, 8, 8, 8>(p, pair, kShapeNd2<T>, forward, in, out, skip, timeout, may_alloc,
-                                             force, usable);
+    return tile_run<T, 2, 2, 4, kHwNd, 4, 8, 8, 8>(p, pair, kShapeNd2<T>, forward, in, out, fill, skip, timeout,
+                                             may_alloc, force, usable);
   constexpr TileShape sh = f64 ? kShape64 : kShape32;
   if constexpr (f64)
-    DFM2G_TRY((tile_run<T, 3, 2, 4, kHw, 3, 4, 7, 8>(p, pair, sh, forward, in, out, skip, timeout, may_alloc, force, usable)));
+    DFM2G_TRY((tile_run<T, 3, 2, 4, kHw, 3, 4, 7, 8>(p, pair, sh, forward, in, out, fill, skip, timeout,
+                                                     may_alloc, force, usable)));
   else
-    DFM2G_TRY((tile_run<T, 3, 1, 4, kHw, 7, 8, 14, 16>(p, pair, sh, forward, in, out, skip, timeout, may_alloc, force, usable)));
+    DFM2G_TRY((tile_run<T, 3, 1, 4, kHw, 7, 8, 14, 16>(p, pair, sh, forward, in, out, fill, skip, timeout,
+                                                       may_alloc, force, usable)));
   *full = *usable && (forward ? p->max_lower : p->max_upper) <= kTiAutoDeps &&
           2.0 * pair[forward ? 0 : 1].rows_per_step >= sh.segs && (!f64 || p->nblk >= kTi64MinRows);
   return DFM2G_OK;
 }
 
-template int tile_sweep<float>(dfm2g_ilu_s *, bool, const float *, float *, const int *, unsigned long long, bool,
-                               bool, bool *, bool *);
-template int tile_sweep<double>(dfm2g_ilu_s *, bool, const double *, double *, const int *, unsigned long long, bool,
-                                bool, bool *, bool *);
+template int tile_sweep<float>(dfm2g_ilu_s *, bool, const float *, float *, size_t, const int *, unsigned long long,
+                               bool, bool, bool *, bool *);
+template int tile_sweep<double>(dfm2g_ilu_s *, bool, const double *, double *, size_t, const int *, unsigned long long,
+                                bool, bool, bool *, bool *);
 
 // Drops the tiles and records (a new pattern); rebuilt on first use.
 void tile_schedules_reset(dfm2g_ilu_s *p) {
