@@ -306,7 +306,7 @@ __global__ void __launch_bounds__(kChThreads) k_sweep_chain(unsigned nchain, con
           zp1 = u[1];
         }
       }
-      if (lane < (unsigned)B) st_relaxed(out + (size_t)sm.x * B + lane, lane == 0 ? zp0 : zp1);
+      if (lane < (unsigned)B) st_relaxed(out + (size_t)sm.x * B + lane, settled(lane == 0 ? zp0 : zp1));
     };
     auto finish = [&](unsigned t, ChainStage<T, NV> &S) {
       const unsigned s = t % kChSlots;
@@ -384,7 +384,7 @@ __global__ void __launch_bounds__(kChThreads) k_sweep_chain(unsigned nchain, con
         } else {
           za = -pick3(s3, a);
         }
-        if (lane < 3) st_relaxed(out + (size_t)sm.x * 3 + lane, za);
+        if (lane < 3) st_relaxed(out + (size_t)sm.x * 3 + lane, settled(za));
         zp0 = __shfl_sync(0xffffffffu, za, 0);
         zp1 = __shfl_sync(0xffffffffu, za, 1);
         zp2 = __shfl_sync(0xffffffffu, za, 2);

@@ -206,12 +206,18 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
   return t;
 }
 
-// "Not yet written" marker for values produced by the sync-free sweeps: an
-// all-ones NaN. Arithmetic on the GPU only produces the canonical NaN
-// (0x7fffffff / 0x7fffffffffffffff), so a computed value never equals it.
+// "Not yet written" marker for values produced by the sweeps: an all-ones NaN.
+// FP32 arithmetic only produces the NaN 0x7fffffff, so a computed value never
+// equals it. FP64 arithmetic makes 0xfff8000000000000 but hands on the payload of
+// a NaN operand, so an all-ones NaN (or, negated, 0x7fff...f) among the inputs
+// could come out as the marker: settled() is what a sweep stores of a value.
 __device__ __forceinline__ bool is_pending(float v) { return __float_as_uint(v) == 0xffffffffu; }
 __device__ __forceinline__ bool is_pending(double v) {
   return __double_as_longlong(v) == (long long)-1;
+}
+__device__ __forceinline__ float settled(float v) { return v; }
+__device__ __forceinline__ double settled(double v) {
+  return is_pending(v) ? __longlong_as_double(0x7fffffffffffffffll) : v;
 }
 template <typename T>
 __device__ __forceinline__ T pending_value() {

@@ -797,7 +797,7 @@ __device__ __forceinline__ void sweep_finish(const SweepRow<T, NR> &R, const Row
     else
       z = lane == 0 ? t0 : (lane == 1 ? t1 : t2);
     if (WAIT)
-      st_relaxed(out + (size_t)R.i * 3 + lane, z);
+      st_relaxed(out + (size_t)R.i * 3 + lane, settled(z));
     else
       out[(size_t)R.i * 3 + lane] = z;
   }
@@ -957,7 +957,7 @@ __device__ __forceinline__ void nd_sweep_finish(const NdSweepRow<T, B> &R, unsig
     } else {
       z = t;
     }
-    st_relaxed(out + (size_t)R.i * B + lane, z);
+    st_relaxed(out + (size_t)R.i * B + lane, settled(z));
   }
 }
 

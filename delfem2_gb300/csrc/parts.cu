@@ -157,6 +157,7 @@ __device__ __forceinline__ void part_finish(const PartRow<T> &R, const RowLane &
       z = R.d[0] * t0 + R.d[1] * t1 + R.d[2] * t2;
     else
       z = lane == 0 ? t0 : (lane == 1 ? t1 : t2);
+    z = settled(z);
     *(volatile T *)(xs + (size_t)(R.i - r0) * 3 + lane) = z;
     st_relaxed(out + (size_t)R.i * 3 + lane, z);
   }

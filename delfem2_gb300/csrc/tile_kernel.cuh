@@ -490,7 +490,7 @@ __global__ void __launch_bounds__(32 * (NW + HW + 1), 1)
     }
     if (C.row != ~0u && h == kOut) {
       reinterpret_cast<T *>(xs + (size_t)C.local * kRow)[a] = z;
-      st_relaxed(out + (size_t)C.row * B + a, z);
+      st_relaxed(out + (size_t)C.row * B + a, settled(z));
     }
     if (!more) {
       // the end markers need this slot too (they touch only its descriptor)
