@@ -455,7 +455,8 @@ struct dfm2g_ilu_s {
   dfm2g::DevBuf<unsigned> flow_flags;      // and the decomposition each row was last finished in
   unsigned flow_epoch = 0;
   bool flow_ready = false;                 // both are there and filled
-  int last_sched[2][2] = {{-1, -1}, {-1, -1}};  // schedule of the last sweep [f64][backward]
+  // the last sweep [f64][backward]: its schedule's name and the schedule whose kernel ran
+  int last_sched[2][2] = {{-1, -1}, {-1, -1}}, last_kernel[2][2] = {{-1, -1}, {-1, -1}};
 };
 
 struct dfm2g_tetmesh_s {

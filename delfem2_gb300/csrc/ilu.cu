@@ -1042,7 +1042,10 @@ int fill_pending(void *out, size_t bytes) {
 template <typename T, int B>
 static int nd_sweep_impl(dfm2g_ilu_s *p, bool forward, const T *in, T *out, const T *vcrs, const T *vdia,
                          const int *skip, bool prefilled, bool may_alloc) {
-  int &ran = p->last_sched[sizeof(T) == 8 ? 1 : 0][forward ? 0 : 1];
+  auto ran = [&](int sched, int kernel) {
+    p->last_sched[sizeof(T) == 8 ? 1 : 0][forward ? 0 : 1] = sched;
+    p->last_kernel[sizeof(T) == 8 ? 1 : 0][forward ? 0 : 1] = kernel;
+  };
   const unsigned n = p->nblk;
   const uint4 *meta = forward ? p->meta_f.p : p->meta_b.p;
   if (p->sweep_mode == DFM2G_SWEEP_LEVELS) {
@@ -1064,7 +1067,7 @@ static int nd_sweep_impl(dfm2g_ilu_s *p, bool forward, const T *in, T *out, cons
     }
     note_launches((unsigned)(ls.size() - 1) + (in != out ? 1u : 0u));
     DFM2G_LAUNCH_CHECK();
-    ran = DFM2G_SWEEP_LEVELS;
+    ran(DFM2G_SWEEP_LEVELS, DFM2G_SWEEP_LEVELS);
     return DFM2G_OK;
   }
   if ((const void *)in == (const void *)out) return fail(DFM2G_ERR_ARG, "sync-free sweep needs in != out");
@@ -1075,9 +1078,10 @@ static int nd_sweep_impl(dfm2g_ilu_s *p, bool forward, const T *in, T *out, cons
     const unsigned long long timeout = kWaitTimeoutNs + 20000ull * (forward ? p->nlev_f : p->nlev_b);
     bool usable = false, full = false;
     DFM2G_TRY(tile_sweep<T>(p, forward, in, out, fill, skip, timeout, may_alloc, false, &usable, &full));
+    const int kernel = usable ? DFM2G_SWEEP_TILES : DFM2G_SWEEP_CHAINS;
     if (!usable) DFM2G_TRY(chain_sweep<T>(p, forward, in, out, fill, vcrs, vdia, skip, timeout, may_alloc, &usable));
     if (usable) {
-      ran = DFM2G_SWEEP_CHAINS;
+      ran(DFM2G_SWEEP_CHAINS, kernel);
       return DFM2G_OK;
     }  // else (records too long for the ring): the sync-free schedule below
   }
@@ -1095,7 +1099,7 @@ static int nd_sweep_impl(dfm2g_ilu_s *p, bool forward, const T *in, T *out, cons
                   (void *)&out, (void *)&err, (void *)&timeout, (void *)&skip};
   DFM2G_CUDA(cudaLaunchCooperativeKernel(kernel, dim3(blocks), dim3(256), args, 0, stream()));
   note_launches(1);
-  ran = DFM2G_SWEEP_SYNCFREE;
+  ran(DFM2G_SWEEP_SYNCFREE, DFM2G_SWEEP_SYNCFREE);
   return DFM2G_OK;
 }
 
@@ -1106,7 +1110,10 @@ static int sweep_impl(dfm2g_ilu_s *p, bool forward, const T *in, T *out, const T
   if (n == 0) return DFM2G_OK;
   if (p->ndim == 1) return nd_sweep_impl<T, 1>(p, forward, in, out, vcrs, vdia, skip, prefilled, may_alloc);
   if (p->ndim == 2) return nd_sweep_impl<T, 2>(p, forward, in, out, vcrs, vdia, skip, prefilled, may_alloc);
-  int &ran = p->last_sched[sizeof(T) == 8 ? 1 : 0][forward ? 0 : 1];
+  auto ran = [&](int sched, int kernel) {
+    p->last_sched[sizeof(T) == 8 ? 1 : 0][forward ? 0 : 1] = sched;
+    p->last_kernel[sizeof(T) == 8 ? 1 : 0][forward ? 0 : 1] = kernel;
+  };
   if (p->sweep_mode == DFM2G_SWEEP_LEVELS) {
     // levels in order; rows of one level are independent (in == out allowed)
     if (in != out) {
@@ -1126,7 +1133,7 @@ static int sweep_impl(dfm2g_ilu_s *p, bool forward, const T *in, T *out, const T
     }
     note_launches((unsigned)(ls.size() - 1) + (in != out ? 1u : 0u));
     DFM2G_LAUNCH_CHECK();
-    ran = DFM2G_SWEEP_LEVELS;
+    ran(DFM2G_SWEEP_LEVELS, DFM2G_SWEEP_LEVELS);
     return DFM2G_OK;
   }
   if ((const void *)in == (const void *)out) return fail(DFM2G_ERR_ARG, "sync-free sweep needs in != out");
@@ -1134,7 +1141,7 @@ static int sweep_impl(dfm2g_ilu_s *p, bool forward, const T *in, T *out, const T
     bool usable = false;
     DFM2G_TRY(cluster_sweep<T>(p, forward, in, out, vcrs, vdia, skip, &usable));
     if (usable) {
-      ran = DFM2G_SWEEP_CLUSTER;
+      ran(DFM2G_SWEEP_CLUSTER, DFM2G_SWEEP_CLUSTER);
       return DFM2G_OK;
     }  // else (the vector exceeds shared memory): the automatic choice below
   }
@@ -1144,14 +1151,14 @@ static int sweep_impl(dfm2g_ilu_s *p, bool forward, const T *in, T *out, const T
     DFM2G_TRY(stream_sweep<T>(p, forward, in, out, vcrs, vdia, skip, kWaitTimeoutNs + 20000ull * nlev, may_alloc,
                               &usable));
     if (usable) {
-      ran = DFM2G_SWEEP_BLOCK;
+      ran(DFM2G_SWEEP_BLOCK, DFM2G_SWEEP_BLOCK);
       return DFM2G_OK;
     }  // else (a row too long for a unit, or not built): the sync-free schedule below
   }
   if (p->sweep_mode == DFM2G_SWEEP_PARTS && p->parts_ok) {
     if (!prefilled) DFM2G_TRY(fill_pending(out, sizeof(T) * n * 3));
     const unsigned nlev = forward ? p->nlev_f : p->nlev_b;
-    ran = DFM2G_SWEEP_PARTS;
+    ran(DFM2G_SWEEP_PARTS, DFM2G_SWEEP_PARTS);
     return part_sweep<T>(p, forward, in, out, vcrs, vdia, skip, kWaitTimeoutNs + 20000ull * nlev);
   }
   // sync-free, tile, chain and blob schedules: `out` is filled with the pending
@@ -1165,19 +1172,19 @@ static int sweep_impl(dfm2g_ilu_s *p, bool forward, const T *in, T *out, const T
     DFM2G_TRY(tile_sweep<T>(p, forward, in, out, fill, skip, timeout, may_alloc, p->sweep_mode == DFM2G_SWEEP_TILES,
                             &usable, &full));
     if (usable) {
-      ran = !auto_pick ? p->sweep_mode : full ? DFM2G_SWEEP_TILES : DFM2G_SWEEP_CHAINS;
+      ran(!auto_pick ? p->sweep_mode : full ? DFM2G_SWEEP_TILES : DFM2G_SWEEP_CHAINS, DFM2G_SWEEP_TILES);
       return DFM2G_OK;
     }  // else (rows too long for the tiles' records, or not built): one warp per chain
     DFM2G_TRY(chain_sweep<T>(p, forward, in, out, fill, vcrs, vdia, skip, timeout, may_alloc, &usable));
     if (usable) {
-      ran = DFM2G_SWEEP_CHAINS;
+      ran(DFM2G_SWEEP_CHAINS, DFM2G_SWEEP_CHAINS);
       return DFM2G_OK;
     }  // else (records too long for the ring): the sync-free schedule below
   }
   if constexpr (sizeof(T) == 4) {
     const GroupSched &gs = forward ? p->gs_f : p->gs_b;
     if (p->sweep_mode == DFM2G_SWEEP_GROUPS && gs.ok && gs.values_ok) {
-      ran = DFM2G_SWEEP_GROUPS;
+      ran(DFM2G_SWEEP_GROUPS, DFM2G_SWEEP_GROUPS);
       DFM2G_TRY(fill_pending(out, fill));
       return group_sweep(p, forward, (const float *)in, (float *)out, skip);
     }
@@ -1199,7 +1206,7 @@ static int sweep_impl(dfm2g_ilu_s *p, bool forward, const T *in, T *out, const T
                   (void *)&out, (void *)&err, (void *)&timeout, (void *)&skip};
   DFM2G_CUDA(cudaLaunchCooperativeKernel(kernel, dim3(blocks), dim3(256), args, 0, stream()));
   note_launches(1);
-  ran = DFM2G_SWEEP_SYNCFREE;
+  ran(DFM2G_SWEEP_SYNCFREE, DFM2G_SWEEP_SYNCFREE);
   return DFM2G_OK;
 }
 
@@ -1358,10 +1365,9 @@ static int ilu_install_pattern(dfm2g_ilu p, unsigned n, unsigned ndim, size_t nn
     p->gs_f.ok = p->gs_b.ok = false;
     p->parts_ok = false;
   }
-  // Default: tiles or chains, picked per pattern and precision (3.24M DOF on
-  // GB300, FP32 / FP64 forward sweep: 0.47 / 0.88 ms over tiles against 0.58
-  // / 1.23 ms over chains and 0.91 / 2.19 ms sync-free; scalar Poisson on the
-  // same mesh, chains: mixed solve 165 ms against 225 ms sync-free).
+  // Default: over tiles where the records fit and the tiles are not thin, else
+  // over chains (3.24M DOF on GB300, forward sweep: 0.21 ms FP32 over tiles
+  // against 0.58 over chains and 0.91 sync-free).
   p->sweep_mode = DFM2G_SWEEP_AUTO;
   const size_t nvec = (size_t)n * ndim + 1;
   DFM2G_TRY(p->tmp64a.resize(nvec));
@@ -1717,6 +1723,16 @@ int dfm2g_ilu_last_schedule(dfm2g_ilu p, int prec, int backward, int *mode) try 
   if (!mode) return fail(DFM2G_ERR_ARG, "last_schedule: null out");
   if (prec != DFM2G_F64 && prec != DFM2G_F32) return fail(DFM2G_ERR_ARG, "last_schedule: bad precision");
   *mode = p->last_sched[prec == DFM2G_F64 ? 1 : 0][backward ? 1 : 0];
+  return DFM2G_OK;
+} catch (...) {
+  return host_failure();
+}
+
+int dfm2g_ilu_last_kernel(dfm2g_ilu p, int prec, int backward, int *mode) try {
+  DFM2G_TRY(check_ilu(p, false, false));
+  if (!mode) return fail(DFM2G_ERR_ARG, "last_kernel: null out");
+  if (prec != DFM2G_F64 && prec != DFM2G_F32) return fail(DFM2G_ERR_ARG, "last_kernel: bad precision");
+  *mode = p->last_kernel[prec == DFM2G_F64 ? 1 : 0][backward ? 1 : 0];
   return DFM2G_OK;
 } catch (...) {
   return host_failure();

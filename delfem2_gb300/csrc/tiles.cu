@@ -210,8 +210,8 @@ constexpr unsigned kSrcNone = 0xFFFFFFFFu, kSrcDia = 0xFFFFFFFEu;
 // voxels, nodes permuted at random, 10 rows a tile: 230 us FP32 a sweep, 425
 // over tiles; permuted within windows of 400, 20 rows: 1,640 against 950).
 constexpr unsigned kTiLeastRows = 16;
-constexpr unsigned kTiAutoDeps = 8;             // most dependency blocks of a row, and
-constexpr unsigned kTi64MinRows = 76u * 1024u;  // least rows in FP64, for DFM2G_SWEEP_AUTO to report tiles
+constexpr unsigned kTiAutoDeps = 8;             // most dependency blocks of a row, and least
+constexpr unsigned kTi64MinRows = 76u * 1024u;  // rows in FP64, of what tile_sweep calls full
 
 inline unsigned pad128u(unsigned x) { return (x + 127u) & ~127u; }
 
@@ -651,9 +651,11 @@ constexpr TileShape kShapeNd1{1, 2, 64 * 65, 64, 64, sizeof(T), sizeof(T), {4, 8
 
 // The tile schedule of one direction (force: thin tiles too). *full tells whether its steps are full
 // (at least half a step's segments on average, at most kTiAutoDeps
-// dependencies a row, and in FP64 kTi64MinRows rows): what DFM2G_SWEEP_AUTO
-// reports as tiles; the same sweep over thinner patterns (cloth sheets, fill-in,
-// 1x1 and 2x2 blocks, small FP64 systems) it reports as chains.
+// dependencies a row, and in FP64 kTi64MinRows rows): the patterns that
+// dfm2g_ilu_last_schedule calls tiles under DFM2G_SWEEP_AUTO. It is a name that
+// callers know, and decides nothing: the same sweep over thinner patterns (cloth
+// sheets, fill-in, 1x1 and 2x2 blocks, small FP64 systems) it calls chains, and
+// dfm2g_ilu_last_kernel says what ran.
 template <typename T>
 int tile_sweep(dfm2g_ilu_s *p, bool forward, const T *in, T *out, size_t fill, const int *skip,
                unsigned long long timeout, bool may_alloc, bool force, bool *usable, bool *full) {

@@ -248,9 +248,16 @@ class CPreconditionerILU:
         return m.value
 
     def last_schedule(self, fp64: bool, backward: bool) -> int:
-        """Schedule the last forward/backward sweep in FP64 or FP32 ran (-1: none yet)."""
+        """Schedule of the last forward/backward sweep in FP64 or FP32 (-1: none yet); for the automatic choice the
+        name its rule gives the pattern."""
         m = C.c_int(0)
         N.call("dfm2g_ilu_last_schedule", self._h, N.F64 if fp64 else N.F32, int(backward), C.byref(m))
+        return m.value
+
+    def last_kernel(self, fp64: bool, backward: bool) -> int:
+        """Kernel of that sweep: SWEEP_TILES (over tiles), SWEEP_CHAINS (a warp per chain) or the schedule's own."""
+        m = C.c_int(0)
+        N.call("dfm2g_ilu_last_kernel", self._h, N.F64 if fp64 else N.F32, int(backward), C.byref(m))
         return m.value
 
     def row_start(self):

@@ -77,19 +77,21 @@ enum dfm2g_sweep {
                                in global memory (when a range's results fit
                                in shared memory)                            */
   DFM2G_SWEEP_CHAINS = 5,   /* chains of consecutive rows in which each row
-                               depends on the one before, bundled into tiles
-                               as below; one warp per chain (that dependency
-                               in registers, the others polled) where rows
-                               have more than 15 blocks in a triangle or
-                               tiles would hold fewer than 16 rows           */
+                               depends on the one before, swept bundled into
+                               tiles as DFM2G_SWEEP_TILES does; one warp per
+                               chain (that dependency in registers, the others
+                               polled) where rows have more than 15 blocks in
+                               a triangle or tiles would hold fewer than 16
+                               rows (random node orders)                     */
   DFM2G_SWEEP_TILES = 6,    /* 3x3: rows in tiles of up to 36 (FP32) or 16
                                (FP64) segments of dependency chains (squares
                                of grid lines on voxel meshes), one CTA per
                                tile walking the tile's local levels with
                                shared-memory hand-offs inside the tile and
                                polls only across tiles; records TMA-streamed
-                               per level. Patterns whose rows have more than
-                               15 blocks in a triangle use a warp per chain  */
+                               per level, however few rows a tile holds.
+                               Patterns whose rows have more than 15 blocks
+                               in a triangle use a warp per chain            */
   DFM2G_SWEEP_CLUSTER = 8,  /* 3x3 systems whose solution vector fits in
                                shared memory (9,400 block rows FP64, 18,900
                                FP32): one thread-block cluster of 8 CTAs
@@ -100,12 +102,15 @@ enum dfm2g_sweep {
                                the chains on the systems measured except the
                                smallest (a cluster barrier and broadcast cost
                                about 1.3 us per level in FP32, 2.9 in FP64)  */
-  DFM2G_SWEEP_AUTO = 7      /* the default: DFM2G_SWEEP_TILES where the tiles'
-                               steps are at least half full, rows have at
-                               most 8 dependency blocks per triangle and, for
-                               FP64, the pattern has at least 77,824 rows;
-                               DFM2G_SWEEP_CHAINS otherwise (2-D meshes,
-                               fill-in patterns, small grids)                */
+  DFM2G_SWEEP_AUTO = 7      /* the default: sweeps as DFM2G_SWEEP_CHAINS does,
+                               over tiles or with a warp per chain
+                               (dfm2g_ilu_last_kernel tells which).
+                               dfm2g_ilu_last_schedule names it
+                               DFM2G_SWEEP_TILES for 3x3 blocks where the
+                               tiles' steps are at least half full, rows have
+                               at most 8 dependency blocks per triangle and,
+                               for FP64, the pattern has at least 77,824
+                               rows; DFM2G_SWEEP_CHAINS otherwise            */
 };
 
 typedef struct dfm2g_bsr_s *dfm2g_bsr;       /* CMatrixSparse<double>       */
@@ -231,21 +236,27 @@ DFM2G_API int dfm2g_ilu_solve_precond(dfm2g_ilu p, int prec, void *vec, int mem)
  * (DFM2G_ERR_STATE otherwise). Schedules whose data is built on first use
  * fall back to the sync-free schedule until an ordinary sweep of the same
  * precision has built that data: DFM2G_SWEEP_TILES (tile records),
- * DFM2G_SWEEP_CHAINS (chain records) and DFM2G_SWEEP_BLOCK (the level-ordered
- * stream and its input buffer). The other schedules (sync-free, levels,
+ * DFM2G_SWEEP_CHAINS and DFM2G_SWEEP_AUTO (tile or chain records) and
+ * DFM2G_SWEEP_BLOCK (the level-ordered stream and its input buffer). The other schedules (sync-free, levels,
  * groups, parts) need nothing built. */
 DFM2G_API int dfm2g_ilu_solve_precond_noalloc(dfm2g_ilu p, int prec, void *vec);
 /* 1x1 and 2x2 patterns take DFM2G_SWEEP_SYNCFREE, DFM2G_SWEEP_LEVELS, DFM2G_SWEEP_CHAINS and
- * DFM2G_SWEEP_AUTO (the chains). */
+ * DFM2G_SWEEP_AUTO (the same as DFM2G_SWEEP_CHAINS). */
 DFM2G_API int dfm2g_ilu_set_sweep_mode(dfm2g_ilu p, int mode);
 /* Current schedule (a new pattern starts with DFM2G_SWEEP_AUTO). */
 DFM2G_API int dfm2g_ilu_get_sweep_mode(dfm2g_ilu p, int *mode);
-/* Schedule the last forward (backward = 0) or backward (backward = 1) sweep of
- * precision `prec` ran: one of the DFM2G_SWEEP_* schedules other than
- * DFM2G_SWEEP_AUTO (which picks among them), or -1 before the first sweep.
- * Shows which schedule the automatic choice, or a fallback of an explicit
- * mode, took. Host only: reads a value the host recorded at launch. */
+/* Schedule of the last forward (backward = 0) or backward (backward = 1) sweep
+ * of precision `prec`: one of the DFM2G_SWEEP_* schedules other than
+ * DFM2G_SWEEP_AUTO, or -1 before the first sweep. An explicit mode's own
+ * unless a fallback ran; for DFM2G_SWEEP_AUTO the name that its rule gives the
+ * pattern (see there). DFM2G_SWEEP_TILES and DFM2G_SWEEP_CHAINS share two
+ * kernels: dfm2g_ilu_last_kernel tells which of them ran. Host only: reads a
+ * value the host recorded at launch. */
 DFM2G_API int dfm2g_ilu_last_schedule(dfm2g_ilu p, int prec, int backward, int *mode);
+/* Kernel of that sweep: DFM2G_SWEEP_TILES for the one over tiles,
+ * DFM2G_SWEEP_CHAINS for a warp per chain, else what dfm2g_ilu_last_schedule
+ * says. The same arguments and values. */
+DFM2G_API int dfm2g_ilu_last_kernel(dfm2g_ilu p, int prec, int backward, int *mode);
 /* Inspection (host outputs): sorted pattern (col: nnz, dia_ind: nblk), factor
  * values, level sets (level: nblk, order: nblk, level_start: nlevels+1 with
  * room for nblk+1). */
