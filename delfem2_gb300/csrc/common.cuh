@@ -398,7 +398,8 @@ struct ChainSched {
 // descriptors, the groups' header words and slot sources, and the records
 // (rewritten after each decomposition).
 struct TileSched {
-  bool built = false, ok = false, thin = false;  // thin: too few rows per tile, not swept unless asked for
+  bool built = false, ok = false;
+  bool thin = false, forced = false;  // too few rows per tile, only swept when asked for; built although thin
   unsigned ntiles = 0, nsteps = 0, ms = 0, max_groups = 0, max_tile = 0;  // ms: slots per lane
   unsigned max_list = 0, max_record = 0;  // longest row list, longest record / 16
   size_t stream16 = 0;                // bytes of the records / 16
@@ -506,7 +507,7 @@ int cluster_sweep(dfm2g_ilu_s *p, bool forward, const T *in, T *out, const T *vc
 void tile_partition(unsigned n, const unsigned *rs, const unsigned *dia, const unsigned *col, const unsigned *order,
                     bool fwd, unsigned max_rows, unsigned max_segs, unsigned max_width,
                     std::vector<unsigned> &tile_of, std::vector<unsigned> &lev, unsigned &ntiles, unsigned &m,
-                    unsigned give_up);
+                    unsigned give_up, bool force, bool *gave_up);
 template <typename T>
 int part_sweep(dfm2g_ilu_s *p, bool forward, const T *in, T *out, const T *vcrs, const T *vdia, const int *skip,
                unsigned long long timeout);

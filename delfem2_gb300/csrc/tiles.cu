@@ -59,15 +59,17 @@ namespace dfm2g {
 // segment is in the tile or the tile has fewer than max_segs segments, and
 // its local level has fewer than max_width rows. The tiles are numbered along
 // the wavefront. Outputs per row: its tile and local level; m = the most
-// dependencies of a row. give_up > 0: stops (ntiles = 0) once a sixteenth of the
-// rows is in tiles of fewer than give_up rows on average.
+// dependencies of a row. give_up > 0: *gave_up tells whether, once a sixteenth
+// of the rows was assigned, they were ever in tiles of fewer than give_up rows on
+// average; without force the partition stops there (ntiles = 0).
 constexpr unsigned kTiSegFar = 1u << 20;  // layer step to the next segment of the same strand
 
 void tile_partition(unsigned n, const unsigned *rs, const unsigned *dia, const unsigned *col, const unsigned *order,
                     bool fwd, unsigned max_rows, unsigned max_segs, unsigned max_width,
                     std::vector<unsigned> &tile_of, std::vector<unsigned> &lev, unsigned &ntiles, unsigned &m,
-                    unsigned give_up) {
+                    unsigned give_up, bool force, bool *gave_up) {
   const unsigned none = ~0u;
+  if (gave_up) *gave_up = false;
   tile_of.assign(n, none);
   lev.assign(n, 0u);
   m = 0;
@@ -148,8 +150,11 @@ void tile_partition(unsigned n, const unsigned *rs, const unsigned *dia, const u
     while (cursor < n && tile_of[order[cursor]] != none) ++cursor;
     if (cursor >= n) break;
     if (give_up && assigned >= n / 16u && assigned < (size_t)give_up * t) {
-      ntiles = 0;
-      return;
+      *gave_up = true;
+      if (!force) {
+        ntiles = 0;
+        return;
+      }
     }
     const unsigned seed = order[cursor];
     for (unsigned r : offered) layer_of[r] = none;
@@ -241,9 +246,9 @@ void tile_host_build(unsigned n, const std::vector<unsigned> &rs, const std::vec
   std::vector<unsigned> tile_of, lev;
   unsigned ntiles = 0, m = 0;
   tile_partition(n, rs.data(), dia.data(), col.data(), order.data(), fwd, sh.rows, sh.segs, sh.width, tile_of, lev,
-                 ntiles, m, force ? 0u : kTiLeastRows / 3u);
-  out.thin = !force && (ntiles == 0 || (ntiles > 1 && n < (size_t)kTiLeastRows * ntiles));
-  if (out.thin) return;
+                 ntiles, m, kTiLeastRows / 3u, force, &out.thin);
+  out.thin |= ntiles > 1 && n < (size_t)kTiLeastRows * ntiles;  // the pattern's, whether asked for or not
+  if (out.thin && !force) return;
   const unsigned S = sh.S, G = 32u / (sh.B * S);
   const unsigned need = std::max(1u, (m + (fwd ? 1u : 0u) + S - 1u) / S);
   unsigned ms = 0;
@@ -409,9 +414,12 @@ int tile_build(dfm2g_ilu_s *p, TileSched *pair, const TileShape &sh, bool force)
   const unsigned n = p->nblk;
   bool need[2], any = false;
   for (int d = 0; d < 2; ++d) {
-    need[d] = !pair[d].built || (force && pair[d].thin);
+    need[d] = !pair[d].built || (force && pair[d].thin && !pair[d].forced);
     pair[d].built = true;
-    if (need[d]) pair[d].ok = pair[d].thin = false;
+    if (need[d]) {
+      pair[d].ok = pair[d].thin = false;
+      pair[d].forced = force;
+    }
     any |= need[d];
   }
   if (!any) return DFM2G_OK;
@@ -627,8 +635,8 @@ int tile_run(dfm2g_ilu_s *p, TileSched *pair, const TileShape &sh, bool forward,
              const int *skip, unsigned long long timeout, bool may_alloc, bool force, bool *usable) {
   TileSched &ts = pair[forward ? 0 : 1];
   if (!may_alloc && (!ts.built || !ts.ok || !ts.bytes.p)) return DFM2G_OK;
-  if (!ts.built || (force && ts.thin)) DFM2G_TRY(tile_build(p, pair, sh, force));
-  if (!ts.ok) return DFM2G_OK;
+  if (!ts.built || (force && ts.thin && !ts.forced)) DFM2G_TRY(tile_build(p, pair, sh, force));
+  if (!ts.ok || (ts.thin && !force)) return DFM2G_OK;
   return tile_launch<T, B, S, NW, HW, MSA, MSB, MSC, MSD>(p, ts, forward, in, out, fill, skip, timeout, usable);
 }
 
@@ -689,7 +697,7 @@ template int tile_sweep<double>(dfm2g_ilu_s *, bool, const double *, double *, s
 void tile_schedules_reset(dfm2g_ilu_s *p) {
   for (auto &pair : p->tiles)
     for (TileSched &ts : pair) {
-      ts.built = ts.ok = ts.thin = false;
+      ts.built = ts.ok = ts.thin = ts.forced = false;
       ts.ntiles = ts.nsteps = ts.ms = ts.max_groups = ts.max_tile = ts.max_list = ts.max_record = 0;
       ts.rows_per_step = 0;
       ts.ngroups = ts.stream16 = 0;
@@ -723,7 +731,8 @@ int dfm2g_tile_partition(unsigned n, const unsigned *row_start, const unsigned *
   if (max_rows == 0 || max_width == 0) return fail(DFM2G_ERR_ARG, "tile_partition: zero tile size");
   std::vector<unsigned> t, lv;
   unsigned nt = 0, m = 0;
-  tile_partition(n, row_start, dia_ind, col, order, backward == 0, max_rows, max_width, max_width, t, lv, nt, m, 0u);
+  tile_partition(n, row_start, dia_ind, col, order, backward == 0, max_rows, max_width, max_width, t, lv, nt, m, 0u,
+                 false, nullptr);
   if (n) {
     std::copy(t.begin(), t.end(), tile_of);
     std::copy(lv.begin(), lv.end(), level);

@@ -79,3 +79,21 @@ def test_last_kernel_rejects_bad_arguments(gpu):
     assert gpu.dfm2g_ilu_last_kernel(ilu._h, 5, 0, C.byref(m)) != 0
     assert gpu.dfm2g_ilu_last_kernel(ilu._h, N.F32, 0, None) != 0
     assert gpu.dfm2g_ilu_last_kernel(None, N.F32, 0, C.byref(m)) != 0
+
+
+@pytest.mark.parametrize("modes", [(TILES, AUTO), (AUTO, TILES, AUTO), (TILES, CHAINS, TILES)])
+def test_a_forced_schedule_is_not_taken_unasked(gpu, modes):
+    """Thin tiles, once built for DFM2G_SWEEP_TILES, stay off the other modes' sweeps; the results agree."""
+    ilu, n = _handle((14, 13, 12), 3, perm=True)
+    b = np.random.default_rng(1).standard_normal(n)
+    first = None
+    for mode in modes:
+        ilu.set_sweep_mode(mode)
+        for fp64, dtype in ((True, np.float64), (False, np.float32)):
+            x = b.astype(dtype)
+            ilu.SolvePrecond(x)
+            want = TILES if mode == TILES else CHAINS
+            assert [ilu.last_kernel(fp64, k) for k in (False, True)] == [want, want], (mode, fp64)
+            if first is None:
+                first = x
+            assert np.abs(x - first).max() < (1e-12 if fp64 else 1e-5) * np.abs(first).max()
