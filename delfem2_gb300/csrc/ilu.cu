@@ -572,7 +572,9 @@ __global__ void __launch_bounds__(32 * kFlowWarps) k_ilu_factor_flow(
     // readiness of the lower triangle's rows, 32 at a time: bit l of `ready`
     // once row col[s0 + r0 + l] carries this decomposition's flag. need(l)
     // waits (bounded) for it, so that the updates from rows of earlier levels
-    // are done while the level just before is still at work.
+    // are done while the level just before is still at work. One lane acquires a
+    // row's flag and all of them read the row: the barrier behind the vote, which
+    // orders nothing itself, hands the acquired writes to the other lanes.
     unsigned ready = 0, r0 = ~0u;
     const unsigned *flag = nullptr;
     auto need = [&](unsigned l) -> bool {
@@ -583,7 +585,9 @@ __global__ void __launch_bounds__(32 * kFlowWarps) k_ilu_factor_flow(
       }
       unsigned long long t0 = 0;
       unsigned spins = 0;
+      bool voted = false;
       while (!((ready >> (l & 31u)) & 1u)) {
+        voted = true;
         bool ok = r0 + lane < nk && ((ready >> lane) & 1u || ld_acquire(flag) == epoch);
         ready = __ballot_sync(0xffffffffu, ok);
         if ((++spins & 63u) == 0) {
@@ -596,6 +600,7 @@ __global__ void __launch_bounds__(32 * kFlowWarps) k_ilu_factor_flow(
           }
         }
       }
+      if (voted) __syncwarp();
       return true;
     };
     auto known = [&](unsigned l) { return (l & ~31u) == r0 && ((ready >> (l & 31u)) & 1u); };
