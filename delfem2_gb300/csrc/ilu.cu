@@ -1558,6 +1558,7 @@ int dfm2g_ilu_decompose(dfm2g_ilu p, int *n_singular) try {
       k_ilu_factor_level_nd<1><<<blocks, 256, 0, stream()>>>(p->order_f.p + ls[l], nrows, p->row_start.p, p->col.p,
                                                              p->dia_ind.p, p->vcrs.p, p->vdia.p, p->nsing.p);
   }
+  if (!flowed && ls.size() > 1) note_launches((unsigned)ls.size() - 1);
   DFM2G_LAUNCH_CHECK();
   int ns = 0, e = 0;
   DFM2G_CUDA(cudaMemcpyAsync(&ns, p->nsing.p, sizeof(int), cudaMemcpyDeviceToHost, stream()));
