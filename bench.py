@@ -103,24 +103,22 @@ class ClockSampler:
 
 
 # ---------------------------------------------------------------------------
-def algorithmic_bytes(kind: str, nb: int, nz: int, s: int, fused: bool = False) -> float:
+def algorithmic_bytes(kind: str, nb: int, nz: int, s: int) -> float:
     """Bytes one launch of a kernel class must move (each array once per pass).
 
     nb block rows, nz off-diagonal blocks, s = bytes per value; index arrays u32.
-    nz/2 blocks lie in each triangle (the pattern is symmetric). fused: a solve
-    whose SpMV launch also runs the update pass and whose dot launch the p update
-    (no "update" class in its profile)."""
+    nz/2 blocks lie in each triangle (the pattern is symmetric)."""
     v3 = 3 * s * nb
-    if kind == "spmv":      # K values + col + row_start, p read, Ap written (+ the update pass)
-        return 9 * s * (nz + nb) + 4 * nz + 4 * (nb + 1) + 2 * v3 + (8 * v3 if fused else 0)
+    if kind == "spmv":      # K values + col + row_start, p read, Ap written
+        return 9 * s * (nz + nb) + 4 * nz + 4 * (nb + 1) + 2 * v3
     if kind == "fwd":       # L blocks + D^-1 + col/row_start/dia_ind/order, in read, out written
         return 9 * s * (nz / 2 + nb) + 4 * nz / 2 + 4 * (3 * nb + 1) + 2 * v3
     if kind == "bwd":       # U' blocks + col/row_start/dia_ind/order, in read, out written
         return 9 * s * (nz / 2) + 4 * nz / 2 + 4 * (3 * nb + 1) + 2 * v3
     if kind == "update":    # r, x, p, Ap read; r, x and the sweeps' two pending-marker outputs written
         return 8 * v3
-    if kind == "dot":       # r, z read (+ the p update pass: p, z read, p written)
-        return 2 * v3 + (3 * v3 if fused else 0)
+    if kind == "dot":       # r, z read
+        return 2 * v3
     if kind == "pupdate":   # p, z read; p written
         return 3 * v3
     return float("nan")
@@ -582,10 +580,9 @@ def run_ours(args):
     hbm, peak_kind = peaks()
     dom = max((k for k in prof if k in ("spmv", "fwd", "bwd", "update", "dot", "pupdate")),
               key=lambda k: prof[k]["ms_total"])
-    fused = "update" not in prof  # the update ran inside the SpMV launch, the p update inside the dot's
-    alg = algorithmic_bytes(dom, nb, nz, 4, fused)
+    alg = algorithmic_bytes(dom, nb, nz, 4)
     achieved = alg / (prof[dom]["ms_avg"] * 1e-3) / 1e9
-    per_kernel = {k: dict(v, gbs=(algorithmic_bytes(k, nb, nz, 4, fused) / (v["ms_avg"] * 1e-3) / 1e9
+    per_kernel = {k: dict(v, gbs=(algorithmic_bytes(k, nb, nz, 4) / (v["ms_avg"] * 1e-3) / 1e9
                                   if k != "outer" else None)) for k, v in prof.items()}
 
     cpu = None

@@ -286,7 +286,8 @@ __device__ __forceinline__ bool grid_sum_last(double partial, double *partials,
   return threadIdx.x == 0;
 }
 
-// Barrier of all CTAs of a cooperative launch over one word (*bar, 0 at the
+// Barrier of all CTAs of a cooperative launch (the solvers' kernels no longer meet at
+// one; dfm2g_debug_grid_barrier checks it) over one word (*bar, 0 at the
 // start): its low 16 bits count arrivals, its high 16 bits the barriers passed.
 // An arrival adds 1 and learns the generation it waits out from the old value;
 // the last one adds what takes the count back to 0 and the generation on by one
@@ -328,7 +329,7 @@ __device__ __forceinline__ bool grid_barrier(unsigned *bar, int *err, unsigned l
 // ---- handle layouts -----------------------------------------------------------------
 struct dfm2g_bsr_s {
   unsigned nblk = 0;
-  unsigned ndim = 3;  // block size: 3x3 (TMA SpMV, every sweep schedule), 1x1 or 2x2 (nd.cuh kernels)
+  unsigned ndim = 3;  // block size: 3x3 (every sweep schedule), 2x2 or 1x1
   size_t nnz = 0;
   bool has_pattern = false;
   std::vector<unsigned> h_row_start, h_col;  // host copy of the pattern

@@ -1222,8 +1222,8 @@ int ilu_sweep(dfm2g_ilu_s *p, int prec, bool forward, const void *in, void *out)
   return sweep_impl<float>(p, forward, (const float *)in, (float *)out, p->vcrs32.p, p->vdia32.p, nullptr, false);
 }
 
-// A sweep that allocates nothing: the chain schedule is used only when its
-// records already exist, otherwise the sync-free one. The FP32 factors must exist.
+// A sweep that allocates nothing: the tile and chain schedules are used only when
+// their records already exist, otherwise the sync-free one. The FP32 factors must exist.
 static int ilu_sweep_noalloc(dfm2g_ilu_s *p, int prec, bool forward, const void *in, void *out) {
   if (prec == DFM2G_F64)
     return sweep_impl<double>(p, forward, (const double *)in, (double *)out, p->vcrs.p, p->vdia.p, nullptr, false,

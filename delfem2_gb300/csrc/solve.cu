@@ -52,9 +52,10 @@ constexpr int kThreads = 256;
 // Reliable updates ask for the deciding FP64 residual once the FP32 one is
 // below this share of the tolerance. Asked for at the tolerance itself, the
 // true residual stops anywhere near it and the solution's error with it, by the
-// summation order alone (48^3 gradients at a tolerance of 2e-11, 14 seeds: 1.2e-11
-// to 2.0e-9; at 0.7 of it 1.1e-11 to 2.0e-9 with fewer above 5e-10, 1 against
-// 3), for about 1% more iterations.
+// summation order alone. Gradients at a tolerance of 2e-11, 24 seeds, error
+// against 64 bits, mean and largest: 48^3 cells 1.9e-10 and 9.1e-10 at 0.7,
+// 4.6e-10 and 5.1e-9 at 1.0; 25 x 41 x 30 cells 1.9e-10 and 7.0e-10, 2.8e-10 and
+// 8.1e-10; for 2-3% more time.
 constexpr double kFinalRefresh = 0.7;
 
 // p.Ap fused into the SpMV Ap = K p (warp per block row); the last block sets
@@ -748,7 +749,7 @@ static int pcg_core(dfm2g_bsr_s *m, dfm2g_ilu_s *p, T *r, T *x, T *w0, T *w1, T 
   for (;;) {
     for (int k = 0; k < chunk; ++k) {
       T *Ap = Pr;
-      // the sweeps' outputs get their pending marker in the update (Ap is Pr: read first, element by element)
+      // the sweeps' outputs get their pending marker in the update (Ap is Pr: read first, chunk by chunk)
       const bool fill = mode != 1 && p->sweep_mode != DFM2G_SWEEP_LEVELS;
       T *fa = fill ? mid : nullptr, *fb = fill ? Pr : nullptr;
       {

@@ -23,9 +23,9 @@
  *    and one stream: call it from one host thread at a time (the error
  *    message is per thread; handles and cached kernel settings are shared
  *    and not locked).
- *  - Block sizes 1x1, 2x2 and 3x3 (ndim 1, 2, 3). The 3x3 path is the tuned
- *    one (TMA-staged SpMV, every sweep schedule); 1x1 and 2x2 matrices run
- *    warp-per-row kernels with the sync-free and level sweep schedules.
+ *  - Block sizes 1x1, 2x2 and 3x3 (ndim 1, 2, 3). Every size has the TMA-staged
+ *    SpMV and the tile sweeps; the other sweep schedules but the sync-free, level
+ *    and chain ones are written for 3x3.
  *    Entry points written for one block size (the linear-tet elasticity and
  *    cloth assemblers: 3x3; Poisson: 1x1; the 2-D solid: 2x2) return
  *    DFM2G_ERR_UNSUPPORTED for another.
