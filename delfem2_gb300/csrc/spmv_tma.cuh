@@ -43,17 +43,17 @@ __device__ __forceinline__ void round16(size_t off, size_t end, size_t &a, unsig
 // sums over whole blocks take a fourth instruction, the addition, per block).
 // The rounding error is no larger: root mean square 0.299 against 0.305 units
 // of 1e-16 |K||x| over 14-block rows that cancel, 0.180 against 0.212 on smooth
-// vectors. 1x1 and 2x2 rows keep four sums in both types, for as little error as
-// eight lanes' sums and a tree: over 14 terms 0.410 against 0.418 units of
-// random ones, 0.256 against 0.275 of smooth vectors, 0.440 against 0.551 with a
-// dominant diagonal (two sums: 0.425, 0.256, 0.503).
+// vectors. 1x1 and 2x2 rows sum the same way in both types: over 14 terms 0.425
+// units against eight lanes' sums and a tree's 0.418 (random ones), 0.256
+// against 0.275 (smooth vectors), 0.503 against 0.551 (a dominant diagonal).
 //
 // One lane works through a row, so a long row is a long serial chain, of time
 // and of roundings: patterns with a row of more than kLongest blocks take the
-// kernels with a warp or eight lanes a row. 1x1 and 2x2: at 24 blocks four sums
-// have 0.78 to 1.04 of the eight lanes' error, at 64 up to 1.2; a 2,000-block
-// row takes 106 us FP64 (52 ns a block) against 50. 3x3: a 1,400-block row takes
-// 240 us FP64 against 35.
+// kernels with a warp or eight lanes a row. 1x1 and 2x2: the two sums' error is
+// 0.91 to 1.02 of the eight lanes' at 14 blocks, 0.91 to 1.16 at 24, up to 1.5 at
+// 64 (four sums: 0.78 to 1.04 at 24, but 1.2 us more in 25 for the FP64 scalar
+// product at 64^3); a 2,000-block row takes 106 us FP64 (52 ns a block) against
+// 50. 3x3: a 1,400-block row takes 240 us FP64 against 35.
 #ifndef DFM2G_SPMV_F32_CONSUMERS
 #define DFM2G_SPMV_F32_CONSUMERS 15u  // FP32 tile: consumer warps (ten rows each)
 #endif
@@ -70,7 +70,7 @@ struct TileCfgC {
   static constexpr unsigned kWarpRows = 32u / B;
   static constexpr unsigned kRows = kConsumers * kWarpRows;
   static constexpr unsigned kBlocks = B < 3 ? kRows * 16u : sizeof(T) == 8 ? 1424u : DFM2G_SPMV_F32_BLOCKS;
-  static constexpr unsigned kLongest = B < 3 ? 24u : 1152u;
+  static constexpr unsigned kLongest = B < 3 ? 16u : 1152u;
   static constexpr unsigned kStages = sizeof(T) == 8 ? 2u : DFM2G_SPMV_F32_STAGES;
   static constexpr unsigned kValBytes = kBlocks * B * B * sizeof(T) + 32;
   static constexpr unsigned kColBytes = kBlocks * 4 + 32;
@@ -161,8 +161,8 @@ __device__ __forceinline__ void spmv_tma_rows_c(const unsigned *__restrict__ til
       const T *d = dv + (size_t)(i - r0) * BB + a * B, *xi = x + (size_t)i * B;
       unsigned u = s0;
       if constexpr (sizeof(T) == 8 || B < 3) {
-        constexpr unsigned W = B == 3 ? 2 : 4;  // blocks per step, each with sums of its own
-        T sum[W][B] = {};
+        constexpr unsigned W = B == 3 ? 2 : 4;  // blocks per step
+        T e[B] = {}, o[B] = {};                 // sums over the blocks of either parity
         // the next step's x gathered under this step's products, the first
         // step's under the row's remainder
         T g[W * B] = {};
@@ -179,7 +179,7 @@ __device__ __forceinline__ void spmv_tma_rows_c(const unsigned *__restrict__ til
           if (w < rem) {
             const T *v = vv + (size_t)u * BB + a * B, *y = x + (size_t)cv[u] * B;
 #pragma unroll
-            for (unsigned c = 0; c < B; ++c) sum[w][c] += v[c] * __ldg(y + c);
+            for (unsigned c = 0; c < B; ++c) (w & 1 ? o : e)[c] += v[c] * __ldg(y + c);
             ++u;
           }
         }
@@ -193,21 +193,17 @@ __device__ __forceinline__ void spmv_tma_rows_c(const unsigned *__restrict__ til
 #pragma unroll
           for (unsigned w = 0; w < W; ++w)
 #pragma unroll
-            for (unsigned c = 0; c < B; ++c) sum[w][c] += v[w * BB + c] * h[w * B + c];
+            for (unsigned c = 0; c < B; ++c) (w & 1 ? o : e)[c] += v[w * BB + c] * h[w * B + c];
         }
         // the diagonal block, the largest terms, summed apart and added late: few
         // sums are rounded at its size
         T t = d[0] * __ldg(xi);
 #pragma unroll
         for (unsigned c = 1; c < B; ++c) t += d[c] * __ldg(xi + c);
+        T se = e[0], so = o[0];
 #pragma unroll
-        for (unsigned w = 0; w < W; ++w)
-#pragma unroll
-          for (unsigned c = 1; c < B; ++c) sum[w][0] += sum[w][c];
-        if constexpr (W == 2)
-          epi(i, a, sum[0][0] + (sum[1][0] + t));
-        else
-          epi(i, a, ((sum[0][0] + sum[1][0]) + (sum[2][0] + sum[3][0])) + t);
+        for (unsigned c = 1; c < B; ++c) se += e[c], so += o[c];
+        epi(i, a, se + (so + t));
       } else {
         T acc0 = T(0), acc1 = T(0);
         for (; u + 1 < s1; u += 2) {

@@ -1,6 +1,6 @@
 """The kernels that ordinary patterns do not reach: the factorisation by levels (rows too long for the one-launch kernel's
 shared memory), a warp per chain in the sweeps (rows of more than 15 blocks in a triangle), and the row products with
-eight lanes or a warp a row (a row of more than 24 blocks, 1,152 for 3x3) inside every solver. Each test shows by the
+eight lanes or a warp a row (a row of more than 16 blocks, 1,152 for 3x3) inside every solver. Each test shows by the
 launch count or dfm2g_ilu_last_kernel, or by the rule's own limit on both sides, that it is there. Factors within
 1e-10 of the oracle's (3x3; equal bits for 1x1 and 2x2), sweeps within 1e-12 FP64 and 1e-5 FP32, products within
 (ndim k + 8) eps |K||x| of a k-block row, solves of diagonally dominant systems to 1e-10."""
@@ -128,7 +128,7 @@ def _hub(n, ndim, blocks, seed=0):
     return np.searchsorted(row, np.arange(n + 1)).astype(np.uint32), col.astype(np.uint32), row, val, dia
 
 
-@pytest.mark.parametrize("ndim,blocks", [(1, 24), (1, 25), (1, 700), (2, 24), (2, 25), (2, 700), (3, 1152), (3, 1153)])
+@pytest.mark.parametrize("ndim,blocks", [(1, 16), (1, 17), (1, 700), (2, 16), (2, 17), (2, 700), (3, 1152), (3, 1153)])
 def test_solves_with_a_long_row(gpu, ndim, blocks):
     import delfem2_gb300 as D
     n = 1500
