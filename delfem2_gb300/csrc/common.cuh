@@ -210,14 +210,16 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
 // FP32 arithmetic only produces the NaN 0x7fffffff, so a computed value never
 // equals it. FP64 arithmetic makes 0xfff8000000000000 but hands on the payload of
 // a NaN operand, so an all-ones NaN (or, negated, 0x7fff...f) among the inputs
-// could come out as the marker: settled() is what a sweep stores of a value.
+// could come out as the marker. A sweep passes what it stores through settled(),
+// or (the tile kernel, whose stores are on its critical path) all that it reads.
 __device__ __forceinline__ bool is_pending(float v) { return __float_as_uint(v) == 0xffffffffu; }
 __device__ __forceinline__ bool is_pending(double v) {
   return __double_as_longlong(v) == (long long)-1;
 }
 __device__ __forceinline__ float settled(float v) { return v; }
-__device__ __forceinline__ double settled(double v) {
-  return is_pending(v) ? __longlong_as_double(0x7fffffffffffffffll) : v;
+__device__ __forceinline__ double settled(double v) {  // such a high word is a NaN's, whatever the low one
+  const int hi = __double2hiint(v), lo = __double2loint(v);
+  return __hiloint2double(hi, (hi & 0x7fffffff) == 0x7fffffff ? 0 : lo);
 }
 template <typename T>
 __device__ __forceinline__ T pending_value() {

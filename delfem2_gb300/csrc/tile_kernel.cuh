@@ -365,7 +365,7 @@ __global__ void __launch_bounds__(32 * (NW + HW + 1), 1)
       }
 #pragma unroll
       for (unsigned k = 0; k < kFo; ++k)
-        if (on && lr + kRp * k < own) area[kRp * k * kXw] = rhs[k];
+        if (on && lr + kRp * k < own) area[kRp * k * kXw] = settled(rhs[k]);
       __threadfence_block();
       __syncwarp();
       asm volatile("bar.arrive %0, %1;" ::"r"(slot + 1u == A.nslots ? 1u : slot + 2u), "n"(kMeet) : "memory");
@@ -490,7 +490,7 @@ __global__ void __launch_bounds__(32 * (NW + HW + 1), 1)
     }
     if (C.row != ~0u && h == kOut) {
       reinterpret_cast<T *>(xs + (size_t)C.local * kRow)[a] = z;
-      st_relaxed(out + (size_t)C.row * B + a, settled(z));
+      st_relaxed(out + (size_t)C.row * B + a, z);
     }
     if (!more) {
       // the end markers need this slot too (they touch only its descriptor)

@@ -516,7 +516,7 @@ __global__ void k_tile_fill(size_t ngroups, const double *__restrict__ vcrs, con
           x = vcrs[(size_t)s * (B * B) + a * B + c];
         }
       }
-      v[i] = (T)x;
+      v[i] = settled((T)x);  // as the right-hand side, in the kernel
     }
     stream16[(size_t)goff[g] + geo.vo / 16u + r] = *reinterpret_cast<const uint4 *>(v);
   }
