@@ -402,11 +402,11 @@ static int check_bsr(dfm2g_bsr m, bool need_pattern = true) {
   return DFM2G_OK;
 }
 
-// A product of host vectors ends with its one wait, the error word read under
-// it. Of device vectors only the 3x3 product waits (and reports at once); a
-// 1x1 or 2x2 one is queued and returns, as it always has, so that it can be
-// captured, and a wait of its copies that gave up is reported by the next call
-// on the matrix that waits. (Waiting, 1,000 scalar rows took 31 us a call, 15 without.)
+// A 3x3 product waits and reports before its result is handed out. A 1x1 or 2x2
+// product of device vectors is queued and returns, so that it can be captured
+// (waiting, 1,000 scalar rows took 31 us a call, 15 without); should a wait for
+// its copies ever give up, the next call on the matrix that waits reports it.
+// Of host vectors it reads the error word under its one wait.
 template <typename T>
 static int matvec(dfm2g_bsr m, int prec, T *y, double alpha, const T *x, double beta, int mem) {
   const size_t n = (size_t)m->nblk * m->ndim;
@@ -414,7 +414,11 @@ static int matvec(dfm2g_bsr m, int prec, T *y, double alpha, const T *x, double 
   DFM2G_TRY(ay.in(y, n, mem, true));
   DFM2G_TRY(ax.in(x, n, mem, true));
   DFM2G_TRY(bsr_spmv(m, prec, ay.dev(), alpha, ax.dev(), beta));
-  if (mem == DFM2G_MEM_DEVICE) return m->ndim == 3 ? bsr_check_err(m) : DFM2G_OK;
+  if (m->ndim == 3) {
+    DFM2G_TRY(bsr_check_err(m));
+    return ay.copy_back();
+  }
+  if (mem == DFM2G_MEM_DEVICE) return DFM2G_OK;
   DFM2G_TRY(bsr_queue_err(m));
   DFM2G_TRY(ay.copy_back());
   return bsr_take_err(m);
